@@ -71,6 +71,7 @@
 
 #include "../../include/sdgpu.h"
 #include "sdg_dense.h"
+#include "sdg_kth.cuh"
 #include "sdg_tc_ptx.cuh"
 
 namespace sdg {
@@ -131,15 +132,10 @@ struct TcArgs {
   int stall;                  // failure-detection test: the MMA issuer's first wait never completes
 };
 
-// Order-preserving map of a float onto uint32 (ascending value -> ascending
-// key), so that atomicMax on the keys is a max on the floats.
-__device__ __forceinline__ unsigned fkey(float f) {
-  const unsigned b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float fkey_value(unsigned k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
+// The order-preserving map of a float onto uint32: atomicMax on the keys is a
+// max on the floats.
+using kth::fkey;
+using kth::fkey_value;
 constexpr int SHARE_TILES = 8;          // tiles between exchanges of the shared running key
 
 // the first and the last work unit (a CTA, or a CTA pair) whose span holds an
@@ -568,25 +564,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
 }
 
 // ---- merge: the final cut of each query over its lists ---------------------
-constexpr int MW = 8;   // warps per block
-
-__device__ __forceinline__ void warp_insert_desc_tc(float* lst, int K, int& n, unsigned m, float v, int lane) {
-  while (m) {
-    const int src = __ffs(m) - 1;
-    m &= m - 1;
-    const float x = __shfl_sync(0xffffffffu, v, src);
-    if (n == K && !(x > lst[K - 1])) continue;
-    int a = 0, b = n;
-    while (a < b) { const int mid = (a + b) >> 1; if (lst[mid] >= x) a = mid + 1; else b = mid; }
-    const int last = (n < K) ? n : K - 1;
-    if (lane == 0) {                               // K <= 64: a serial shift is short
-      for (int e = last; e > a; --e) lst[e] = lst[e - 1];
-      lst[a] = x;
-    }
-    __syncwarp();
-    if (n < K) ++n;
-  }
-}
+// Warps per query: 32 for a handful of queries, 8 while a warp per query would
+// leave an SM fewer than 16 warps, else 1.  One query over 302 lists: 113 us
+// with 8 warps; 777 over 44: 47 us with 8 against 150 with 1; 3,000: 98 and
+// 99; 4,096: 124 and 114; 16,384: 302 and 137.
+constexpr int64_t MERGE_WIDEST_MAX = 152 * 2, MERGE_WIDE_MAX = 152 * 16;
 
 struct MergeArgs {
   int64_t q0, nq;
@@ -609,6 +591,7 @@ struct MergeArgs {
   float* cand_s;               // [nq][cap] the candidates' GEMM values
   int32_t* count;
   int32_t* over;
+  size_t smem_query;           // shared-memory bytes of one query's prefix and keys
 };
 
 // The per-pair bound of one candidate from the columns' BF16 copies: with v
@@ -646,78 +629,118 @@ __device__ __forceinline__ void tight_bounds(const MergeArgs& A, float s, int64_
 // most the exact k-th best key (k candidates reach it), so every member of the
 // exact top k (ties included) has its per-pair upper bound at or above
 // dense_cut(max(T, T2)) and is kept.
-__global__ void k_tc_merge(MergeArgs A) {
-  __shared__ float sl[MW][KT];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ql = (int64_t)blockIdx.x * MW + warp;
+//
+// A list keeps only keys above the shared key it saw, so when some list's
+// view of the shared key reached the final k-th best, fewer than k keys at or
+// above it may be listed; the shared key (the k-th best of a subset, never
+// above the final) then is the final k-th best.  So only keys above the
+// shared key are collected (in shared memory), and T is their k-th largest
+// (kth::largest) or, with fewer than k of them, the shared key.
+//
+// WPQ warps work on a query, its appended references as one flat range over
+// the lists (a shared-memory prefix of their counts, a binary search per
+// reference), so their loads do not wait on one another.  What bounds it is
+// latency: one warp taking a query's lists in turn, with k-long sorted
+// insertions, took 606 us for one query over 302 lists, 209 us for 777 queries
+// over 44, 170 us for 3,000 (k = 30) over 14 and 143 us for 4,096 over 12.
+__host__ __device__ __forceinline__ size_t merge_prefix_bytes(int64_t nslots) { return (size_t)((nslots + 4) / 4 * 4) * 4; }
+
+template <int WPQ>
+__global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArgs A) {
+  extern __shared__ __align__(16) unsigned char msm[];
+  constexpr int QPB = WPQ == 1 ? 8 : 1;
+  __shared__ uint32_t red[WPQ];
+  __shared__ int s_count[QPB], s_kept[QPB];
+  const int lane = threadIdx.x & 31;
+  const int slot_q = WPQ == 1 ? (int)(threadIdx.x >> 5) : 0;
+  const int64_t ql = (int64_t)blockIdx.x * QPB + slot_q;
   if (ql >= A.nq) return;
+  const kth::Group<WPQ> G{red};
+  const int rank = G.rank(), nt = G.size();
   const int K = A.K;
+  int32_t* pre = reinterpret_cast<int32_t*>(msm + (size_t)slot_q * A.smem_query);    // inclusive list counts
+  uint32_t* keys = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(pre) + merge_prefix_bytes(A.nslots));
   if (A.qempty[A.q0 + ql]) {
-    if (lane == 0) { A.count[ql] = 0; A.over[ql] = 0; }
+    if (rank == 0) { A.count[ql] = 0; A.over[ql] = 0; }
     return;
   }
   const int64_t g = ql / A.gm;
-  const int64_t used = 2 * (last_cta(g, A.ntiles, A.per) - first_cta(g, A.ntiles, A.per) + 1);
-  float* lst = sl[warp];
-  int n = 0;
-  const float* in = A.lists + ql * A.nslots * (int64_t)K;
-  const int64_t tot = used * K;
-  for (int64_t p0 = 0; p0 < tot; p0 += 32) {
-    const float v = p0 + lane < tot ? in[p0 + lane] : -INFINITY;
-    const unsigned m = __ballot_sync(0xffffffffu, v > -INFINITY && (n < K || v > lst[K - 1]));
-    if (m) warp_insert_desc_tc(lst, K, n, m, v, lane);
+  const int used = (int)(2 * (last_cta(g, A.ntiles, A.per) - first_cta(g, A.ntiles, A.per) + 1));
+  const float ts = fkey_value(A.tshared[ql]);
+  if (rank == 0) s_count[slot_q] = s_kept[slot_q] = 0;
+  // the lists' counts, scanned by the group's first warp
+  bool big = false;
+  if (rank < 32) {
+    int run = 0;
+    for (int r0 = 0; r0 < used; r0 += 32) {
+      const int c = r0 + lane < used ? A.ecount[ql * A.nslots + r0 + lane] : 0;
+      if (c > A.ecap) big = true;
+      int x = min(c, A.ecap);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (r0 + lane < used) pre[r0 + lane] = run + x;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
   }
-  // A list keeps only keys above the shared key it saw, so when some list's
-  // view of the shared key reached the final k-th best, fewer than k keys at
-  // or above it may be listed; the shared key (the k-th best of a subset,
-  // never above the final) then is the final k-th best.
-  const float T = fmaxf((n == K) ? lst[K - 1] : -INFINITY, fkey_value(A.tshared[ql]));
+  bool ovf = G.sum(big ? 1u : 0u) != 0;
+  G.sync();
+  if (ovf) {
+    if (rank == 0) { A.count[ql] = 0; A.over[ql] = 1; }
+    return;
+  }
+  // T from the keys above the shared one
+  const float* in = A.lists + ql * A.nslots * (int64_t)K;
+  const int tot = used * K;
+  for (int p = rank; p < tot; p += nt) {
+    const float v = in[p];
+    if (v > ts) keys[atomicAdd(&s_count[slot_q], 1)] = fkey(v);
+  }
+  G.sync();
+  int n = s_count[slot_q];
+  const float T = n >= K ? fkey_value(kth::largest<WPQ>(G, keys, n, K)) : ts;
   const float cut = dense_cut(T);
   const int64_t q = A.q0 + ql;
   const float Nq = A.qnorm2[q];
-  bool ovf = false;
-  int total = 0;
   int32_t* out = A.cand + ql * (int64_t)A.cap;
   float* out_s = A.cand_s + ql * (int64_t)A.cap;
-  for (int64_t r = 0; r < used && !ovf; ++r) {
-    const int64_t slot = ql * A.nslots + r;
-    const int c = A.ecount[slot];
-    if (c > A.ecap) { ovf = true; break; }
-    for (int p0 = 0; p0 < c; p0 += 32) {
-      const int p = p0 + lane;
-      bool keep = false;
-      int32_t ref = 0;
-      float sv = 0.f;
-      if (p < c) {
-        ref = A.eidx[slot * A.ecap + p];
-        sv = A.es[slot * A.ecap + p];
-        float key, err;
-        dense_key(A.method, 0, A.d, sv, Nq, A.norm2[ref], key, err);
-        keep = key + err >= cut;
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      const int rank = __popc(m & ((1u << lane) - 1u));
-      if (keep && total + rank < A.cap) { out[total + rank] = ref; out_s[total + rank] = sv; }
-      total += __popc(m);
+  const int all = pre[used - 1];
+  for (int p = rank; p < all; p += nt) {
+    int lo = 0, hi = used - 1;                       // the first list whose inclusive count exceeds p
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (pre[mid] > p) hi = mid;
+      else lo = mid + 1;
     }
-    if (total > A.cap) ovf = true;
+    const int64_t at = (ql * A.nslots + lo) * (int64_t)A.ecap + (p - (lo ? pre[lo - 1] : 0));
+    const int32_t ref = A.eidx[at];
+    const float sv = A.es[at];
+    float key, err;
+    dense_key(A.method, 0, A.d, sv, Nq, A.method == COSINE ? 0.f : A.norm2[ref], key, err);
+    if (key + err >= cut) {
+      const int w = atomicAdd(&s_kept[slot_q], 1);
+      if (w < A.cap) { out[w] = ref; out_s[w] = sv; }
+    }
   }
+  G.sync();                                          // the kept pairs are visible to the group
+  int total = s_kept[slot_q];
+  ovf = total > A.cap;
   if (!ovf && total > K) {
     const float qe = A.qe[q], qn = A.qn[q];
-    n = 0;
-    __syncwarp();
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int p = p0 + lane;
-      float lo = -INFINITY, hi;
-      if (p < total) tight_bounds(A, out_s[p], out[p], Nq, qe, qn, lo, hi);
-      const unsigned m = __ballot_sync(0xffffffffu, p < total && (n < K || lo > lst[K - 1]));
-      if (m) warp_insert_desc_tc(lst, K, n, m, lo, lane);
+    for (int p = rank; p < total; p += nt) {
+      float lo, hi;
+      tight_bounds(A, out_s[p], out[p], Nq, qe, qn, lo, hi);
+      keys[p] = fkey(fmaxf(lo, -INFINITY));          // NaN: no lower bound
     }
-    const float T2 = (n == K) ? lst[K - 1] : -INFINITY;
+    G.sync();
+    const float T2 = fkey_value(kth::largest<WPQ>(G, keys, total, K));
     const float cut2 = dense_cut(fmaxf(T, T2));
-    int kept = 0;
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int p = p0 + lane;
+    if (rank == 0) s_kept[slot_q] = 0;
+    G.sync();
+    for (int p0 = 0; p0 < total; p0 += nt) {
+      const int p = p0 + rank;
       bool keep = false;
       int32_t ref = 0;
       float sv = 0.f;
@@ -728,15 +751,17 @@ __global__ void k_tc_merge(MergeArgs A) {
         tight_bounds(A, sv, ref, Nq, qe, qn, lo, hi);
         keep = hi >= cut2;
       }
-      const unsigned m = __ballot_sync(0xffffffffu, keep);   // every lane has read slot p first
-      const int rank = __popc(m & ((1u << lane) - 1u));
-      if (keep) { out[kept + rank] = ref; out_s[kept + rank] = sv; }
-      kept += __popc(m);
-      __syncwarp();
+      G.sync();                                      // every slot of this round is read before one is written
+      if (keep) {
+        const int w = atomicAdd(&s_kept[slot_q], 1);
+        out[w] = ref;
+        out_s[w] = sv;
+      }
     }
-    total = kept;
+    G.sync();
+    total = s_kept[slot_q];
   }
-  if (lane == 0) { A.count[ql] = ovf ? 0 : total; A.over[ql] = ovf ? 1 : 0; }
+  if (rank == 0) { A.count[ql] = ovf ? 0 : total; A.over[ql] = ovf ? 1 : 0; }
 }
 
 __global__ void k_tc_key_init(int64_t nq, unsigned* keys) {
@@ -912,7 +937,15 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     M.re = (method == COSINE) ? D->ue : D->xe; M.rn = (method == COSINE) ? D->un : D->xn;
     M.qe = (method == COSINE) ? Q->ue : Q->xe; M.qn = (method == COSINE) ? Q->un : Q->xn;
     M.cap = cap; M.cand = cand; M.cand_s = cand_s; M.count = count; M.over = over;
-    k_tc_merge<<<(unsigned)((nq + MW - 1) / MW), MW * 32, 0, s>>>(M);
+    M.smem_query = merge_prefix_bytes(nslots) + (size_t)std::max<int64_t>(nslots * k, cap) * 4;
+    M.smem_query = (M.smem_query + 15) / 16 * 16;
+    const bool narrow = nq >= MERGE_WIDE_MAX && M.smem_query * 8 <= 220 * 1024;
+    const bool widest = nq <= MERGE_WIDEST_MAX;
+    auto mk = narrow ? k_tc_merge<1> : widest ? k_tc_merge<32> : k_tc_merge<8>;
+    const size_t msm = M.smem_query * (narrow ? 8 : 1);
+    if (msm > 48 * 1024) chk(cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm));
+    if (e == cudaSuccess)
+      mk<<<(unsigned)(narrow ? (nq + 7) / 8 : nq), widest ? 1024 : 256, msm, s>>>(M);
     chk(cudaGetLastError());
   }
   // stream-ordered frees: the caller reads *status with its own results
