@@ -21,8 +21,15 @@ struct ScreenCache {
   float* fxl = nullptr;      // js: per stored entry, x log x of the value (FP32)
   float* cnorm = nullptr;    // per column: norm term of the method (js: sum of |x log x| + x, rounded up)
   int32_t* nnz = nullptr;    // per column: stored entries
-  int32_t* perm = nullptr;   // columns in descending-nnz order
   int64_t nnz_total = 0;
+  // the entries in row order, built by the first FP32 screen against the
+  // matrix (see k_rows_fill in sdg_screen.cu): (column, value) pairs and js's x
+  // log x, in cells of 2^sub_lg columns, nsub cells a row
+  uint32_t* rows = nullptr;  // [nrow * nsub + 1] cell offsets
+  void* ent = nullptr;       // int2[nnz]
+  float* exl = nullptr;      // js: [nnz]
+  int32_t nsub = 0;
+  int sub_lg = 0;
   // js / pearson / covariance: every nonzero stored value lies in the range
   // the method's FP32 bound is derived for ([2^-100, 2^100] for js, |value| in
   // [2^-50, 2^50] for the moment methods); else the searches of this matrix
