@@ -667,28 +667,6 @@ __global__ void k_self_diag(int method, int dist, DevCsc m, ColAux a, int diag, 
   D[r * m.ncol + r] = v;
 }
 
-__global__ void k_exact_pairs(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry,
-                              ColAux qa, const int32_t* ref_idx, const int32_t* qry_idx,
-                              int64_t npairs, double* out) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= npairs) return;
-  out[t] = pair_value(method, dist != 0, ref, ra, ref_idx[t], qry, qa, qry_idx[t]);
-}
-
-// Candidate pairs of the screened engine: slots with ref_idx < 0 are unused;
-// with restore_self the self pair (ref == query) takes self_value.
-__global__ void k_exact_pairs_sparse(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry,
-                                     ColAux qa, const int32_t* ref_idx, const int32_t* qry_idx,
-                                     int64_t npairs, int restore_self, double self_value,
-                                     double* out) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= npairs) return;
-  const int32_t c = ref_idx[t], q = qry_idx[t];
-  if (c < 0 || q < 0) return;
-  out[t] = (restore_self && c == q) ? self_value
-                                    : pair_value(method, dist != 0, ref, ra, c, qry, qa, q);
-}
-
 // The value of a match-only pair from the ascending-row sum of matched
 // products (`sum`) and the matched-row count (`common`): Jaccard
 // (jacc_value, src/sparseDist.cpp:549-556), cosine (unit_cosine's NaN / clamp,
@@ -723,127 +701,337 @@ __device__ double match_finish(int method, bool dist, double sum, int64_t common
   return dist ? dsub(1.0, c) : c;
 }
 
-// Match-only methods (binary, cosine, pearson): the value depends on the rows
-// both columns store, summed in ascending row order.  One warp per query row
-// of the candidate table: for each candidate, lanes take 32 consecutive
-// entries of the shorter column and binary-search them in the longer one; the
-// matched products are then added by lane 0 in ascending row order, so the sum
-// is the reference's sequential sum bit for bit.
-__device__ double warp_match_value(int method, bool dist, const DevCsc& A, const ColAux& aa,
-                                   int32_t i, const DevCsc& B, const ColAux& ba, int32_t j,
-                                   int lane) {
-  const int64_t ia0 = A.p[i], ia1 = A.p[i + 1], jb0 = B.p[j], jb1 = B.p[j + 1];
-  if (method == COSINE) {
-    const bool ea = (aa.scale[i] == 0.0), eb = (ba.scale[j] == 0.0);
-    if (ea || eb) { const double c = (ea && eb) ? 1.0 : 0.0; return dist ? dsub(1.0, c) : c; }
-  }
-  const bool a_short = (ia1 - ia0) <= (jb1 - jb0);
-  const int32_t* si = a_short ? A.i : B.i;
-  const int32_t* li = a_short ? B.i : A.i;
-  const int64_t s0 = a_short ? ia0 : jb0, s1 = a_short ? ia1 : jb1;
-  int64_t l0 = a_short ? jb0 : ia0;
-  const int64_t l1 = a_short ? jb1 : ia1;
-  const double* av = (method == COSINE) ? aa.uval : A.x;
-  const double* bv = (method == COSINE) ? ba.uval : B.x;
-  double sum = 0.0;
-  int64_t common = 0;
-  for (int64_t c0 = s0; c0 < s1 && l0 < l1; c0 += 32) {
-    const int64_t s = c0 + lane;
-    bool hit = false;
-    double prod = 0.0;
-    int64_t lb = l1;
-    if (s < s1) {
-      const int32_t r = __ldg(si + s);
-      int64_t lo = l0, hi = l1;                        // first index with row >= r
-      while (lo < hi) { const int64_t mid = (lo + hi) >> 1; if (__ldg(li + mid) < r) lo = mid + 1; else hi = mid; }
-      lb = lo;
-      if (lo < l1 && __ldg(li + lo) == r) {
-        hit = true;
-        if (method != BINARY) {
-          const int64_t ea_ = a_short ? s : lo, eb_ = a_short ? lo : s;
-          prod = dmul(av[ea_], bv[eb_]);
-        }
-      }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    common += __popc(m);
-    if (method != BINARY) {
-      for (int t = 0; t < 32; ++t) {
-        const double p = __shfl_sync(0xffffffffu, prod, t);
-        if ((m >> t) & 1u) sum = dadd(sum, p);
-      }
-    }
-    l0 = __shfl_sync(0xffffffffu, lb, 31);
-  }
-  return match_finish(method, dist, sum, common, A, aa, i, B, ba, j);
-}
+// ---- exact values of the screens' candidates ---------------------------------
+//
+// GB300's FP64 pipe holds a warp's instruction for 64 cycles whatever its
+// active lanes and whether or not the next one depends on it (19 cycles of an
+// SM with all four schedulers), so FP64 warp instructions are what counts: a
+// pair's sequential sum (one dadd per row, in ascending row order, as the
+// reference adds them) runs one pair per LANE of one warp, and the terms of the
+// sums are formed 32 at a time.
+//
+// A CTA takes one query of the candidate table, 32 candidates at a time.  Warps
+// 1 .. produce: for each candidate in turn a warp streams the column,
+// coalesced, and writes the next (at most RM) terms of its sum, in row order,
+// to the candidate's list in shared memory.  Warp 0 adds: lane j runs candidate
+// j's list of the pass before, so producing and adding overlap; one block
+// barrier a pass.  Each lane's sum is the reference's sequential sum bit for bit.
+//
+// The query's rows are a shared-memory bitmap (bit r % 32 of word r / 32) with
+// each word's count of entries before it, so rank(r) = base[r / 32] + popc(word
+// & below(r)) query entries lie below row r.
+//
+// Products (cosine, pearson, covariance) and js need the matched rows: the
+// matched values are compacted first and the terms (dmul; js_shared_term) formed
+// from the compacted lists.  Manhattan and euclidean need the union of the
+// rows: candidate entry i is term i + rank(r_i) - (shared rows before it), and
+// the terms between two candidate entries are query entries; a lane finds its
+// term's place by a binary search over the 32 loaded entries.
+//
+// Before: products, eight warps a query with three candidates each in its
+// lanes, 4.26 ms for 4,096 queries of 30,000 log-count columns; manhattan, a
+// thread per pair walking both columns in global memory, 5.29 ms for 1,000 of
+// 20,000.  One warp a query, reading and adding in turn: 5.56 and 3.84 ms (the
+// longest columns outlast the rest).  As it is: 1.55 and 0.97 ms, of which the
+// FP64 pipe is busy a quarter; the rest is the producers' instructions and the
+// passes' barriers.
+constexpr int RR_MAX_WARPS = 8;
 
-__global__ void k_rerank_warp(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry, ColAux qa,
-                              const int32_t* cand, const int32_t* count, int cap, int64_t nq_local,
-                              int64_t q_begin, int restore_self, double self_value, double* out) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ql = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp;
-  if (ql >= nq_local) return;
+// KIND 0: binary (counts), 1: products, 2: js, 3: manhattan, 4: euclidean; RM:
+// list slots per candidate per pass
+template <int KIND, int RM>
+__global__ void __launch_bounds__(RR_MAX_WARPS * 32) k_rerank(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry,
+                                                              ColAux qa, const int32_t* cand, const int32_t* count,
+                                                              int cap, int64_t q_begin, int restore_self,
+                                                              double self_value, double* out) {
+  constexpr int LD = RM + 1;
+  constexpr int LISTS = KIND == 0 ? 0 : KIND == 2 ? 3 : 1;    // js: terms, reference values, query values
+  extern __shared__ __align__(16) unsigned char rr_smem[];
+  __shared__ int64_t s_pos[32], s_end[32];                     // the candidates' columns still to read
+  __shared__ int32_t s_b[32];                                  // union: query entries consumed
+  __shared__ int32_t s_fill[2][32];
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int W = (qry.nrow + 31) >> 5;
+  double* lists = reinterpret_cast<double*>(rr_smem);          // [2][LISTS][32][LD]
+  double* stage = lists + (size_t)2 * LISTS * 32 * LD + (size_t)warp * RM;     // KIND 1, 3, 4
+  uint32_t* bits = reinterpret_cast<uint32_t*>(lists + (size_t)2 * LISTS * 32 * LD +
+                                               (KIND == 1 || KIND >= 3 ? (size_t)nw * RM : 0));
+  int32_t* base = reinterpret_cast<int32_t*>(bits + W);
+  int32_t* su = base + W + warp * 64;                          // union: the loaded entries' terms and ranks
+  const int64_t ql = blockIdx.x;
   const int32_t q = (int32_t)(q_begin + ql);
   const int n = count[ql];
-  for (int t = 0; t < n; ++t) {
-    const int32_t c = cand[ql * cap + t];
-    double v;
-    if (restore_self && c == q) v = self_value;
-    else v = warp_match_value(method, dist != 0, ref, ra, c, qry, qa, q, lane);
-    if (lane == 0) out[ql * cap + t] = v;
+  if (n == 0) return;
+  const int64_t qb = qry.p[q];
+  const int32_t nq = (int32_t)(qry.p[q + 1] - qb);
+  for (int w = threadIdx.x; w < W; w += blockDim.x) bits[w] = 0u;
+  __syncthreads();
+  for (int32_t e = threadIdx.x; e < nq; e += blockDim.x) {
+    const int32_t r = __ldg(qry.i + qb + e);
+    atomicOr(bits + (r >> 5), 1u << (r & 31));
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int32_t run = 0;
+    for (int w0 = 0; w0 < W; w0 += 32) {
+      const int32_t own = w0 + lane < W ? __popc(bits[w0 + lane]) : 0;
+      int32_t x = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (w0 + lane < W) base[w0 + lane] = run + x - own;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  const double* qv = ((method == COSINE) ? qa.uval : qry.x) + qb;
+  const double* qxl = KIND == 2 ? qa.xl + qb : nullptr;
+  const double* rv = (method == COSINE) ? ra.uval : ref.x;
+  const unsigned below = (1u << lane) - 1u;
+  const bool q_empty = (method == COSINE) && qa.scale[q] == 0.0;
+  for (int g = 0; g < n; g += 32) {
+    const int ng = min(32, n - g);
+    // warp 0, lane j: candidate g + j and its sums
+    int32_t c = -1;
+    double v = 0.0, sum = 0.0, sp = 0.0, sq = 0.0;
+    bool special = false;
+    __syncthreads();                                   // the last group's state and the tables
+    if (warp == 0) {
+      int64_t a = 0, a_end = 0;
+      int32_t b = nq;
+      if (lane < ng) {
+        c = cand[ql * (int64_t)cap + g + lane];
+        if (restore_self && c == q) {
+          v = self_value;
+          special = true;
+        } else if (method == COSINE && (q_empty || ra.scale[c] == 0.0)) {
+          const double cv = (q_empty && ra.scale[c] == 0.0) ? 1.0 : 0.0;
+          v = dist ? dsub(1.0, cv) : cv;
+          special = true;
+        } else {
+          a = ref.p[c];
+          a_end = ref.p[c + 1];
+          b = 0;
+        }
+      }
+      s_pos[lane] = a;
+      s_end[lane] = a_end;
+      s_b[lane] = b;
+    }
+    __syncthreads();
+    if (KIND == 0) {
+      // matched rows counted by every warp
+      for (int j = warp; j < ng; j += nw) {
+        int64_t common = 0;
+        for (int64_t p = s_pos[j]; p < s_end[j]; p += 128) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int64_t e = p + 32 * u + lane;
+            const int32_t r = e < s_end[j] ? __ldg(ref.i + e) : -1;
+            const bool hit = r >= 0 && ((bits[r >> 5] >> (r & 31)) & 1u);
+            common += __popc(__ballot_sync(0xffffffffu, hit));
+          }
+        }
+        if (lane == 0) s_fill[0][j] = (int32_t)common;
+      }
+      __syncthreads();
+      if (warp == 0 && lane < ng) {
+        if (!special) v = match_finish(method, dist != 0, 0.0, s_fill[0][lane], ref, ra, c, qry, qa, q);
+        out[ql * (int64_t)cap + g + lane] = v;
+      }
+      continue;
+    }
+    for (int pass = 0;; ++pass) {
+      bool produced = false;
+      double* L = lists + (size_t)(pass & 1) * LISTS * 32 * LD;
+      if (warp > 0) {
+        for (int j = warp - 1; j < ng; j += nw - 1) {
+          int64_t pos = s_pos[j];
+          const int64_t end = s_end[j];
+          double* lj = L + j * LD;
+          int fill = 0;
+          if constexpr (KIND <= 2) {
+            double* wp = lj + 32 * LD;
+            double* wq = wp + 32 * LD;
+            bool full = false;
+            while (pos < end && !full) {
+              int32_t r[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int64_t e = pos + 32 * u + lane;
+                r[u] = (e < end) ? __ldg(ref.i + e) : -1;
+              }
+              int qe[4];
+              unsigned m[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                qe[u] = -1;
+                if (r[u] >= 0) {
+                  const uint32_t wd = bits[r[u] >> 5], bit = 1u << (r[u] & 31);
+                  if (wd & bit) qe[u] = base[r[u] >> 5] + __popc(wd & (bit - 1u));
+                }
+                m[u] = __ballot_sync(0xffffffffu, qe[u] >= 0);
+              }
+              // the rounds whose matches still fit, then their values
+              int at[4], rounds = 0;
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                at[u] = -1;
+                if (!full && pos + 32 * u < end) {
+                  const int cnt = __popc(m[u]);
+                  if (fill + cnt > RM) {
+                    full = true;
+                  } else {
+                    if (qe[u] >= 0) at[u] = fill + __popc(m[u] & below);
+                    fill += cnt;
+                    rounds = u + 1;
+                  }
+                }
+              }
+              double pv[4], pq[4], px[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                if (at[u] >= 0) {
+                  pv[u] = __ldg(rv + pos + 32 * u + lane);
+                  pq[u] = __ldg(qv + qe[u]);
+                  if (KIND == 2) px[u] = dadd(__ldg(ra.xl + pos + 32 * u + lane), __ldg(qxl + qe[u]));
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                if (at[u] >= 0) {
+                  if (KIND == 1) {
+                    lj[at[u]] = pv[u];
+                    stage[at[u]] = pq[u];
+                  } else {
+                    lj[at[u]] = px[u];
+                    wp[at[u]] = pv[u];
+                    wq[at[u]] = pq[u];
+                  }
+                }
+              }
+              pos += 32 * rounds;
+            }
+            if (pos > end) pos = end;
+            __syncwarp();
+            for (int i = lane; i < fill; i += 32) {
+              if (KIND == 1) {
+                lj[i] = dmul(lj[i], stage[i]);
+              } else {                                 // js_shared_term
+                const double PQ = dadd(wp[i], wq[i]);
+                lj[i] = dadd(dsub(lj[i], xlogx(PQ)), dmul(PQ, 0.69314718055994530942));
+              }
+            }
+          } else {
+            int32_t b = s_b[j];
+            while (fill < RM && (pos < end || b < nq)) {
+              const bool valid = pos + lane < end;
+              const int32_t r = valid ? __ldg(ref.i + pos + lane) : 0;
+              const double av = valid ? __ldg(ref.x + pos + lane) : 0.0;
+              int32_t rank = nq;
+              bool shared = false;
+              if (valid) {
+                const uint32_t wd = bits[r >> 5], bit = 1u << (r & 31);
+                rank = base[r >> 5] + __popc(wd & (bit - 1u));
+                shared = (wd & bit) != 0u;
+              }
+              const unsigned sm = __ballot_sync(0xffffffffu, shared);
+              const int nvalid = (int)(end - pos < 32 ? end - pos : 32);
+              // terms left when this chunk ends the column
+              const int total = nvalid + (nq - b) - __popc(sm);
+              const int u = valid ? lane + (rank - b) - __popc(sm & below) : total;
+              const int avail = (end - pos > 32) ? __shfl_sync(0xffffffffu, u, 31) + 1 : total;
+              const int take = min(avail, RM - fill);
+              su[lane] = u;
+              su[32 + lane] = rank;
+              stage[lane] = av;
+              __syncwarp();
+              for (int o = lane; o < take; o += 32) {
+                int lo = 0, hi = 32;                   // the first loaded entry at or after term o
+                while (lo < hi) {
+                  const int mid = (lo + hi) >> 1;
+                  if (su[mid] >= o) hi = mid;
+                  else lo = mid + 1;
+                }
+                double x;
+                if (lo < nvalid && su[lo] == o) {
+                  x = stage[lo];
+                  // an FP64 instruction only where some lane's row is shared
+                  if ((sm >> lo) & 1u) x = dsub(x, __ldg(qv + su[32 + lo]));
+                } else {
+                  x = __ldg(qv + (lo < nvalid ? su[32 + lo] - (su[lo] - o) : nq - (total - o)));
+                }
+                lj[fill + o] = KIND == 4 ? dmul(x, x) : fabs(x);
+              }
+              const unsigned cm = __ballot_sync(0xffffffffu, valid && u < take);
+              pos += __popc(cm);
+              b += take - __popc(cm) + __popc(cm & sm);
+              fill += take;
+              __syncwarp();
+            }
+            if (lane == 0) s_b[j] = b;
+          }
+          if (lane == 0) { s_pos[j] = pos; s_fill[pass & 1][j] = fill; }
+          if (fill > 0) produced = true;
+        }
+      } else if (pass > 0) {
+        const double* P = lists + (size_t)((pass - 1) & 1) * LISTS * 32 * LD + lane * LD;
+        const int fill = lane < ng ? s_fill[(pass - 1) & 1][lane] : 0;
+        const int mx = __reduce_max_sync(0xffffffffu, fill);
+#pragma unroll 4
+        for (int t = 0; t < mx; ++t) {
+          if (t < fill) {
+            sum = dadd(sum, P[t]);
+            if (KIND == 2) {
+              sp = dadd(sp, P[32 * LD + t]);
+              sq = dadd(sq, P[2 * 32 * LD + t]);
+            }
+          }
+        }
+      }
+      if (!__syncthreads_or(produced)) break;
+    }
+    if (warp == 0 && lane < ng) {
+      if (!special) {
+        if (KIND == 1) v = match_finish(method, dist != 0, sum, 0, ref, ra, c, qry, qa, q);
+        else if (KIND == 2) { if (!js_bulk(ra.xsum[c], qa.xsum[q], sp, sq, sum, &v)) v = pair_js_walk(ref, ra, c, qry, qa, q); }
+        else v = KIND == 4 ? sqrt(sum) : sum;
+      }
+      out[ql * (int64_t)cap + g + lane] = v;
+    }
   }
 }
 
-// Query-centric re-rank of the match-only methods, one CTA per query row of
-// the candidate table.  The query column's rows go into a shared-memory
-// bitmap (bit r % 32 of word r / 32) with, for each word holding a row, the
-// index of its first entry, so a matched row r is entry
-// first[r / 32] + popc(word & below(r)) of the query; the query's values sit
-// in shared memory too (up to RQ_MAX_QV entries, else they are read from
-// global memory).  The candidates are sorted by column length (bitonic, in
-// shared memory) and dealt round-robin to the warps' lanes.
-//
-// GB300's FP64 pipe spends the same time on an FP64 warp instruction whatever
-// the number of active lanes, so the sequential sum of a pair (one dadd per
-// matched row, in ascending row order, as the reference adds them) runs one
-// pair per LANE.  A warp works on its 32 candidates in passes: (scan) for
-// each candidate in turn, the warp streams the column 32 entries a round
-// (coalesced, four rounds' loads in flight), tests the rows against the
-// bitmap, multiplies the matched values (dmul, the same product the
-// reference forms) and appends the products, in row order, to that
-// candidate's list of RM slots until it is full or the column ends; (sum)
-// lane j then adds candidate j's list in order, all lanes at once, operands
-// in shared memory.  Each lane's sum is the reference's sequential sum bit for
-// bit.
-//
-// kTri (the single-matrix sparseDist): no candidate table; CTA (x, y) takes
-// column q = x of m as the query and the reference columns c = y * 2048 ..
-// of m below it (c < q) as its candidates, in the reference's orientation
-// (first operand c, second q), and writes the strict upper triangle entry
-// out[q * ncol + c].
+// The single-matrix sparseDist of the match-only methods: CTA (x, y) takes
+// column q = x of m as the query and the reference columns c = y * 2048 .. of m
+// below it (c < q) as its candidates, in the reference's orientation (first
+// operand c, second q), and writes the strict upper triangle entry out[q *
+// ncol + c].  The candidates are sorted by column length (bitonic, in shared
+// memory) and dealt round-robin to the lanes of eight warps.  A
+// warp works in passes: it streams each of its candidates in turn, appends the
+// matched products in row order to the candidate's list until that is full,
+// then lane j adds candidate j's list.  The query's values sit in shared memory
+// (up to RQ_MAX_QV entries, else global).
+constexpr int RM = 32;                // list slots per candidate per pass
+constexpr int RLD = RM + 1;           // their stride: the lanes' list reads fall on different banks
 constexpr int RQ_THREADS = 256;
 constexpr int RQ_WARPS = RQ_THREADS / 32;
 constexpr int32_t RQ_MAX_NROW = 1 << 18;
 constexpr int RQ_MAX_QV = 2048;
 constexpr int RQ_MAX_CAND = 2048;     // candidates sorted in shared memory
-constexpr int RM = 32;                // list slots per candidate per pass
 
-template <bool kTri>
-__global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry, ColAux qa,
-                           const int32_t* cand, const int32_t* count, int cap, int64_t q_begin,
-                           int restore_self, double self_value, double* out) {
+__global__ void k_self_tri(int method, int dist, DevCsc m, ColAux aux, double* out) {
   extern __shared__ __align__(16) uint32_t rq_smem[];
-  const int W = (qry.nrow + 31) >> 5;
+  const int W = (m.nrow + 31) >> 5;
   double* qvs = reinterpret_cast<double*>(rq_smem);                          // RQ_MAX_QV
   uint64_t* order = reinterpret_cast<uint64_t*>(rq_smem + 2 * RQ_MAX_QV);    // RQ_MAX_CAND
-  double* lists = reinterpret_cast<double*>(order + RQ_MAX_CAND);           // [warp][32][RM]
-  uint32_t* bits = reinterpret_cast<uint32_t*>(lists + RQ_WARPS * 32 * RM);
+  double* lists = reinterpret_cast<double*>(order + RQ_MAX_CAND);           // [warp][32][RLD]
+  uint32_t* bits = reinterpret_cast<uint32_t*>(lists + RQ_WARPS * 32 * RLD);
   int32_t* first = reinterpret_cast<int32_t*>(bits + W);
-  const int64_t ql = blockIdx.x;
-  const int32_t q = (int32_t)(q_begin + ql);
-  const int32_t cbase = kTri ? (int32_t)blockIdx.y * RQ_MAX_CAND : 0;
-  const int n = kTri ? max(0, min(q - cbase, RQ_MAX_CAND)) : min(count[ql], RQ_MAX_CAND);
+  const int32_t q = (int32_t)blockIdx.x;
+  const int32_t cbase = (int32_t)blockIdx.y * RQ_MAX_CAND;
+  const int n = max(0, min(q - cbase, RQ_MAX_CAND));
   if (n == 0) return;
   for (int w = threadIdx.x; w < W; w += blockDim.x) bits[w] = 0u;
   // sort keys: (column length, position in the list), longest first
@@ -852,21 +1040,21 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
   for (int t = threadIdx.x; t < np2; t += blockDim.x) {
     uint64_t key = 0;                       // padding sorts last
     if (t < n) {
-      const int32_t c = kTri ? cbase + t : cand[ql * (int64_t)cap + t];
-      const int64_t len64 = ref.p[c + 1] - ref.p[c];
+      const int32_t c = cbase + t;
+      const int64_t len64 = m.p[c + 1] - m.p[c];
       const uint32_t len = (uint32_t)(len64 < 0x7fffffff ? len64 : 0x7fffffff);
       key = ((uint64_t)(len + 1u) << 32) | (uint32_t)t;
     }
     order[t] = key;
   }
   __syncthreads();
-  const int64_t q0 = qry.p[q], q1 = qry.p[q + 1];
-  const double* qsrc = ((method == COSINE) ? qa.uval : qry.x) + q0;
+  const int64_t q0 = m.p[q], q1 = m.p[q + 1];
+  const double* qsrc = ((method == COSINE) ? aux.uval : m.x) + q0;
   const bool qv_shared = (q1 - q0) <= RQ_MAX_QV;
   for (int64_t e = q0 + threadIdx.x; e < q1; e += blockDim.x) {
-    const int32_t r = qry.i[e];
+    const int32_t r = m.i[e];
     atomicOr(&bits[r >> 5], 1u << (r & 31));
-    if (e == q0 || (qry.i[e - 1] >> 5) != (r >> 5)) first[r >> 5] = (int32_t)(e - q0);
+    if (e == q0 || (m.i[e - 1] >> 5) != (r >> 5)) first[r >> 5] = (int32_t)(e - q0);
     if (qv_shared && method != BINARY) qvs[e - q0] = qsrc[e - q0];
   }
   for (int k2 = 2; k2 <= np2; k2 <<= 1) {             // bitonic sort, descending
@@ -886,9 +1074,9 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
   const double* qv = qv_shared ? qvs : qsrc;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  const double* rv = (method == COSINE) ? ra.uval : ref.x;
-  const bool q_empty = (method == COSINE) && qa.scale[q] == 0.0;
-  double* wl = lists + warp * 32 * RM;
+  const double* rv = (method == COSINE) ? aux.uval : m.x;
+  const bool q_empty = (method == COSINE) && aux.scale[q] == 0.0;
+  double* wl = lists + warp * 32 * RLD;
   for (int g = 0; g < n; g += RQ_WARPS * 32) {
     // lane j of warp w owns sorted candidate g + 8 j + w: the candidates are
     // dealt round-robin, so every warp gets work even for short lists
@@ -899,17 +1087,14 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
     bool special = false;
     int64_t a = 0, a_end = 0, c0 = 0;
     if (t >= 0) {
-      c = kTri ? cbase + t : cand[ql * (int64_t)cap + t];
-      if (restore_self && c == q) {
-        v = self_value;
-        special = true;
-      } else if (method == COSINE && (q_empty || ra.scale[c] == 0.0)) {
-        const double cv = (q_empty && ra.scale[c] == 0.0) ? 1.0 : 0.0;
+      c = cbase + t;
+      if (method == COSINE && (q_empty || aux.scale[c] == 0.0)) {
+        const double cv = (q_empty && aux.scale[c] == 0.0) ? 1.0 : 0.0;
         v = dist ? dsub(1.0, cv) : cv;
         special = true;
       } else {
-        c0 = a = ref.p[c];
-        a_end = ref.p[c + 1];
+        c0 = a = m.p[c];
+        a_end = m.p[c + 1];
       }
     }
     bool active = (t >= 0) && !special && a < a_end;
@@ -922,7 +1107,7 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
         if (!__shfl_sync(0xffffffffu, active, j)) continue;
         int64_t pos = __shfl_sync(0xffffffffu, a, j);
         const int64_t end = __shfl_sync(0xffffffffu, a_end, j);
-        double* lj = wl + j * RM;
+        double* lj = wl + j * RLD;
         int fill = 0;
         bool full = false;
         while (pos < end && !full) {
@@ -930,7 +1115,7 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int64_t e = pos + 32 * u + lane;
-            r[u] = (e < end) ? __ldg(ref.i + e) : -1;
+            r[u] = (e < end) ? __ldg(m.i + e) : -1;
           }
           int qe[4];
 #pragma unroll
@@ -953,11 +1138,11 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
           for (int u = 0; u < 4; ++u) {
             if (full || pos >= end) break;
             const bool hit = qe[u] >= 0;
-            const unsigned m = __ballot_sync(0xffffffffu, hit);
-            const int cnt = __popc(m);
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            const int cnt = __popc(hits);
             if (method != BINARY) {
               if (fill + cnt > RM) { full = true; break; }
-              if (hit) lj[fill + __popc(m & below)] = pv[u];
+              if (hit) lj[fill + __popc(hits & below)] = pv[u];
             }
             fill += cnt;
             pos += 32;
@@ -974,16 +1159,15 @@ __global__ void k_rerank_q(int method, int dist, DevCsc ref, ColAux ra, DevCsc q
       // sum: lane j runs candidate j's list in order
       if (method != BINARY) {
         const int mx = __reduce_max_sync(0xffffffffu, my_fill);
-        const double* ll = wl + lane * RM;
+        const double* ll = wl + lane * RLD;
         for (int s2 = 0; s2 < mx; ++s2)
           if (s2 < my_fill) sum = dadd(sum, ll[s2]);
       }
       __syncwarp();
     }
     if (t >= 0) {
-      if (!special) v = match_finish(method, dist != 0, sum, common, ref, ra, c, qry, qa, q);
-      if (kTri) out[(int64_t)q * ref.ncol + c] = v;
-      else out[ql * (int64_t)cap + t] = v;
+      if (!special) v = match_finish(method, dist != 0, sum, common, m, aux, c, m, aux, q);
+      out[(int64_t)q * m.ncol + c] = v;
     }
   }
 }
@@ -1167,13 +1351,12 @@ void launch_self_tri(int method, int dist, const DevCsc& m, const ColAux& a, int
   const int64_t n = m.ncol;
   if (n == 0) return;
   if (n > 1) {
-    const size_t smem = (size_t)RQ_MAX_QV * 8 + (size_t)RQ_MAX_CAND * 8 + (size_t)RQ_WARPS * 32 * RM * 8 +
+    const size_t smem = (size_t)RQ_MAX_QV * 8 + (size_t)RQ_MAX_CAND * 8 + (size_t)RQ_WARPS * 32 * RLD * 8 +
                         (size_t)((m.nrow + 31) / 32) * 8;
     if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_rerank_q<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_self_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const unsigned chunks = (unsigned)((n - 1 + RQ_MAX_CAND - 1) / RQ_MAX_CAND);
-    k_rerank_q<true><<<dim3((unsigned)n, chunks), RQ_THREADS, smem, s>>>(method, dist, m, a, m, a, nullptr,
-                                                                        nullptr, 0, 0, 0, 0.0, D);
+    k_self_tri<<<dim3((unsigned)n, chunks), RQ_THREADS, smem, s>>>(method, dist, m, a, D);
   }
   k_self_diag<<<blocks_for(n, 256), 256, 0, s>>>(method, dist, m, a, diag, D);
 }
@@ -1192,44 +1375,27 @@ void launch_mirror_lower(double* D, int64_t n, cudaStream_t s) {
   k_mirror_lower<<<dim3(T, T), dim3(32, 8), 0, s>>>(D, n);
 }
 
-void launch_exact_pairs(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                        const DevCsc& qry, const ColAux& qa, const int32_t* ref_idx,
-                        const int32_t* qry_idx, int64_t npairs, double* out, cudaStream_t s) {
-  if (npairs > 0)
-    k_exact_pairs<<<blocks_for(npairs, 128), 128, 0, s>>>(method, dist, ref, ra, qry, qa,
-                                                           ref_idx, qry_idx, npairs, out);
-}
-
-bool rerank_warp_supported(int method) {
-  return method == BINARY || method == COSINE || method == PEARSON;
-}
-
-void launch_rerank_warp(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                        const DevCsc& qry, const ColAux& qa, const int32_t* cand,
-                        const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
-                        int restore_self, double self_value, double* out, cudaStream_t s) {
-  if (nq_local <= 0) return;
-  if (qry.nrow <= RQ_MAX_NROW && cap <= RQ_MAX_CAND) {
-    const size_t smem = (size_t)RQ_MAX_QV * 8 + (size_t)RQ_MAX_CAND * 8 + (size_t)RQ_WARPS * 32 * RM * 8 +
-                        (size_t)((qry.nrow + 31) / 32) * 8;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_rerank_q<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_rerank_q<false><<<(unsigned)nq_local, RQ_THREADS, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap,
-                                                           q_begin, restore_self, self_value, out);
-  } else {
-    k_rerank_warp<<<blocks_for(nq_local, 8), 256, 0, s>>>(method, dist, ref, ra, qry, qa, cand,
-                                                          count, cap, nq_local, q_begin,
-                                                          restore_self, self_value, out);
+int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, const DevCsc& qry, const ColAux& qa,
+                  const int32_t* cand, const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
+                  int restore_self, double self_value, double* out, double mean_nnz, cudaStream_t s) {
+  if (nq_local <= 0) return 0;
+  const int kind = method == BINARY ? 0 : method == JS ? 2 : method == MANHATTAN ? 3 : method == EUCLIDEAN ? 4 : 1;
+  // eight warps (products, 4,096 queries of 30,000 log-count columns: 1.55 ms
+  // where five take 1.92 and sixteen 1.76); counts of short columns have less
+  // to stream than a wide block costs
+  const int nw = kind != 0 || mean_nnz > 256.0 ? RR_MAX_WARPS : mean_nnz > 64.0 ? 5 : 3;
+  const int rm = kind == 2 ? 32 : 64, lists = kind == 0 ? 0 : kind == 2 ? 3 : 1;
+  const size_t smem = (size_t)2 * lists * 32 * (rm + 1) * 8 + (kind == 1 || kind >= 3 ? (size_t)nw * rm * 8 : 0) +
+                      (size_t)((qry.nrow + 31) / 32) * 8 + (kind >= 3 ? (size_t)nw * 64 * 4 : 0);
+  auto k = kind == 0 ? k_rerank<0, 64> : kind == 1 ? k_rerank<1, 64> : kind == 2 ? k_rerank<2, 32>
+         : kind == 3 ? k_rerank<3, 64> : k_rerank<4, 64>;
+  if (smem > 40 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
   }
-}
-
-void launch_exact_pairs_sparse(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                               const DevCsc& qry, const ColAux& qa, const int32_t* ref_idx,
-                               const int32_t* qry_idx, int64_t npairs, int restore_self,
-                               double self_value, double* out, cudaStream_t s) {
-  if (npairs > 0)
-    k_exact_pairs_sparse<<<blocks_for(npairs, 128), 128, 0, s>>>(
-        method, dist, ref, ra, qry, qa, ref_idx, qry_idx, npairs, restore_self, self_value, out);
+  k<<<(unsigned)nq_local, nw * 32, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin, restore_self,
+                                              self_value, out);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace sdg

@@ -74,26 +74,13 @@ void launch_self_tri(int method, int dist, const DevCsc& m, const ColAux& a, int
 // upper triangle is zeroed after it is read.
 void launch_mirror_upper(double* D, int64_t n, int clear, cudaStream_t s);
 
-// Exact values of listed pairs: out[t] = value(ref col ref_idx[t], query col
-// qry_idx[t]).
-void launch_exact_pairs(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                        const DevCsc& qry, const ColAux& qa, const int32_t* ref_idx,
-                        const int32_t* qry_idx, int64_t npairs, double* out, cudaStream_t s);
-
-// Candidate pairs (screened engine): slots with ref_idx < 0 are skipped; with
-// restore_self the self pair takes self_value.
-void launch_exact_pairs_sparse(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                               const DevCsc& qry, const ColAux& qa, const int32_t* ref_idx,
-                               const int32_t* qry_idx, int64_t npairs, int restore_self,
-                               double self_value, double* out, cudaStream_t s);
-
-// Warp-cooperative exact values of a candidate table (cand[ql * cap + t] for
-// t < count[ql]) for the match-only methods (binary, cosine, pearson).
-bool rerank_warp_supported(int method);
-void launch_rerank_warp(int method, int dist, const DevCsc& ref, const ColAux& ra,
-                        const DevCsc& qry, const ColAux& qa, const int32_t* cand,
-                        const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
-                        int restore_self, double self_value, double* out, cudaStream_t s);
+// Exact values of a candidate table, cand[ql * cap + t] for t < count[ql] of
+// the query columns q_begin + ql, into out at the same places; with
+// restore_self the self pair takes self_value.  nrow <= 2^18; mean_nnz: the mean
+// reference column's stored entries.  Returns 0 or a cudaError_t value.
+int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, const DevCsc& qry, const ColAux& qa,
+                  const int32_t* cand, const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
+                  int restore_self, double self_value, double* out, double mean_nnz, cudaStream_t s);
 
 // ---- sdg_select.cu: exact top-k selection --------------------------------------
 

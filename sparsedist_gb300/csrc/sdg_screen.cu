@@ -714,15 +714,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
   }
 }
 
-__global__ void k_exact_candidates_prep(const int32_t* count, int64_t nq, int cap, int32_t* qidx,
-                                        const int32_t* cand, int32_t* ridx, int64_t q_begin) {
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= nq * cap) return;
-  const int64_t ql = s / cap, t = s % cap;
-  if (t < count[ql]) { qidx[s] = (int32_t)(q_begin + ql); ridx[s] = cand[s]; }
-  else { qidx[s] = -1; ridx[s] = -1; }
-}
-
 // ---------------------------------------------------------------------------
 // the tensor-core screen
 //
@@ -1200,7 +1191,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   }
 
   float* S = nullptr;
-  int32_t *cand = nullptr, *count = nullptr, *over = nullptr, *qidx = nullptr, *ridx = nullptr;
+  int32_t *cand = nullptr, *count = nullptr, *over = nullptr;
   unsigned long long* work = nullptr;
   int2* order = nullptr;
   int32_t* units = nullptr;
@@ -1212,8 +1203,6 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   SK(cudaMallocAsync(&cand, sizeof(int32_t) * (size_t)cslots, s));
   SK(cudaMallocAsync(&count, sizeof(int32_t) * (size_t)chunk, s));
   SK(cudaMallocAsync(&over, sizeof(int32_t) * (size_t)chunk, s));
-  SK(cudaMallocAsync(&qidx, sizeof(int32_t) * (size_t)cslots, s));
-  SK(cudaMallocAsync(&ridx, sizeof(int32_t) * (size_t)cslots, s));
   SK(cudaMallocAsync(&rvals, sizeof(double) * (size_t)cslots, s));
   SK(cudaMallocAsync(&work, sizeof(*work), s));
   if (!use_t) {
@@ -1318,15 +1307,9 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     }
 
     // exact FP64 values of the kept pairs, then the exact top-k
-    if (rerank_warp_supported(r.method)) {
-      launch_rerank_warp(r.method, r.dist, ref, ra, qry, qa, cand, count, cap, nb, q0,
-                         r.selfmode && r.include_self && r.method != COVARIANCE, r.self_value, rvals, s);
-    } else {
-      k_exact_candidates_prep<<<blocks_for(nb * cap, 256), 256, 0, s>>>(count, nb, cap, qidx,
-                                                                          cand, ridx, q0);
-      launch_exact_pairs_sparse(r.method, r.dist, ref, ra, qry, qa, ridx, qidx, nb * cap,
-                                r.selfmode && r.include_self && r.method != COVARIANCE, r.self_value, rvals, s);
-    }
+    SK((cudaError_t)launch_rerank(r.method, r.dist, ref, ra, qry, qa, cand, count, cap, nb, q0,
+                                  r.selfmode && r.include_self && r.method != COVARIANCE, r.self_value, rvals,
+                                  nr > 0 ? (double)rc->nnz_total / (double)nr : 0.0, s));
     SelectArgs sa;
     sa.vals = rvals; sa.seg_stride = cap; sa.elem_stride = 1; sa.nseg = nb;
     sa.cand = cand; sa.cand_count = count; sa.cand_ld = cap;
@@ -1353,7 +1336,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   stats[2] += (int64_t)overflow_queries.size();
   if (S) SK(cudaFreeAsync(S, s));
   SK(cudaFreeAsync(cand, s)); SK(cudaFreeAsync(count, s));
-  SK(cudaFreeAsync(over, s)); SK(cudaFreeAsync(qidx, s)); SK(cudaFreeAsync(ridx, s));
+  SK(cudaFreeAsync(over, s)); 
   SK(cudaFreeAsync(rvals, s));
   SK(cudaFreeAsync(work, s));
   if (order) SK(cudaFreeAsync(order, s));
