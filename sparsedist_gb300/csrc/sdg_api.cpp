@@ -434,9 +434,49 @@ void exact_engine(sdg_ctx* c, const KnnPlan& P, sdg_matrix* ref, sdg_matrix* qry
   CK(cudaGetLastError());
 }
 
-// 1: exact FP64 slab; 2: FP32 sparse screen; 3: BF16 tensor-core screen
-// (cosine / euclidean; falls back to 2 inside screen_knn when a matrix's
-// values do not admit the BF16 bound or its dense copy does not fit).
+// Reference density from which the tensor screen is the faster one of the two
+// screens (it does 2 nrow nr nq dense flops; the FP32 screen adds the matched
+// rows alone).  Measured, FP32 / tensor, us, cosine: 10,000 x 10,000 at 2 % of
+// 2,000 rows 860 / 1,272, 5,000 x 20,000 at 2 % of 5,000 rows 1,084 / 1,308, 3,000
+// x 10,000 at 3 % of 20,000 rows 1,569 / 1,272, 4,096 x 10,000 at 5 % of 2,000 rows
+// 784 / 483, 4,096 x 30,000 log counts at 5 % 39,209 / 6,510.
+constexpr double kTensorMinDensity = 0.025;
+
+// Whether the exact FP64 slab beats the screens, for searches of at most 2^22
+// pairs (above, the screens always win).  Exact: merge steps (nr nnz_q + nq
+// nnz_r) at the method's measured rate, plus the selection over every pair;
+// screened: about 250 us of launches and per-column preparation plus the
+// screen's work per pair (pearson and covariance bound every pair in FP64).
+// Measured, exact / FP32 screen, us, euclidean: 301 x 301 at 9e6 steps 190 /
+// 117 resident, 519 / 557 from the host; 1,000 x 1,000 at 2e7 steps 347 / 106,
+// 663 / 556; at 8e7 982 / 127, 1,365 / 610; binary, 2,000 x 2,000 at 3e8 306 /
+// 156, 747 / 710; log counts, 128 x 30,000 at 1.2e10 steps 222,000 / 2,400.
+// Where a query matches few columns, the screen keeps whole tied sets and
+// falls back to the exact slab query by query (2,000 x 2,000 at 0.5 % of 500
+// rows: 225 / 10,300): it is taken only with 16 k matched columns expected.
+bool exact_is_cheaper(int method, int k, int64_t nr, int64_t nq, int32_t nrow, double nnz_r, double nnz_q) {
+  if (nr * nq > (int64_t)1 << 22) return false;
+  const double pairs = (double)nr * (double)nq;
+  const double shared = nrow > 0 ? nnz_q * nnz_r / (pairs * (double)nrow) : 0.0;   // expected rows per pair
+  if ((double)nr * std::min(shared, 1.0) < 16.0 * k) return true;
+  const double steps = (double)nr * nnz_q + (double)nq * nnz_r;
+  double rate = 0.0;                                  // merge steps per microsecond
+  switch (method) {
+    case BINARY: rate = 8.0e5; break;
+    case COSINE: rate = 3.3e5; break;
+    case EUCLIDEAN: rate = 8.8e4; break;
+    case MANHATTAN: rate = 1.7e5; break;
+    case JS: rate = 5.5e4; break;
+    default: rate = 1.9e5;                            // pearson, covariance
+  }
+  const double exact_us = steps / rate + pairs / 2.0e4;
+  const double screen_us = 250.0 + pairs / ((method == PEARSON || method == COVARIANCE) ? 2.0e3 : 4.0e4);
+  return exact_us <= screen_us;
+}
+
+// 1: exact FP64 slab; 2: FP32 sparse screen; 3: FP16 tensor-core screen
+// (binary / cosine / euclidean; falls back to 2 inside screen_knn when a
+// matrix's values do not admit the FP16 bound or its dense copy does not fit).
 int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_matrix* X, int64_t nq) {
   const int32_t nrow = ref->nrow;
   const int64_t nr = ref->ncol;
@@ -444,11 +484,10 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
   if (!screen_supported(P.method, P.k) || !screen_fits(nrow)) return 1;
   if (c->engine == 2) return 2;
   if (c->engine == 3) return (tensor_supported(P.method) && stc_supported(P.k)) ? 3 : 2;
-  // Small problems: the exact slab is already latency-bound.
-  if (nr * nq <= (int64_t)1 << 22) return 1;
-  // The tensor screen does 2 nrow nr nq dense flops where the FP32 screen
-  // visits nq / 16 * nnz(ref) stored entries: it wins from ~0.5 % density
-  // on, if the dense copies fit in half of the free device memory.
+  const double nnz_q = (double)X->nnz * (double)nq / (double)std::max<int64_t>(X->ncol, 1);
+  if (exact_is_cheaper(P.method, P.k, nr, nq, nrow, (double)ref->nnz, nnz_q)) return 1;
+  // the tensor screen where the reference is dense enough and the dense copies
+  // fit in half of the free device memory
   if (tensor_supported(P.method) && stc_supported(P.k) && nrow > 0 && nr > 0 &&
       (c->tensor_lazy || (ref->tensor[P.method].method == P.method && ref->tensor[P.method].usable))) {
     const double density = (double)ref->nnz / ((double)nrow * (double)nr);
@@ -456,7 +495,7 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
     if (X != ref) bytes += tensor_cache_bytes(nrow, X->ncol);
     size_t fr = 0, tot = 0;
     if (ref->tensor[P.method].method == P.method && ref->tensor[P.method].usable) bytes = 0;   // already resident
-    if (density >= 0.005 && cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2) return 3;
+    if (density >= kTensorMinDensity && cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2) return 3;
     cudaGetLastError();
   }
   return 2;
@@ -1229,25 +1268,27 @@ struct SearchShape {
 
 // Engine choice per search direction.  A cost model predicts each engine's
 // time from the shape (merge steps of the exact walk at the measured exact
-// rate; screened stored entries and slab bytes of the FP32 screen; dense flops
-// and copy bytes of the tensor screen), corrected per (shape class, engine) by
+// rate; matched rows and pairs of the FP32 screen; dense flops, copy bytes and
+// pairs of the tensor screen), corrected per (shape class, engine) by
 // the ratio of measured to predicted time (exponential average, learned from
-// every timed search and kept for the process); an engine a class has not
-// tried yet is tried once when its prediction is within 2x of the best.  The
+// every timed search and kept for the process); a screen a class has tried
+// less than twice is tried when its prediction is within 2x of the best.  The
 // persistent exact launch's work-item size (merge steps per item) is tuned the
 // same way over {2^20, 2^22, 2^24}.
 struct Autotuner {
   std::mutex mu;
   std::map<std::pair<ShapeClass, int>, std::pair<double, int>> corr;   // (ratio, samples)
+  uint32_t loaded = 0;                   // (method, engine) pairs that have run, a bit each
   double exact_rate = 2.0e11;            // merge steps per second, batched exact kernel
   std::map<int, std::pair<double, int>> item_rate;                      // log2 size -> (steps/s, samples)
 
   static double predict(int engine, const SearchShape& sh) {
     const double nq = (double)sh.nq, nr = (double)sh.nr;
     if (engine == 1) return 0.0;                                        // scaled by exact_rate
-    if (engine == 2) return nq / 16.0 * (double)sh.nnz_r / 1.1e11 + nq * nr * 8.0 / 4.0e12 + 2e-3;
+    const double matches = (double)sh.nnz_q * (double)sh.nnz_r / std::max(1.0, (double)sh.nrow);
+    if (engine == 2) return matches * 2.5e-12 + nq * nr * 7.0e-12 + 3e-4;
     const double ld = std::ceil((double)sh.nrow / 64.0) * 64.0;
-    return 2.0 * ld * nq * nr / 1.9e15 + ld * (nq + nr) * 2.0 / 3.0e12 + 3e-3;
+    return 2.0 * ld * nq * nr / 1.9e15 + ld * (nq + nr) * 2.0 / 3.0e12 + nq * nr * 7.0e-12 + 5e-4;
   }
   double predict_exact(const SearchShape& sh) const {
     return ((double)sh.nr * (double)sh.nnz_q + (double)sh.nq * (double)sh.nnz_r) / exact_rate;
@@ -1265,17 +1306,23 @@ struct Autotuner {
       const double c = cost(e, sh);
       if (c < bc) { bc = c; best = e; }
     }
-    for (int e : engines)
-      if (e != best && corr.find({sh.cls(), e}) == corr.end() && cost(e, sh) <= 2.0 * bc) return e;
+    for (int e : engines) {
+      if (e == best || e == 1) continue;           // the exact launch is learned as a whole (learn_exact)
+      const auto it = corr.find({sh.cls(), e});
+      if ((it == corr.end() || it->second.second < 2) && cost(e, sh) <= 2.0 * bc) return e;
+    }
     return best;
   }
   void learn(int engine, const SearchShape& sh, double seconds) {
     std::lock_guard<std::mutex> lock(mu);
     const double pred = engine == 1 ? predict_exact(sh) : predict(engine, sh);
     if (!(pred > 0.0) || !(seconds > 0.0)) return;
+    // a method's first search on an engine also loads its kernels
+    if (!(loaded & (1u << (4 * sh.method + engine)))) { loaded |= 1u << (4 * sh.method + engine); return; }
     auto& c = corr[{sh.cls(), engine}];
     const double r = seconds / pred;
-    c.first = c.second == 0 ? r : 0.7 * c.first + 0.3 * r;
+    // a first sample may hold the memory pool's growth: the second replaces it if shorter
+    c.first = c.second == 0 ? r : c.second == 1 ? std::min(c.first, r) : 0.7 * c.first + 0.3 * r;
     ++c.second;
   }
   int item_log2() {
@@ -1309,11 +1356,15 @@ Autotuner& autotuner() {
 std::vector<int> candidate_engines(const SearchShape& sh, bool drop) {
   (void)drop;
   std::vector<int> e;
-  if (sh.k <= kBatchMaxK) e.push_back(1);
+  if (sh.k <= kBatchMaxK) {
+    e.push_back(1);
+    // small, or too few matched columns for the screens (exact_is_cheaper)
+    if (exact_is_cheaper(sh.method, sh.k, sh.nr, sh.nq, sh.nrow, (double)sh.nnz_r, (double)sh.nnz_q)) return e;
+  }
   if (screen_supported(sh.method, sh.k) && screen_fits(sh.nrow)) {
     e.push_back(2);
     const double density = (sh.nrow > 0 && sh.nr > 0) ? (double)sh.nnz_r / ((double)sh.nrow * (double)sh.nr) : 0.0;
-    if (tensor_supported(sh.method) && stc_supported(sh.k) && density >= 0.005) {
+    if (tensor_supported(sh.method) && stc_supported(sh.k) && density >= 0.5 * kTensorMinDensity) {
       const size_t bytes = tensor_cache_bytes(sh.nrow, sh.nr) + tensor_cache_bytes(sh.nrow, sh.nq);
       size_t fr = 0, tot = 0;
       if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2) e.push_back(3);
@@ -1484,6 +1535,17 @@ SDG_API int sdg_knn_cross_batch(sdg_ctx* c, int nprob, const sdg_csc* X, const s
         double total_steps = 0.0;
         int kmax = 1, lwords = 0;
         for (size_t b = 0; b < probs.size(); ++b) {
+          const Held& h = held[(size_t)prob_of[b]];
+          for (int dir = 0; dir < 2; ++dir)
+            if ((dir == 0 ? h.ef : h.er) == 1)
+              total_steps += (double)h.fs.nr * (double)h.fs.nnz_q + (double)h.fs.nq * (double)h.fs.nnz_r;
+        }
+        // merge steps per item: the tuned size, less where the wave would leave
+        // warps idle (110 x 684 columns of 2,180 entries: 110 items of 22 rounds
+        // took 17 to 44 ms)
+        const double item_steps = std::min(std::ldexp(1.0, lg), std::max(1.0, total_steps / ((double)sms * 32.0)));
+        total_steps = 0.0;
+        for (size_t b = 0; b < probs.size(); ++b) {
           Held& h = held[(size_t)prob_of[b]];
           for (int dir = 0; dir < 2; ++dir) {
             if ((dir == 0 ? h.ef : h.er) != 1) continue;
@@ -1501,7 +1563,7 @@ SDG_API int sdg_knn_cross_batch(sdg_ctx* c, int nprob, const sdg_csc* X, const s
                 const double steps = (double)Rc.ncol * (double)(Qc.p[q + 1] - Qc.p[q]) + (double)nnz_r;
                 total_steps += steps;
                 const int64_t parts = std::max<int64_t>(
-                    1, std::min<int64_t>((Rc.ncol + 31) / 32, (int64_t)std::ceil(steps / std::ldexp(1.0, lg))));
+                    1, std::min<int64_t>((Rc.ncol + 31) / 32, (int64_t)std::ceil(steps / item_steps)));
                 for (int64_t t = 0; t < parts; ++t) {
                   BatchItem it;
                   it.prob = (int32_t)b; it.dir = dir; it.q = q; it.pad = 0;
@@ -1852,7 +1914,7 @@ SDG_API int sdg_server_create(sdg_ctx* ctx, const sdg_matrix* ref, int workers, 
         size_t fr = 0, tot = 0;
         const size_t bytes = tensor_cache_bytes(S->ref->nrow, S->ref->ncol);
         // the copy must leave the admission budget free for the requests
-        if (density < 0.005 || cudaMemGetInfo(&fr, &tot) != cudaSuccess || bytes > fr / 2 ||
+        if (density < kTensorMinDensity || cudaMemGetInfo(&fr, &tot) != cudaSuccess || bytes > fr / 2 ||
             (int64_t)(bytes + (size_t)mem_budget) > (int64_t)fr) {
           cudaGetLastError();
           continue;
