@@ -124,7 +124,10 @@ struct TcArgs {
   const float* qnorm2;        // query sums of squares (index in Q)
   const uint8_t* qempty;      // degenerate queries (no list)
   unsigned* tshared;          // [nq]: the best running k-th pessimistic key of any list (ordered bits)
-  float* lists;               // [nq][nslots][k]
+  float* lists;               // [nq][nslots][k] (one pass)
+  float* maxima;              // MODE 1: [nq][2 * ntiles * gran]
+  int gran;                   // MODE 1: maxima per tile half (1 or 4)
+  int use_w;                  // MODE 1, cosine: some reference is degenerate
   int32_t* ecount;            // [nq][nslots]
   int32_t* eidx;              // [nq][nslots][ecap]
   float* es;                  // [nq][nslots][ecap]: the appended references' GEMM values
@@ -147,7 +150,19 @@ __host__ __device__ __forceinline__ int64_t last_cta(int64_t g, int64_t ntiles, 
   return ((g + 1) * ntiles - 1) / per;
 }
 
-template <int KL, bool PAIR>
+// MODE 0: the running lists described above, one pass over the references.
+// MODE 1 and 2: two passes for blocks whose pass is short.  MODE 1 keeps no
+// list: every thread stores the largest x' = a s - w[r] of each tile half (or of
+// each of its four 32-column chunks) with w[r] chosen so that x' less a
+// constant of the query is at most the reference's pessimistic key
+// (k_tc_maxima); the k-th largest of a query's maxima (k_tc_threshold) is then
+// reached by k references, so it is at most the k-th best key, and with several
+// times k maxima hardly below it.  MODE 2 appends the references that pass the
+// hot test at that threshold.  A running list starts from nothing in every CTA
+// and column half: for 777 queries x 150,001 references each of a query's 44
+// lists saw 3,500 references and took the slow path for a hundred of them, 80 %
+// of the launch's instructions.
+template <int KL, bool PAIR, int MODE>
 __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__ CUtensorMap qmap,
                                                        const __grid_constant__ CUtensorMap rmap, TcArgs P) {
   using C = Cfg<PAIR>;
@@ -465,6 +480,52 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       __syncwarp();
     };
 
+    // MODE 2: the passing references of one chunk straight to the list
+    auto append = [&](const uint32_t (&v)[32], uint32_t mask, int64_t r0) {
+      while (mask) {
+        const int jj = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const float sv = pick(v, jj);
+        const int64_t r = r0 + jj;
+        if ((P.self && r == q) || (sv == 0.f && P.w[r] == INFINITY)) continue;
+        if (cnt < P.ecap) { my_idx[cnt] = (int32_t)r; my_s[cnt] = sv; }
+        ++cnt;
+      }
+      __syncwarp();
+    };
+    // MODE 1: the largest x' of one chunk; weigh: subtract w[r] (+inf for
+    // degenerate and padding references)
+    auto chunk_max = [&](const uint32_t (&v)[32], int64_t r0, bool weigh) -> float {
+      float x[32];
+      if (weigh) {
+        const float4* w4 = reinterpret_cast<const float4*>(P.w + r0);
+#pragma unroll
+        for (int j4 = 0; j4 < 8; ++j4) {
+          const float4 ww = __ldg(w4 + j4);
+          x[4 * j4 + 0] = fmaf(P.a, __uint_as_float(v[4 * j4 + 0]), -ww.x);
+          x[4 * j4 + 1] = fmaf(P.a, __uint_as_float(v[4 * j4 + 1]), -ww.y);
+          x[4 * j4 + 2] = fmaf(P.a, __uint_as_float(v[4 * j4 + 2]), -ww.z);
+          x[4 * j4 + 3] = fmaf(P.a, __uint_as_float(v[4 * j4 + 3]), -ww.w);
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) x[t] = __uint_as_float(v[t]);
+      }
+      if (P.self && __any_sync(0xffffffffu, q >= r0 && q < r0 + 32)) {
+#pragma unroll
+        for (int t = 0; t < 32; ++t)
+          if (r0 + t == q) x[t] = -INFINITY;
+      }
+      float m[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) m[t] = fmaxf(x[2 * t], x[2 * t + 1]);
+#pragma unroll
+      for (int wdt = 8; wdt > 0; wdt >>= 1)
+#pragma unroll
+        for (int t = 0; t < wdt; ++t) m[t] = fmaxf(m[t], m[t + wdt]);
+      return m[0];
+    };
+
     int64_t j = 0;                                    // tile counter (the MMA's order)
     bool ok = true;
     for (int64_t f = f0; f < f1 && ok;) {
@@ -478,7 +539,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
 #pragma unroll
       for (int i = 0; i < KL; ++i) lst[i] = (i < KL - K) ? INFINITY : -INFINITY;
       T = -INFINITY;
-      Ts = active ? fkey_value(*(volatile unsigned*)(P.tshared + ql)) : -INFINITY;
+      Ts = (MODE != 1 && active) ? fkey_value(*(volatile unsigned*)(P.tshared + ql)) : -INFINITY;
       e_thr = -FLT_MAX;
       if (Ts > -INFINITY) set_thr();
       cnt = 0;
@@ -505,7 +566,28 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             else mbar_arrive(acc_empty + buf);
           }
         };
-        if constexpr (KL <= 32) {
+        if constexpr (MODE == 1) {
+          // the chunks' largest x'
+          float cm[4];
+          const bool weigh = !cosine || P.use_w || r_half + BN / 2 > P.n;
+#pragma unroll
+          for (int hh = 0; hh < BN / 64; hh += 2) {
+            uint32_t va[32], vb[32];
+            tmem_ld32_issue(tb + hh * 32, va);
+            tmem_ld32_issue(tb + hh * 32 + 32, vb);
+            tmem_ld_wait(va);
+            tmem_ld_wait(vb);
+            if (hh == BN / 64 - 2) release();
+            cm[hh] = chunk_max(va, r_half + hh * 32, weigh);
+            cm[hh + 1] = chunk_max(vb, r_half + hh * 32 + 32, weigh);
+          }
+          if (active) {
+            const int64_t tile = f - g * ntiles;
+            float* out = P.maxima + ql * (2 * ntiles * P.gran) + (tile * 2 + half) * P.gran;
+            if (P.gran == 4) *reinterpret_cast<float4*>(out) = make_float4(cm[0], cm[1], cm[2], cm[3]);
+            else *out = fmaxf(fmaxf(cm[0], cm[1]), fmaxf(cm[2], cm[3]));
+          }
+        } else if constexpr (KL <= 32) {
           // chunks in pairs (the TMEM loads take a few tens of cycles; the
           // pair's hot tests overlap)
 #pragma unroll 1
@@ -518,8 +600,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             if (hh == BN / 64 - 2) release();
             const uint32_t ma = hot_mask(va, r_half + hh * 32), mb = hot_mask(vb, r_half + hh * 32 + 32);
             if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
-              take(va, ma, r_half + hh * 32);
-              take(vb, mb, r_half + hh * 32 + 32);
+              if constexpr (MODE == 2) {
+                append(va, ma, r_half + hh * 32);
+                append(vb, mb, r_half + hh * 32 + 32);
+              } else {
+                take(va, ma, r_half + hh * 32);
+                take(vb, mb, r_half + hh * 32 + 32);
+              }
             }
           }
         } else {
@@ -533,22 +620,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             if (__any_sync(0xffffffffu, ma != 0u)) take(va, ma, r_half + hh * 32);
           }
         }
-        if ((j & (SHARE_TILES - 1)) == SHARE_TILES - 1 && active) {
+        if (MODE == 0 && (j & (SHARE_TILES - 1)) == SHARE_TILES - 1 && active) {
           // publish this list's running key and take the best one published
           const unsigned prev = atomicMax(P.tshared + ql, fkey(T));
           const float best = fmaxf(fkey_value(prev), T);
           if (best > Ts) { Ts = best; set_thr(); }
         }
       }
-      flush();
-      if (active) atomicMax(P.tshared + ql, fkey(T));
-      if (active) {
-        float* out = P.lists + slot * K;
+      if constexpr (MODE == 0) {
+        flush();
+        if (active) atomicMax(P.tshared + ql, fkey(T));
+        if (active) {
+          float* out = P.lists + slot * K;
 #pragma unroll
-        for (int i = 0; i < KL; ++i)
-          if (i >= KL - K) out[i - (KL - K)] = lst[i];
-        P.ecount[slot] = cnt;
+          for (int i = 0; i < KL; ++i)
+            if (i >= KL - K) out[i - (KL - K)] = lst[i];
+        }
       }
+      if (MODE != 1 && active) P.ecount[slot] = cnt;
     }
   }
   fence_before();
@@ -692,8 +781,8 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
     return;
   }
   // T from the keys above the shared one
-  const float* in = A.lists + ql * A.nslots * (int64_t)K;
-  const int tot = used * K;
+  const float* in = A.lists ? A.lists + ql * A.nslots * (int64_t)K : nullptr;   // two passes: T is the shared key
+  const int tot = in ? used * K : 0;
   for (int p = rank; p < tot; p += nt) {
     const float v = in[p];
     if (v > ts) keys[atomicAdd(&s_count[slot_q], 1)] = fkey(v);
@@ -770,14 +859,65 @@ __global__ void k_tc_key_init(int64_t nq, unsigned* keys) {
 }
 
 // w[r]: +inf for degenerate references and the padding; 0 (cosine) or
-// (1 - c) Nr (euclidean) otherwise
-__global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_c, const float* norm2,
-                             const uint8_t* empty, float* w) {
+// (1 - c) Nr (euclidean) otherwise; wp (two passes, or null): the same with
+// one_plus_c for the first pass's x'
+__global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_c, float one_plus_c,
+                             const float* norm2, const uint8_t* empty, float* w, float* wp) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= nw) return;
-  float v = INFINITY;
-  if (r < n && !empty[r]) v = (method == COSINE) ? 0.f : one_minus_c * norm2[r];
+  float v = INFINITY, vp = INFINITY;
+  if (r < n && !empty[r]) {
+    v = (method == COSINE) ? 0.f : one_minus_c * norm2[r];
+    vp = (method == COSINE) ? 0.f : one_plus_c * norm2[r];
+  }
   w[r] = v;
+  if (wp) wp[r] = vp;
+}
+
+// Two passes: each query's threshold, the k-th largest of its maxima less what
+// separates x' from the pessimistic key.  Cosine: x' = s, lo = s - rel.
+// Euclidean: x' = 2 s - (1 + c') Nr with c' = rel + 2^-19; 2 rel sqrt(Nq Nr) <=
+// rel (Nq + Nr), so lo = 2 s - (Nq + Nr) - 2 rel sqrt(Nq Nr) - 2^-20 (Nq + Nr) -
+// 1e-30 >= x' - (1 + c') Nq + 2^-20 (Nq + Nr) - 1e-30: the last but one term
+// covers the FP32 roundings of (1 + c') N, 2^-21 |x'| that of x' and of the
+// differences.  One block per query.
+__global__ void __launch_bounds__(256) k_tc_threshold(int method, int64_t q0, int m, int K, float rel,
+                                                      float one_plus_c, const float* qnorm2, const uint8_t* qempty,
+                                                      const float* maxima, unsigned* tshared) {
+  extern __shared__ uint32_t tkeys[];
+  __shared__ uint32_t red[8];
+  const int64_t ql = blockIdx.x;
+  if (qempty[q0 + ql]) {
+    if (threadIdx.x == 0) tshared[ql] = fkey(-INFINITY);
+    return;
+  }
+  for (int i = threadIdx.x; i < m; i += 256) tkeys[i] = fkey(fmaxf(maxima[ql * m + i], -INFINITY));
+  __syncthreads();
+  const kth::Group<8> G{red};
+  const float x = fkey_value(kth::largest<8>(G, tkeys, m, K));
+  if (threadIdx.x == 0) {
+    float T = -INFINITY;
+    if (x > -INFINITY) {
+      const float base = (method == COSINE) ? rel : one_plus_c * qnorm2[q0 + ql];
+      T = x - base - (4.76837158203125e-7f * (fabsf(x) + base) + 1e-30f);
+    }
+    tshared[ql] = fkey(T);
+  }
+}
+
+// Whether two passes beat one for a block of nq queries: a pass costs 1.4 us a
+// tile up to d = 128 and 2.1 beyond (1.4 times that where the references exceed
+// the L2), the running lists about 50 + 8 k us of filling; with few queries in a
+// group hardly any lane fills a list.  One pass / two passes, us: 777 x 150,001, d =
+// 100, k = 15: 254 / 131; 3,000 x 60,000, d = 64, k = 30: 319 / 164; 500 x
+// 1,000,000, d = 128, k = 50: 622 / 280; 4,096 x 150,000, d = 256, k = 20: 490 /
+// 515; 1,024 x 800,000, d = 200, k = 20: 608 / 975; 1 x 400,000, d = 256: 60 / 80.
+constexpr int64_t TWO_PASS_MAXIMA = 12288;            // per query, held in shared memory
+bool two_passes(int64_t nq, int64_t n, int dpad, int k, int64_t tiles_per_cta, int64_t maxima) {
+  if (nq < 64 || maxima < 4 * (int64_t)k || maxima > TWO_PASS_MAXIMA) return false;
+  double pass_us = (double)tiles_per_cta * (dpad <= 128 ? 1.4 : 2.1);
+  if (n * dpad * 2 > (int64_t)96 << 20) pass_us *= 1.4;
+  return pass_us < 50.0 + 8.0 * k;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -830,10 +970,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   // the list length: the smallest of 16 / 24 / 32 / 48 / 64 that holds k
   auto pick_kernel = [&](bool pair) {
     if (pair)
-      return (k <= 16) ? k_dense_tc<16, true> : (k <= 24) ? k_dense_tc<24, true> : (k <= 32) ? k_dense_tc<32, true>
-           : (k <= 48) ? k_dense_tc<48, true> : k_dense_tc<64, true>;
-    return (k <= 16) ? k_dense_tc<16, false> : (k <= 24) ? k_dense_tc<24, false> : (k <= 32) ? k_dense_tc<32, false>
-         : (k <= 48) ? k_dense_tc<48, false> : k_dense_tc<64, false>;
+      return (k <= 16) ? k_dense_tc<16, true, 0> : (k <= 24) ? k_dense_tc<24, true, 0>
+           : (k <= 32) ? k_dense_tc<32, true, 0> : (k <= 48) ? k_dense_tc<48, true, 0> : k_dense_tc<64, true, 0>;
+    return (k <= 16) ? k_dense_tc<16, false, 0> : (k <= 24) ? k_dense_tc<24, false, 0>
+         : (k <= 32) ? k_dense_tc<32, false, 0> : (k <= 48) ? k_dense_tc<48, false, 0> : k_dense_tc<64, false, 0>;
   };
   // CTA pairs (clusters of two) where the block has more than one 128-query
   // group and the device can hold such clusters; the work unit is then a pair
@@ -881,14 +1021,25 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   const float rel = 0.0040f + (float)D->d * 2.384185791015625e-7f;
   const float omc = 1.f - (rel + 9.5367431640625e-7f);
 
-  float *w = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
+  // two passes (MODE 1 and 2) where a pass is short
+  const int gran = n >= (int64_t)(BN / 2) * 8 * k ? 1 : 4;
+  const int64_t m = 2 * ntiles * gran;
+  const bool two = !pair && two_passes(nq, n, D->dpad, k, per, m);
+  const float opc = 1.f + rel + 1.9073486328125e-6f;     // 2^-19
+
+  float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
   int32_t *ecount = nullptr, *eidx = nullptr;
   unsigned* tshared = nullptr;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   const int64_t nw = ntiles * BN;
   chk(cudaMallocAsync(&w, sizeof(float) * (size_t)nw, s));
-  chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
+  if (two) {
+    chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw, s));
+    chk(cudaMallocAsync(&maxima, sizeof(float) * (size_t)(nq * m), s));
+  } else {
+    chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
+  }
   chk(cudaMallocAsync(&ecount, sizeof(int32_t) * (size_t)(nq * nslots), s));
   chk(cudaMallocAsync(&eidx, sizeof(int32_t) * (size_t)(nq * nslots * ecap), s));
   chk(cudaMallocAsync(&es, sizeof(float) * (size_t)(nq * nslots * ecap), s));
@@ -896,9 +1047,9 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   chk(cudaMallocAsync(&tshared, sizeof(unsigned) * (size_t)nq, s));
   if (e == cudaSuccess) {
     // every query's shared key starts at fkey(-inf)
-    k_tc_key_init<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(nq, tshared);
+    if (!two) k_tc_key_init<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(nq, tshared);
     chk(cudaMemsetAsync(ecount, 0, sizeof(int32_t) * (size_t)(nq * nslots), s));
-    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, D->norm2, D->empty, w);
+    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, opc, D->norm2, D->empty, w, wp);
     TcArgs P;
     P.method = method; P.k = k; P.dch = dch; P.ecap = ecap;
     P.self = self ? 1 : 0;
@@ -908,11 +1059,26 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     P.w = w; P.norm2 = D->norm2; P.qnorm2 = Q->norm2; P.qempty = Q->empty;
     P.tshared = tshared;
     P.lists = lists; P.ecount = ecount; P.eidx = eidx; P.es = es;
+    P.maxima = maxima; P.gran = gran; P.use_w = D->n_empty > 0 ? 1 : 0;
     P.status = status;
     P.stall = tc_take_stall() ? 1 : 0;
-    auto kern = pick_kernel(pair);
+    auto kern = two ? k_dense_tc<1, false, 2> : pick_kernel(pair);
     chk(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     sdg_time_begin(ctx);
+    if (two && e == cudaSuccess) {
+      chk(cudaFuncSetAttribute(k_dense_tc<1, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)SMEM_BYTES));
+      TcArgs P1 = P;
+      P1.w = wp;
+      if (e == cudaSuccess) k_dense_tc<1, false, 1><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(qmap, rmap, P1);
+      P.stall = 0;                                     // one launch is stalled at a time
+      const size_t tsm = sizeof(uint32_t) * (size_t)m;
+      if (tsm > 48 * 1024)
+        chk(cudaFuncSetAttribute(k_tc_threshold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+      if (e == cudaSuccess)
+        k_tc_threshold<<<(unsigned)nq, 256, tsm, s>>>(method, q0, (int)m, k, rel, opc, Q->norm2, Q->empty, maxima,
+                                                      tshared);
+    }
     if (e == cudaSuccess) {
       if (pair) {
         cudaLaunchConfig_t cfg = {};
@@ -949,7 +1115,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     chk(cudaGetLastError());
   }
   // stream-ordered frees: the caller reads *status with its own results
-  for (void* p : {(void*)w, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared})
+  for (void* p : {(void*)w, (void*)wp, (void*)maxima, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared})
     if (p) cudaFreeAsync(p, s);
   if (e != cudaSuccess) {
     set_error(cudaGetErrorString(e));
