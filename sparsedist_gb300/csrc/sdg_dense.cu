@@ -111,6 +111,96 @@ __global__ void k_dense_errnorm(int32_t d, int64_t n, const double* u64, const d
   }
 }
 
+// A query block's forms, for one method only, padding included (warp per
+// column of npad).  k_query_prep: the FP64 copy, sum of squares, empty flag and
+// finiteness check as k_dense_prep; euclidean (xb set): also the BF16 copies
+// (d rows, and dpad rows with zeros below d) and their error norms as
+// k_dense_errnorm.  k_query_unit, cosine, after the unit columns: their FP32 and
+// BF16 copies and error norms.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ __forceinline__ void bf16_forms(double v, float f, int32_t r, int64_t j, int32_t d, int32_t dpad,
+                                           __nv_bfloat16* b, __nv_bfloat16* bp, double& e, double& nn) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(f);
+  b[j * d + r] = h;
+  if (bp != b) bp[j * (int64_t)dpad + r] = h;
+  const double bv = (double)__bfloat162float(h), dv = v - bv;
+  e += dv * dv;
+  nn += bv * bv;
+}
+
+__global__ void k_query_prep(int32_t d, int32_t dpad, int64_t n, int64_t npad, const float* x32, double* x64,
+                             float* norm2, uint8_t* empty, __nv_bfloat16* xb, __nv_bfloat16* xbp, float* xe, float* xn,
+                             int* err) {
+  const int lane = threadIdx.x & 31;
+  const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (j >= npad) return;
+  if (j >= n) {
+    if (lane == 0) {
+      norm2[j] = 0.f;
+      empty[j] = 1;
+      if (xb) { xe[j] = 0.f; xn[j] = 0.f; }
+    }
+    return;
+  }
+  double s = 0.0, e = 0.0, nn = 0.0;
+  bool nz = false, bad = false;
+  for (int32_t r = lane; r < d; r += 32) {
+    const float v = x32[j * d + r];
+    bad |= !isfinite(v);
+    nz |= (v != 0.f);
+    const double dv = (double)v;
+    x64[j * d + r] = dv;
+    s += dv * dv;
+    if (xb) bf16_forms(dv, v, r, j, d, dpad, xb, xbp, e, nn);
+  }
+  if (xb && xbp != xb)
+    for (int32_t r = d + lane; r < dpad; r += 32) xbp[j * (int64_t)dpad + r] = __float2bfloat16_rn(0.f);
+  s = warp_sum(s);
+  nz = __any_sync(0xffffffffu, nz);
+  bad = __any_sync(0xffffffffu, bad);
+  if (xb) { e = warp_sum(e); nn = warp_sum(nn); }
+  if (lane == 0) {
+    norm2[j] = (float)s;
+    empty[j] = nz ? 0 : 1;
+    if (bad) atomicOr(err, 1);
+    if (xb) {
+      xe[j] = __double2float_ru(sqrt(e) * (1.0 + 1e-12));
+      xn[j] = __double2float_ru(sqrt(nn) * (1.0 + 1e-12));
+    }
+  }
+}
+
+__global__ void k_query_unit(int32_t d, int32_t dpad, int64_t n, int64_t npad, const double* u64, float* u32,
+                             __nv_bfloat16* ub, __nv_bfloat16* ubp, float* ue, float* un) {
+  const int lane = threadIdx.x & 31;
+  const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (j >= npad) return;
+  if (j >= n) {
+    if (lane == 0) { ue[j] = 0.f; un[j] = 0.f; }
+    return;
+  }
+  double e = 0.0, nn = 0.0;
+  for (int32_t r = lane; r < d; r += 32) {
+    const double v = u64[j * d + r];
+    const float f = (float)v;
+    u32[j * d + r] = f;
+    bf16_forms(v, f, r, j, d, dpad, ub, ubp, e, nn);
+  }
+  if (ubp != ub)
+    for (int32_t r = d + lane; r < dpad; r += 32) ubp[j * (int64_t)dpad + r] = __float2bfloat16_rn(0.f);
+  e = warp_sum(e);
+  nn = warp_sum(nn);
+  if (lane == 0) {
+    ue[j] = __double2float_ru(sqrt(e) * (1.0 + 1e-12));
+    un[j] = __double2float_ru(sqrt(nn) * (1.0 + 1e-12));
+  }
+}
+
 // A query's scan over the n references is split into segments of DSEG
 // references, one warp per (query, segment), so that the slab is streamed at
 // full bandwidth: (1) each warp keeps the top k of its segment's pessimistic
@@ -671,26 +761,17 @@ namespace {
 // Builds the resident form of d x n FP32 columns X (host or device memory):
 // FP64 values and unit columns (unit_csc on each dense column), their FP32
 // and BF16 copies (rows padded to a multiple of 64 with zeros), sums of
-// squares and degenerate flags.  `async` takes the buffers from the stream's
-// pool (a per-request query matrix) instead of cudaMalloc (a resident
-// reference); `blas` creates the cuBLAS handle of the slab and plain modes.
-// keep_err (stream-ordered builds only): instead of reading the finiteness
-// flag back (a stream synchronisation), hand the device flag to the caller,
-// who reads it with its own results and frees it; n_empty is then not counted
-// (a query block needs only the device flags).
-int dense_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, bool async, bool blas, sdg_dense** out,
-                int** keep_err = nullptr) {
+// squares and degenerate flags, and the cuBLAS handle of the slab and plain
+// modes.
+int dense_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, sdg_dense** out) {
   cudaStream_t s = ctx_stream(ctx);
   DK(cudaSetDevice(ctx_device(ctx)));
   auto D = new sdg_dense();
   D->device = ctx_device(ctx);
   D->d = d;
   D->n = n;
-  D->async = async;
   D->stream = s;
-  auto alloc = [&](auto** p, size_t bytes) {
-    return async ? cudaMallocAsync((void**)p, bytes, s) : cudaMalloc((void**)p, bytes);
-  };
+  auto alloc = [&](auto** p, size_t bytes) { return cudaMalloc((void**)p, bytes); };
   const size_t tot = (size_t)d * (size_t)n;
   int* err = nullptr;
   const int64_t npad = (n + 127) / 128 * 128;       // float4 / uchar4 reads past n stay in bounds
@@ -735,26 +816,75 @@ int dense_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, bool async, 
                           cudaMemcpyDeviceToDevice, s));
   }
   chk(cudaGetLastError());
-  if (keep_err && async) {
-    if (e != cudaSuccess) { cudaFreeAsync(err, s); sdg_dense_free(D); return cuda_fail(e); }
-    *keep_err = err;
-    *out = D;
-    return SDG_OK;
-  }
   int herr = 0;
   std::vector<uint8_t> he((size_t)n);
   chk(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   chk(cudaMemcpyAsync(he.data(), D->empty, (size_t)n, cudaMemcpyDeviceToHost, s));
-  if (async) chk(cudaFreeAsync(err, s));
   chk(cudaStreamSynchronize(s));
-  if (!async) cudaFree(err);
+  cudaFree(err);
   if (e != cudaSuccess) { sdg_dense_free(D); return cuda_fail(e); }
   for (uint8_t v : he) D->n_empty += v;
   if (herr) { sdg_dense_free(D); return fail_with(SDG_E_NONFINITE, "Cosine requires finite input (found NA, NaN or Inf)."); }
-  if (blas && cublasCreate(&D->blas) != CUBLAS_STATUS_SUCCESS) {
+  if (cublasCreate(&D->blas) != CUBLAS_STATUS_SUCCESS) {
     sdg_dense_free(D);
     return fail_with(SDG_E_CUDA, "cublasCreate failed");
   }
+  *out = D;
+  return SDG_OK;
+}
+
+// The forms of a query block that `method` reads (see k_query_prep), in one
+// stream-ordered allocation: D->x64 owns it, the other pointers lie inside.  No
+// synchronisation: the finiteness flag *err stays on the device, for the caller
+// to read with its own results; n_empty is not counted (a query block needs only
+// the device flags).
+int query_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, int method, sdg_dense** out, int** err) {
+  cudaStream_t s = ctx_stream(ctx);
+  DK(cudaSetDevice(ctx_device(ctx)));
+  const int64_t npad = (n + 127) / 128 * 128;       // float4 / uchar4 reads past n stay in bounds
+  const int32_t dpad = (d + 63) / 64 * 64;
+  const size_t tot = (size_t)d * (size_t)n;
+  const bool cosine = method == COSINE;
+  size_t at = 0;
+  auto part = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) / 256 * 256; return o; };
+  const size_t o64 = part(tot * 8), ou64 = cosine ? part(tot * 8) : 0, o32 = part(tot * 4);
+  const size_t ou32 = cosine ? part(tot * 4) : 0, ob = part(tot * 2);
+  const size_t obp = dpad != d ? part((size_t)dpad * (size_t)n * 2) : ob;
+  const size_t onorm = part((size_t)npad * 4), oe = part((size_t)npad * 4), on = part((size_t)npad * 4);
+  const size_t oscale = cosine ? part((size_t)n * 8) : 0, oempty = part((size_t)npad), oerr = part(sizeof(int));
+  char* blob = nullptr;
+  DK(cudaMallocAsync((void**)&blob, at, s));
+  auto D = new sdg_dense();
+  D->device = ctx_device(ctx);
+  D->d = d; D->n = n; D->npad = npad; D->dpad = dpad;
+  D->async = true;
+  D->stream = s;
+  D->x64 = reinterpret_cast<double*>(blob + o64);
+  D->x32 = reinterpret_cast<float*>(blob + o32);
+  D->norm2 = reinterpret_cast<float*>(blob + onorm);
+  D->empty = reinterpret_cast<uint8_t*>(blob + oempty);
+  int* flag = reinterpret_cast<int*>(blob + oerr);
+  __nv_bfloat16 *b = reinterpret_cast<__nv_bfloat16*>(blob + ob), *bp = reinterpret_cast<__nv_bfloat16*>(blob + obp);
+  float *e = reinterpret_cast<float*>(blob + oe), *nn = reinterpret_cast<float*>(blob + on);
+  cudaError_t c = cudaMemsetAsync(flag, 0, sizeof(int), s);
+  if (c == cudaSuccess) c = cudaMemcpyAsync(D->x32, X, tot * 4, cudaMemcpyDefault, s);
+  if (c == cudaSuccess) {
+    const unsigned grid = blocks_for(npad * 32, 256);
+    k_query_prep<<<grid, 256, 0, s>>>(d, dpad, n, npad, D->x32, D->x64, D->norm2, D->empty, cosine ? nullptr : b, bp,
+                                      e, nn, flag);
+    if (cosine) {
+      D->u64 = reinterpret_cast<double*>(blob + ou64);
+      D->u32 = reinterpret_cast<float*>(blob + ou32);
+      D->ub = b; D->ubp = bp; D->ue = e; D->un = nn;
+      launch_unit_dense(d, n, D->x64, D->u64, reinterpret_cast<double*>(blob + oscale), flag, s);
+      k_query_unit<<<grid, 256, 0, s>>>(d, dpad, n, npad, D->u64, D->u32, b, bp, e, nn);
+    } else {
+      D->xb = b; D->xbp = bp; D->xe = e; D->xn = nn;
+    }
+    c = cudaGetLastError();
+  }
+  if (c != cudaSuccess) { sdg_dense_free(D); return cuda_fail(c); }
+  *err = flag;
   *out = D;
   return SDG_OK;
 }
@@ -1033,7 +1163,8 @@ int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int
   if (nq < 1) return fail_with(SDG_E_ARG, "'X' must have at least one column.");
   sdg_dense* QD = nullptr;
   int* berr = nullptr;
-  int st = dense_build(ctx, Q, d, nq, true, false, &QD, &berr);
+  // an unsupported method is refused by the search, after the finiteness check
+  int st = query_build(ctx, Q, d, nq, method, &QD, &berr);
   if (st != SDG_OK) return st;
   st = dense_search(ctx, QD, 0, nq, D, false, method, k, mode, idx, dist_out, device_out, k_eff, flags, berr);
   if (st == SDG_OK) ctx_stats_add(ctx, 3, 4);        // the query block's prep, unit columns, cast, error norms
@@ -1045,7 +1176,6 @@ int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int
         cudaStreamSynchronize(QD->stream) == cudaSuccess && h)
       st = fail_with(SDG_E_NONFINITE, "Cosine requires finite input (found NA, NaN or Inf).");
   }
-  cudaFreeAsync(berr, QD->stream);
   sdg_dense_free(QD);
   return st;
 }
@@ -1055,7 +1185,7 @@ extern "C" {
 
 SDG_API int sdg_dense_upload(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, sdg_dense** out) {
   if (!ctx || !X || !out || d < 1 || n < 1) return fail_with(SDG_E_ARG, "invalid dense upload arguments");
-  return dense_build(ctx, X, d, n, false, true, out);
+  return dense_build(ctx, X, d, n, out);
 }
 
 SDG_API int sdg_dense_free(sdg_dense* D) {
@@ -1066,9 +1196,8 @@ SDG_API int sdg_dense_free(sdg_dense* D) {
                   (void*)D->ue, (void*)D->un, (void*)D->xe, (void*)D->xn,
                   (void*)(D->ubp != D->ub ? D->ubp : nullptr), (void*)(D->xbp != D->xb ? D->xbp : nullptr)};
   if (D->async) {
-    // a per-request matrix: stream-ordered frees after the work queued on its stream
-    for (void* p : bufs)
-      if (p) cudaFreeAsync(p, D->stream);
+    // a query block: one allocation, freed after the work queued on its stream
+    cudaFreeAsync(D->x64, D->stream);
   } else {
     cudaDeviceSynchronize();
     for (void* p : bufs)

@@ -37,7 +37,7 @@ struct sdg_dense {
   int64_t n_empty = 0;
   cublasHandle_t blas = nullptr;  // slab (mode 2) and plain (mode 1) GEMMs; resident references only
   std::mutex blas_mu;             // one caller at a time on `blas` (it is bound to a stream)
-  bool async = false;             // buffers from the stream-ordered pool of `stream`
+  bool async = false;             // a query block: one stream-ordered allocation (x64 its start) of `stream`
   cudaStream_t stream = nullptr;
 };
 

@@ -880,22 +880,40 @@ __global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_
 // rel (Nq + Nr), so lo = 2 s - (Nq + Nr) - 2 rel sqrt(Nq Nr) - 2^-20 (Nq + Nr) -
 // 1e-30 >= x' - (1 + c') Nq + 2^-20 (Nq + Nr) - 1e-30: the last but one term
 // covers the FP32 roundings of (1 + c') N, 2^-21 |x'| that of x' and of the
-// differences.  One block per query.
-__global__ void __launch_bounds__(256) k_tc_threshold(int method, int64_t q0, int m, int K, float rel,
+// differences.  A warp per query; the m maxima are first folded into 256 (the
+// k-th largest of the folded ones is reached by k references too, and for k <=
+// 64 it is hardly lower), which sit in registers for the bit search of kth::largest.
+__global__ void __launch_bounds__(256) k_tc_threshold(int method, int64_t q0, int64_t nq, int m, int K, float rel,
                                                       float one_plus_c, const float* qnorm2, const uint8_t* qempty,
                                                       const float* maxima, unsigned* tshared) {
-  extern __shared__ uint32_t tkeys[];
-  __shared__ uint32_t red[8];
-  const int64_t ql = blockIdx.x;
+  const int64_t ql = blockIdx.x * (int64_t)8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (ql >= nq) return;
   if (qempty[q0 + ql]) {
-    if (threadIdx.x == 0) tshared[ql] = fkey(-INFINITY);
+    if (lane == 0) tshared[ql] = fkey(-INFINITY);
     return;
   }
-  for (int i = threadIdx.x; i < m; i += 256) tkeys[i] = fkey(fmaxf(maxima[ql * m + i], -INFINITY));
-  __syncthreads();
-  const kth::Group<8> G{red};
-  const float x = fkey_value(kth::largest<8>(G, tkeys, m, K));
-  if (threadIdx.x == 0) {
+  const float* in = maxima + ql * m;
+  float v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = -INFINITY;
+  for (int i = lane; i < m; i += 256)
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (i + 32 * c < m) v[c] = fmaxf(v[c], in[i + 32 * c]);
+  uint32_t key[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) key[c] = fkey(v[c]);
+  uint32_t ans = 0;
+  for (int b = 31; b >= 0; --b) {
+    const uint32_t t = ans | (1u << b);
+    uint32_t n = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) n += key[c] >= t;
+    if (__reduce_add_sync(0xffffffffu, n) >= (uint32_t)K) ans = t;
+  }
+  const float x = fkey_value(ans);
+  if (lane == 0) {
     float T = -INFINITY;
     if (x > -INFINITY) {
       const float base = (method == COSINE) ? rel : one_plus_c * qnorm2[q0 + ql];
@@ -912,9 +930,8 @@ __global__ void __launch_bounds__(256) k_tc_threshold(int method, int64_t q0, in
 // 100, k = 15: 254 / 131; 3,000 x 60,000, d = 64, k = 30: 319 / 164; 500 x
 // 1,000,000, d = 128, k = 50: 622 / 280; 4,096 x 150,000, d = 256, k = 20: 490 /
 // 515; 1,024 x 800,000, d = 200, k = 20: 608 / 975; 1 x 400,000, d = 256: 60 / 80.
-constexpr int64_t TWO_PASS_MAXIMA = 12288;            // per query, held in shared memory
 bool two_passes(int64_t nq, int64_t n, int dpad, int k, int64_t tiles_per_cta, int64_t maxima) {
-  if (nq < 64 || maxima < 4 * (int64_t)k || maxima > TWO_PASS_MAXIMA) return false;
+  if (nq < 64 || maxima < 4 * (int64_t)k || maxima > INT32_MAX) return false;
   double pass_us = (double)tiles_per_cta * (dpad <= 128 ? 1.4 : 2.1);
   if (n * dpad * 2 > (int64_t)96 << 20) pass_us *= 1.4;
   return pass_us < 50.0 + 8.0 * k;
@@ -1072,12 +1089,9 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
       P1.w = wp;
       if (e == cudaSuccess) k_dense_tc<1, false, 1><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(qmap, rmap, P1);
       P.stall = 0;                                     // one launch is stalled at a time
-      const size_t tsm = sizeof(uint32_t) * (size_t)m;
-      if (tsm > 48 * 1024)
-        chk(cudaFuncSetAttribute(k_tc_threshold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
       if (e == cudaSuccess)
-        k_tc_threshold<<<(unsigned)nq, 256, tsm, s>>>(method, q0, (int)m, k, rel, opc, Q->norm2, Q->empty, maxima,
-                                                      tshared);
+        k_tc_threshold<<<(unsigned)((nq + 7) / 8), 256, 0, s>>>(method, q0, nq, (int)m, k, rel, opc, Q->norm2,
+                                                                Q->empty, maxima, tshared);
     }
     if (e == cudaSuccess) {
       if (pair) {

@@ -102,9 +102,12 @@ __global__ void k_unit_csc_warp(DevCsc M, double* uval, double* scale_out, int* 
 // lanes over the rows (prefix maximum of the magnitudes on their bit
 // patterns, which order non-negative doubles as integers), parks them in
 // shared memory, and then lane c runs column c's sum-of-squares chain over
-// the chunk in the reference's order.  The FP64 pipe issues one instruction
-// for cpw columns' chain steps instead of one per step; cpw (columns per
-// warp, <= 32) trades that against the number of warps for small n.
+// the chunk in the reference's order.  The FP64 pipe holds a scheduler 64
+// cycles per warp instruction: about 80 for a column's ratios and 160 for its
+// two closing divisions, and 256 (d = 256) for the chains of all cpw columns of
+// a warp, so cpw (columns per warp, <= 32) is as small as still gives every
+// scheduler a warp.  us, before (8 columns a warp, two divisions and the
+// squares in the chain) and now, d = 256: 1 column 40 and 31, 4,096 141 and 113.
 constexpr int UD_WARPS = 2;
 
 __global__ void __launch_bounds__(UD_WARPS * 32) k_unit_dense(int32_t d, int64_t n, int cpw, const double* x,
@@ -140,9 +143,11 @@ __global__ void __launch_bounds__(UD_WARPS * 32) k_unit_dense(int32_t d, int64_t
       uint8_t flag = 0;              // 0: skip (zero), 1: new maximum, 2: below maximum
       double r = 0.0;
       if (ab != 0) {
-        const double av = __longlong_as_double(ab), pv = __longlong_as_double(prev);
-        if (prev < ab) { flag = 1; r = pv / av; }
-        else { flag = 2; r = av / pv; }
+        // one division for either branch; below the maximum the chain adds r r
+        const bool up = prev < ab;
+        flag = up ? 1 : 2;
+        r = __longlong_as_double(up ? prev : ab) / __longlong_as_double(up ? ab : prev);
+        if (!up) r = dmul(r, r);
       }
       s_r[warp][lane][c] = r;
       s_f[warp][lane][c] = flag;
@@ -153,9 +158,9 @@ __global__ void __launch_bounds__(UD_WARPS * 32) k_unit_dense(int32_t d, int64_t
     if (lane < nc) {
       for (int t = 0; t < kn; ++t) {
         const uint8_t f = s_f[warp][t][lane];
-        const double rr = s_r[warp][t][lane];
+        const double rr = s_r[warp][t][lane];          // the ratio (new maximum) or its square
         if (f == 1) ssq = dadd(1.0, dmul(dmul(ssq, rr), rr));
-        else if (f == 2) ssq = dadd(ssq, dmul(rr, rr));
+        else if (f == 2) ssq = dadd(ssq, rr);
       }
     }
     __syncwarp();
@@ -1296,7 +1301,8 @@ void launch_unit_csc(const DevCsc& M, double* uval, double* scale, int* err, cud
 void launch_unit_dense(int32_t d, int64_t n, const double* x, double* uval, double* scale, int* err,
                        cudaStream_t s) {
   if (n <= 0) return;
-  const int cpw = (n >= (int64_t)152 * 64 * 32) ? 32 : 8;   // 32 once every SM has 64 warps' worth
+  // one warp per scheduler (4 x 152) for small n, 32 columns once every SM has 64 warps' worth
+  const int cpw = (n >= (int64_t)152 * 64 * 32) ? 32 : (int)std::min<int64_t>(8, (n + 607) / 608);
   const int64_t per_block = (int64_t)cpw * UD_WARPS;
   k_unit_dense<<<(unsigned)((n + per_block - 1) / per_block), UD_WARPS * 32, 0, s>>>(d, n, cpw, x, uval, scale,
                                                                                     err);
