@@ -66,11 +66,12 @@ constexpr uint32_t SLEEP_NS = 20000;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = gtimer();
+  uint64_t t0 = 0;                           // read after a while only: %globaltimer is slow
   for (uint32_t spin = 1;; ++spin) {
     if (mbar_try_wait_sleep(bar, parity, SLEEP_NS)) return true;
     if ((spin & 255u) == 0) {
       if (*abort_flag) return false;
+      if (!t0) t0 = gtimer();
       if (gtimer() - t0 > WAIT_NS) {
         *abort_flag = 1;
         atomicExch(status, 1);
