@@ -530,7 +530,7 @@ void knn_device(sdg_ctx* c, sdg_matrix* X, sdg_matrix* Y, int method, int dist, 
   KnnPlan P;
   P.method = method; P.dist = dist; P.k = k; P.decreasing = decreasing_for(method, dist);
   P.selfmode = selfmode; P.include_self = include_self != 0;
-  P.ref_mask = drop_degenerate ? ref->empty.as<uint8_t>() : nullptr;
+  P.ref_mask = drop_degenerate && ref->n_empty > 0 ? ref->empty.as<uint8_t>() : nullptr;
   P.qry_blank = drop_degenerate ? X->empty.as<uint8_t>() : nullptr;
 
   cudaStream_t s = c->stream;

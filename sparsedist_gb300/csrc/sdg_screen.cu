@@ -234,7 +234,8 @@ struct ScreenArgs {
   const int2* order;          // (local query, stretch), longest first
   const int32_t* units;       // their number
   int nparts, group;          // parts; parts of a group
-  float* S;                   // S[qlocal * nr + column]
+  int64_t ldS;
+  float* S;                   // S[qlocal * ldS + column]
   unsigned long long* work;   // work counter
 };
 
@@ -299,9 +300,9 @@ __global__ void __launch_bounds__(1024) k_screen_order(const int32_t* qnnz, int6
 }
 
 // The slab rows that several stretches add to start at zero.
-__global__ void k_screen_zero(const int32_t* qnnz, int64_t q_begin, int64_t nr, float* S) {
+__global__ void k_screen_zero(const int32_t* qnnz, int64_t q_begin, int64_t nr, int64_t ldS, float* S) {
   if (qnnz[q_begin + blockIdx.x] <= SCREEN_SEG) return;
-  float* row = S + (int64_t)blockIdx.x * nr;
+  float* row = S + (int64_t)blockIdx.x * ldS;
   for (int64_t c = threadIdx.x; c < nr; c += blockDim.x) row[c] = 0.f;
 }
 
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kScreenMaxWarps * 32, 1) k_screen_rows(ScreenA
         }
       }
     }
-    float* out = A.S + ql * A.nr + c0;
+    float* out = A.S + ql * A.ldS + c0;
     if (q1 - q0 > SCREEN_SEG) {
       for (int32_t i = lane; i < nc; i += 32) atomicAdd(out + i, acc[i]);
     } else {
@@ -456,8 +457,8 @@ __global__ void __launch_bounds__(kScreenMaxWarps * 32, 1) k_screen_rows(ScreenA
 // ---------------------------------------------------------------------------
 struct SelectScreenArgs {
   int method, k;
-  const float* S;
-  int64_t nr;
+  const float* S;                            // [qlocal * ldS + column], ldS a multiple of 4
+  int64_t nr, ldS;
   const int32_t* rnnz; const float* rnorm;
   const int32_t* qnnz; const float* qnorm;   // indexed by query column
   const double* rsum;                        // js: reference column sums
@@ -567,49 +568,97 @@ __device__ __forceinline__ void moment_key_and_bound(bool pearson, float s, int3
   err = (float)(0.5 * (hi - lo)) + 2.f * U32 * (fabsf(key) + 1.f) + 1e-30f;
 }
 
-// The key interval [lo, hi] of reference c from its screen value; false: not a
-// candidate.  KIND 0: binary / cosine / euclidean / manhattan, 1: js, 2:
-// pearson / covariance.  A key that is not finite has no lower bound and
-// stays a candidate (its exact value decides).
+// The key intervals [lo, hi] of four consecutive references from their screen
+// values; ok bit u: reference c + u is a candidate.  KIND 0: cosine, 1: euclidean /
+// manhattan, 2: binary, 3: js, 4: pearson / covariance.  For KIND 0 and 1 the
+// term count of the bound is the query's stored entries (min(nnz_q, nnz_c) is at
+// most that), so it is one number per query; KIND 2 divides with __fdividef (2
+// ulp: 4 u of the key, doubled here).  A key that is not finite has no lower
+// bound and stays a candidate (its exact value decides).
 template <int KIND>
-__device__ __forceinline__ bool screen_interval(const SelectScreenArgs& A, int64_t q, int64_t c, int32_t nq_, float Nq,
-                                                float sv, float& lo, float& hi) {
-  if (A.ref_mask && A.ref_mask[c]) return false;
-  if (A.selfmode && c == q && !(A.include_self && A.method == COVARIANCE)) {
-    // a restored self value (R/sparseKNN.R:270-279) is the best key; a
-    // covariance self pair keeps its computed value and is an ordinary pair
-    lo = hi = INFINITY;
-    return A.include_self != 0;
+struct ScreenBounds {
+  const SelectScreenArgs& A;
+  const int64_t q;
+  const int32_t nq_;
+  const float Nq, e, a;
+  __device__ __forceinline__ ScreenBounds(const SelectScreenArgs& A_, int64_t q_)
+      : A(A_), q(q_), nq_(A_.qnnz[q_]), Nq(A_.qnorm ? A_.qnorm[q_] : 0.f),
+        e(((float)nq_ + (KIND == 0 ? 40.f : 46.f)) * U32 * 1.01f + 1e-12f), a(A_.method == EUCLIDEAN ? 2.f : 1.f) {}
+  __device__ __forceinline__ unsigned operator()(int64_t c, int64_t end, const float4& sv, float (&lo)[4],
+                                                 float (&hi)[4]) const {
+    const float s[4] = {sv.x, sv.y, sv.z, sv.w};
+    float4 nc4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    int4 nn4 = make_int4(0, 0, 0, 0);
+    if (KIND == 1 || KIND == 3) nc4 = __ldg(reinterpret_cast<const float4*>(A.rnorm + c));
+    if (KIND >= 2) nn4 = __ldg(reinterpret_cast<const int4*>(A.rnnz + c));
+    const float Nc[4] = {nc4.x, nc4.y, nc4.z, nc4.w};
+    const int32_t nn[4] = {nn4.x, nn4.y, nn4.z, nn4.w};
+    unsigned ok = c + 3 < end ? 15u : (1u << (int)(end - c)) - 1u;
+    if (A.ref_mask) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (((ok >> u) & 1u) && A.ref_mask[c + u]) ok &= ~(1u << u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (KIND == 0) {
+        lo[u] = s[u] - e;
+        hi[u] = s[u] + e;
+        if (!(fabsf(s[u]) <= FLT_MAX)) { lo[u] = -INFINITY; hi[u] = INFINITY; }
+      } else {
+        float key = 0.f, err = 0.f;
+        if (KIND == 1) {
+          const float T = Nq + Nc[u];
+          key = fmaf(a, s[u], -T);
+          err = e * T + 1e-30f;
+        } else if (KIND == 2) {
+          const float denom = (float)(nq_ + nn[u]) - s[u];
+          key = (denom > 0.f) ? __fdividef(s[u], denom) : 1.f;
+          err = key * (8.f * U32) + 1e-30f;
+        } else if ((ok >> u) & 1u) {
+          if (KIND == 3)
+            js_key_and_bound(s[u], A.rsum[c + u], A.qsum[q], Nc[u], Nq, min(nq_, nn[u]), key, err);
+          else
+            moment_key_and_bound(A.method == PEARSON, s[u], min(nq_, nn[u]), A.nrow, A.rs[c + u], A.rss[c + u],
+                                 A.qs[q], A.qss[q], key, err);
+        }
+        lo[u] = key - err;
+        hi[u] = key + err;
+        if (!(fabsf(key) <= FLT_MAX) || !(err <= FLT_MAX)) { lo[u] = -INFINITY; hi[u] = INFINITY; }
+      }
+    }
+    if (A.selfmode && q >= c && q < c + 4 && !(A.include_self && A.method == COVARIANCE)) {
+      // a restored self value (R/sparseKNN.R:270-279) is the best key; a
+      // covariance self pair keeps its computed value and is an ordinary pair
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c + u == q) {
+          lo[u] = hi[u] = INFINITY;
+          if (!A.include_self) ok &= ~(1u << u);
+        }
+    }
+    return ok;
   }
-  float key, err;
-  const int32_t nc = A.rnnz[c];
-  if (KIND == 1)
-    js_key_and_bound(sv, A.rsum[c], A.qsum[q], A.rnorm[c], Nq, min(nq_, nc), key, err);
-  else if (KIND == 2)
-    moment_key_and_bound(A.method == PEARSON, sv, min(nq_, nc), A.nrow, A.rs[c], A.rss[c], A.qs[q], A.qss[q], key, err);
-  else
-    key_and_bound(A.method, sv, nq_, Nq, nc, A.rnorm ? A.rnorm[c] : 0.f, key, err);
-  lo = key - err;
-  hi = key + err;
-  if (!(fabsf(key) <= FLT_MAX) || !(err <= FLT_MAX)) { lo = -INFINITY; hi = INFINITY; }
-  return true;
-}
+};
 
-// One block per query, two passes over its screen values.  First: every
-// thread's largest pessimistic key in each of `slices` stretches of the row, at
-// least four times k of them where the row is that long; their k-th largest T0
-// (found by one warp) is reached by k columns, so it is at most T.  Second:
-// the columns whose optimistic key reaches T0 - margin are the candidates (few
-// more than those that reach T), and T, the k-th largest pessimistic key
+// One block per query, two passes over its screen values, four columns a load.
+// First: every thread's largest pessimistic key in each of `slices` stretches of
+// the row, at least four times k of them where the row is that long; their k-th
+// largest T0 (found by one warp) is reached by k columns, so it is at most T.
+// Second: the columns whose optimistic key reaches T0 - margin are the candidates
+// (few more than those that reach T), and T, the k-th largest pessimistic key
 // among them, makes the cut.  Should they exceed the table, the k-th of those
 // listed is a better T0 and the pass runs again.
 //
-// Bound by the loads' latency: a warp per query with k-long sorted
-// insertions, reading the norms through a column permutation, took 668 us for
-// 1,500 queries x 12,001 references and 1,174 us for 1,000 x 20,000.
+// Bound by the slab's read (the second pass finds its row in the L2) and, for
+// short rows, by the two bit searches.  us: 10,000 queries x 10,000 references
+// (binary) 655 with scalar loads, per-pair term counts and IEEE divisions, 296
+// now; 12,001 x 1,500 163 and 126; 1,500 x 12,001 121 and 52.  A warp per query
+// with k-long sorted insertions, reading the norms through a column permutation,
+// took 668 us for the last and 1,174 us for 1,000 x 20,000.
 template <int KIND, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A) {
-  constexpr int NT = WARPS * 32, V = 4;
+  constexpr int NT = WARPS * 32;
   extern __shared__ uint32_t keys[];                 // max(slices * NT, cap)
   __shared__ float s_t;
   __shared__ int s_n;
@@ -622,27 +671,21 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
     if (tid == 0) { A.count[ql] = 0; A.overflow[ql] = blank ? 0 : 1; }
     return;
   }
-  const int32_t nq_ = A.qnnz[q];
-  const float Nq = A.qnorm ? A.qnorm[q] : 0.f;
-  const float* Srow = A.S + ql * A.nr;
+  const ScreenBounds<KIND> bounds(A, q);
+  const float* Srow = A.S + ql * A.ldS;
+  const float4* S4 = reinterpret_cast<const float4*>(Srow);
   const kth::Group<1> G{nullptr};
-  const int64_t stretch = (A.nr + A.slices - 1) / A.slices;
+  const int64_t n4 = (A.nr + 3) / 4, stretch = (n4 + A.slices - 1) / A.slices;
   for (int sl = 0; sl < A.slices; ++sl) {
-    const int64_t c0 = sl * stretch, c1 = min(c0 + stretch, A.nr);
+    const int64_t g1 = min((sl + 1) * stretch, n4);
     float best = -INFINITY;
-    for (int64_t base = c0; base < c1; base += NT * V) {
-      float sv[V];
+#pragma unroll 2
+    for (int64_t g = sl * stretch + tid; g < g1; g += NT) {
+      float lo[4], hi[4];
+      const unsigned ok = bounds(4 * g, A.nr, S4[g], lo, hi);
 #pragma unroll
-      for (int u = 0; u < V; ++u) {
-        const int64_t c = base + u * NT + tid;
-        sv[u] = c < c1 ? Srow[c] : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < V; ++u) {
-        const int64_t c = base + u * NT + tid;
-        float lo, hi;
-        if (c < c1 && screen_interval<KIND>(A, q, c, nq_, Nq, sv[u], lo, hi)) best = fmaxf(best, lo);
-      }
+      for (int u = 0; u < 4; ++u)
+        if ((ok >> u) & 1u) best = fmaxf(best, lo[u]);
     }
     keys[sl * NT + tid] = kth::fkey(best);
   }
@@ -661,23 +704,17 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
     const float cut = cut_of(s_t);
     if (tid == 0) s_n = 0;
     __syncthreads();
-    for (int64_t base = 0; base < A.nr; base += NT * V) {
-      float sv[V];
+#pragma unroll 2
+    for (int64_t g = tid; g < n4; g += NT) {
+      float lo[4], hi[4];
+      const unsigned ok = bounds(4 * g, A.nr, S4[g], lo, hi);
 #pragma unroll
-      for (int u = 0; u < V; ++u) {
-        const int64_t c = base + u * NT + tid;
-        sv[u] = c < A.nr ? Srow[c] : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < V; ++u) {
-        const int64_t c = base + u * NT + tid;
-        float lo = -INFINITY, hi;
-        const bool keep = c < A.nr && screen_interval<KIND>(A, q, c, nq_, Nq, sv[u], lo, hi) && hi >= cut;
-        if (keep) {
+      for (int u = 0; u < 4; ++u) {
+        if (((ok >> u) & 1u) && hi[u] >= cut) {
           const int at = atomicAdd(&s_n, 1);
           if (at < A.cap) {
-            out[at] = (int32_t)c;
-            keys[at] = kth::fkey(lo);
+            out[at] = (int32_t)(4 * g + u);
+            keys[at] = kth::fkey(lo[u]);
           }
         }
       }
@@ -708,8 +745,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
         bool keep = false;
         if (t < n) {
           c = out[t];
-          float lo, hi;
-          keep = screen_interval<KIND>(A, q, c, nq_, Nq, Srow[c], lo, hi) && hi >= cut;
+          float lo[4], hi[4];
+          bounds(c & ~3, A.nr, S4[c >> 2], lo, hi);
+          const float h = (c & 2) ? ((c & 1) ? hi[3] : hi[2]) : ((c & 1) ? hi[1] : hi[0]);
+          keep = h >= cut;
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);   // every lane has read slot t first
         if (keep) out[kept + __popc(m & ((1u << lane) - 1u))] = c;
@@ -1184,7 +1223,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   // floats; the fused tensor screen writes no slab and takes 4,096 queries
   // (16 query groups of 256, about one CTA per SM at ~10 reference ranges)
   const int64_t sbudget = (int64_t)4 << 30;
-  const int64_t ldS = nr;
+  const int64_t ldS = (nr + 3) / 4 * 4;           // float4 rows for the select
   const int64_t chunk = use_t ? std::min<int64_t>(std::max<int64_t>(q_hi - q_lo, 1), 4096)
                               : std::max<int64_t>(16, std::min<int64_t>(std::max<int64_t>(q_hi - q_lo, 1),
                                                                          sbudget / (4 * std::max<int64_t>(ldS, 1))));
@@ -1268,7 +1307,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     int warps = 1;
     screen_shape(rc, nr, nrow, nb, nsm, &A.part_subs, &warps);
     A.rows = rc->rows; A.ent = static_cast<const int2*>(rc->ent); A.exl = rc->exl;
-    A.nsub = rc->nsub; A.lg = rc->sub_lg; A.nr = nr;
+    A.nsub = rc->nsub; A.lg = rc->sub_lg; A.nr = nr; A.ldS = ldS;
     A.qp = qry.p; A.qi = qry.i; A.qv = qc->fval; A.qxl = qc->fxl; A.q_begin = q0; A.nq = nb;
     A.nparts = (rc->nsub + A.part_subs - 1) / A.part_subs;
     // parts of a group: their entries (kScreenGroupBytes) stay in the L2
@@ -1278,7 +1317,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     SK(cudaMemsetAsync(work, 0, sizeof(*work), s));
     A.order = order; A.units = units;
     k_screen_order<<<1, 1024, 0, s>>>(qc->nnz, q0, nb, order, units);
-    k_screen_zero<<<(unsigned)nb, 256, 0, s>>>(qc->nnz, q0, nr, S);
+    k_screen_zero<<<(unsigned)nb, 256, 0, s>>>(qc->nnz, q0, nr, ldS, S);
     const size_t smem = sizeof(float) * (size_t)warps * ((size_t)A.part_subs << A.lg);
     auto kernel = r.method == MANHATTAN ? k_screen_rows<1> : r.method == JS ? k_screen_rows<2> : k_screen_rows<0>;
     // a function attribute is per device: set on every call (cheap, thread-safe)
@@ -1290,7 +1329,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     SK(cudaGetLastError());
 
     SelectScreenArgs B;
-    B.method = r.method; B.k = r.k; B.S = S; B.nr = nr;
+    B.method = r.method; B.k = r.k; B.S = S; B.nr = nr; B.ldS = ldS;
     const bool normed = r.method == EUCLIDEAN || r.method == MANHATTAN || r.method == JS;
     B.rnnz = rc->nnz; B.rnorm = normed ? rc->cnorm : nullptr;
     B.qnnz = qc->nnz; B.qnorm = normed ? qc->cnorm : nullptr;
@@ -1305,10 +1344,12 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     B.slices = std::max(1, (4 * r.k + nt - 1) / nt);
     const size_t ssmem = sizeof(uint32_t) * (size_t)std::max(B.slices * nt, cap);
     auto pick = [&](auto k8, auto k32) { return wide ? k32 : k8; };
-    auto select = (r.method == JS) ? pick(k_screen_select<1, 8>, k_screen_select<1, 32>)
+    auto select = r.method == COSINE ? pick(k_screen_select<0, 8>, k_screen_select<0, 32>)
+                  : r.method == BINARY ? pick(k_screen_select<2, 8>, k_screen_select<2, 32>)
+                  : r.method == JS ? pick(k_screen_select<3, 8>, k_screen_select<3, 32>)
                   : (r.method == PEARSON || r.method == COVARIANCE)
-                      ? pick(k_screen_select<2, 8>, k_screen_select<2, 32>)
-                      : pick(k_screen_select<0, 8>, k_screen_select<0, 32>);
+                      ? pick(k_screen_select<4, 8>, k_screen_select<4, 32>)
+                      : pick(k_screen_select<1, 8>, k_screen_select<1, 32>);
     select<<<(unsigned)nb, nt, ssmem, s>>>(B);
     SK(cudaGetLastError());
     }
