@@ -289,6 +289,8 @@ def _idx_matrix(idx):
         raise ValueError("'idx' must have at least one row and one column.")
     if idx.dtype.kind not in "iuf":
         raise ValueError("'idx' must be a numeric or integer matrix.")
+    if idx.dtype == np.int32 and idx.min() >= 1 and idx.max() <= n:      # every entry an index: nothing to map
+        return np.asfortranarray(idx), rown
     if idx.dtype.kind == "f":
         na = np.isnan(idx)
         v = np.where(na, 1.0, idx)
