@@ -149,6 +149,14 @@ __host__ __device__ __forceinline__ int64_t first_cta(int64_t g, int64_t ntiles,
 __host__ __device__ __forceinline__ int64_t last_cta(int64_t g, int64_t ntiles, int64_t per) {
   return ((g + 1) * ntiles - 1) / per;
 }
+// The reference tile of item f of group g.  A group's tiles are taken in cyclic
+// order from (g ntiles) mod per, so that every work unit, which starts at a
+// multiple of per, is at a tile congruent to its step number modulo per: at
+// any time the units together read about ntiles / per places of the reference
+// matrix instead of one place each.
+__host__ __device__ __forceinline__ int32_t tile_of(int64_t f, int64_t g, int64_t ntiles, int64_t per) {
+  return (int32_t)((f - g * ntiles + (g * ntiles) % per) % ntiles);
+}
 
 // MODE 0: the running lists described above, one pass over the references.
 // MODE 1 and 2: two passes for blocks whose pass is short.  MODE 1 keeps no
@@ -245,8 +253,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
           mbar_expect_tx(a_full, (uint32_t)dch * A_BYTES);
           for (int c = 0; c < dch; ++c) tma_load_2d(sA + (size_t)c * A_BYTES, &qmap, a_full, c * BK, qy);
         }
-        for (; f < fe && ok; ++f) {
-          const int rcol = (int)((f - g * ntiles) * BN + crank * C::BNL);
+        int32_t tile = tile_of(f, g, ntiles, per);
+        for (; f < fe && ok; ++f, tile = tile + 1 < (int32_t)ntiles ? tile + 1 : 0) {
+          const int rcol = tile * BN + (int)crank * C::BNL;
           for (int c = 0; c < dch; ++c, ++it) {
             const int s = it % STAGES;
             const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
@@ -548,12 +557,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
           active ? (ql * P.nslots + (unit - first_cta(g, ntiles, per)) * 2 + half) : 0;
       my_idx = P.eidx + slot * P.ecap;
       my_s = P.es + slot * P.ecap;
-      for (; f < fe; ++f, ++j) {
+      int32_t tile = tile_of(f, g, ntiles, per);
+      for (; f < fe; ++f, ++j, tile = tile + 1 < (int32_t)ntiles ? tile + 1 : 0) {
         const int buf = (int)(j & 1);
         const bool got = wait(acc_full + buf, (uint32_t)(j >> 1) & 1u);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }   // the warp leaves together
         fence_after();
-        const int64_t r_half = (f - g * ntiles) * BN + half * (BN / 2);
+        const int64_t r_half = (int64_t)tile * BN + half * (BN / 2);
         const uint32_t tb = tmem + lane_base + (uint32_t)(buf * BN + half * (BN / 2));
         // the buffer goes back to the MMAs as soon as its last TMEM reads are
         // done (the values being processed are in registers by then): the
@@ -582,8 +592,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             cm[hh + 1] = chunk_max(vb, r_half + hh * 32 + 32, weigh);
           }
           if (active) {
-            const int64_t tile = f - g * ntiles;
-            float* out = P.maxima + ql * (2 * ntiles * P.gran) + (tile * 2 + half) * P.gran;
+            float* out = P.maxima + ql * (2 * ntiles * P.gran) + ((int64_t)tile * 2 + half) * P.gran;
             if (P.gran == 4) *reinterpret_cast<float4*>(out) = make_float4(cm[0], cm[1], cm[2], cm[3]);
             else *out = fmaxf(fmaxf(cm[0], cm[1]), fmaxf(cm[2], cm[3]));
           }
