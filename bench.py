@@ -81,7 +81,7 @@ def parse():
     ap.add_argument("--serve-ref-cols", type=int, default=1000000)
     ap.add_argument("--dense-cols", type=int, default=2000000)
     ap.add_argument("--dense-mode", type=int, default=0, choices=[0, 3],
-                    help="BF16-screened mode of the dense line: 0 (one CTA per query group), 3 (CTA pairs)")
+                    help="BF16-screened mode of the dense line: 0, 3 (CTA pairs wherever possible)")
     ap.add_argument("--dense-block", type=int, default=4096)
     ap.add_argument("--dense-cpu-cols", type=int, default=128,
                     help="query columns of the dense CPU-baseline / parity sample")
@@ -937,7 +937,7 @@ def run_logcount(args):
                 "kernel": "k_sparse_tc (fused FP16 tcgen05 screen)", "flops_per_launch": flops_launch}
     else:
         roof = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
-                "peak_kind": peak_kind, "kernel": "k_screen", "alg_bytes_per_launch": alg / launches_per_step}
+                "peak_kind": peak_kind, "kernel": "k_screen_rows", "alg_bytes_per_launch": alg / launches_per_step}
     roof["frac"] = (roof["achieved"] / roof["peak"]) if roof["achieved"] else None
     roof["traffic"] = LOGCOUNT_TRAFFIC if (roof["bound"] == "tensor" and args.ncol == 200000 and
                                           args.nrow == 30000 and B == 4096) else None

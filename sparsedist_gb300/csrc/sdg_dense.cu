@@ -957,7 +957,7 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
   }
   const int cap = std::max(512, std::min(16384, 64 * k + 256));
   // modes 0 and 3 run the fused tensor-core screen where it applies (no slab
-  // in HBM; mode 0 one CTA per query group, mode 3 on CTA pairs), else the
+  // in HBM; mode 3 always on CTA pairs, mode 0 where they are faster), else the
   // BF16 slab screen of mode 2; smode is the bound in force
   const bool fused = (mode == 0 || mode == 3) && tc_screen_supported(D, method, k);
   const int smode = (mode == 1) ? 1 : 0;
@@ -1133,12 +1133,12 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
   if (!device_out) { DK(cudaFreeAsync(o_idx, s)); DK(cudaFreeAsync(o_val, s)); }
   DK(cudaStreamSynchronize(s));
   ctx_add_overflow(ctx, (int64_t)overflow.size());
-  // kernels per chunk: the screen (fused: key init, weights, k_dense_tc, merge;
-  // slab: the GEMM, segtop, thresh, keep, overflow), the FP32 cut (scan, dot,
-  // cut) and the scan of the exact values, the exact values and the
-  // selection; two more per overflowing query
+  // kernels per chunk: the screen (the fused one counts its own; slab: the
+  // GEMM, segtop, thresh, keep, overflow), the FP32 cut (scan, dot, cut) and
+  // the scan of the exact values, the exact values and the selection; two more
+  // per overflowing query
   const int64_t chunks = (nq + chunk - 1) / chunk;
-  ctx_stats_add(ctx, 3, chunks * ((fused ? 4 : 5) + (smode == 0 ? 4 : 0) + 2) + 2 * (int64_t)overflow.size());
+  ctx_stats_add(ctx, 3, chunks * ((fused ? 0 : 5) + (smode == 0 ? 4 : 0) + 2) + 2 * (int64_t)overflow.size());
   return SDG_OK;
 }
 
@@ -1151,9 +1151,11 @@ int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int k) {
   const int64_t cap = std::max(512, std::min(16384, 64 * k + 256));
   // the query's forms (FP64 x2, FP32 x2, BF16 x2 + padded), candidates and
   // exact values, results, and the fused screen's per-(query, range) lists
-  // (at most 152 ranges for a single query tile, ~9 for full tiles)
+  // (at most 152 ranges for a single query tile, ~9 for full tiles), the
+  // sample's maxima
   const int64_t ranges = std::max<int64_t>(9, 152 / std::max<int64_t>(1, (nq + 255) / 256));
-  return nq * (36 * (int64_t)D->dpad + cap * 12 + (int64_t)k * 12 + ranges * (768 * 8 + (int64_t)k * 4 + 4)) +
+  return nq * (36 * (int64_t)D->dpad + cap * 12 + (int64_t)k * 12 + ranges * (768 * 8 + (int64_t)k * 4 + 4) +
+               D->n / 96 + 128 * (int64_t)k) +
          ((int64_t)1 << 20);
 }
 int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int64_t nq, int method, int k,
@@ -1167,7 +1169,7 @@ int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int
   int st = query_build(ctx, Q, d, nq, method, &QD, &berr);
   if (st != SDG_OK) return st;
   st = dense_search(ctx, QD, 0, nq, D, false, method, k, mode, idx, dist_out, device_out, k_eff, flags, berr);
-  if (st == SDG_OK) ctx_stats_add(ctx, 3, 4);        // the query block's prep, unit columns, cast, error norms
+  if (st == SDG_OK) ctx_stats_add(ctx, 3, method == COSINE ? 3 : 1);   // prep; the unit columns and their copies
   if (st != SDG_OK && st != SDG_E_NONFINITE) {
     // an argument error found before the flag was read: non-finite input
     // still takes precedence, as when the build checked it at once

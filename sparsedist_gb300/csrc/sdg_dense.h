@@ -74,8 +74,8 @@ __device__ __forceinline__ float dense_cut(float T) {
 // Queries are columns q0.. of Q, references the columns of D (self: Q is D
 // and each query's own column is skipped).
 bool tc_screen_supported(const sdg_dense* D, int method, int k);
-// allow_pairs: run CTA pairs (cta_group::2, M = 256) where the block has more
-// than one 128-query group; otherwise one CTA per query group.  status: a
+// allow_pairs: run CTA pairs (cta_group::2, M = 256) wherever the block has
+// more than one 128-query group; otherwise where they are faster.  status: a
 // device int that a pipeline wait which ran out sets to 1; the call returns
 // without synchronising and the caller reads it with the results.
 int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, int method, int k, int64_t q0,

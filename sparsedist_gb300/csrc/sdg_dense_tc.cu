@@ -11,23 +11,23 @@
 //
 // Per segment the query group's 128 x d BF16 columns are loaded into shared
 // memory once (TMA, SWIZZLE_128B, K-major, 64-row chunks); reference tiles of
-// 256 columns x 64 rows stream through a four-stage TMA ring.  One thread
-// issues tcgen05.mma.cta_group::1.kind::f16 (M = 128 queries, N = 256
-// references, K = 16, BF16 in, FP32 accumulate) into TMEM: two accumulator
+// 256 columns x 64 rows stream through a four-stage TMA ring.  One lane of the
+// issuing warp issues tcgen05.mma.cta_group::1.kind::f16 (M = 128 queries, N =
+// 256 references, K = 16, BF16 in, FP32 accumulate) into TMEM: two accumulator
 // buffers of 256 columns fill all 512, so the MMAs of tile j + 1 run while
 // the epilogue reads tile j back with tcgen05.ld.
 //
 // Epilogue: eight warps; warp w reads TMEM lanes 32 (w % 4) .. + 31 (its 32
 // queries) and one half of the tile's 256 columns ((w - 2) / 4).  A thread
-// owns one (query, column half): it keeps the top k pessimistic keys of its
-// half of the segment's references in registers and appends every reference
-// whose optimistic key reaches its running cut to a per-(query, segment,
-// half) list.  The running cut is the k-th best of a subset, never above the
-// query's final cut, so the union of the lists holds every reference that the
-// slab screen keeps; k_tc_merge applies the final cut (the k-th best over all
-// the query's lists) exactly as the slab screen does, then a second, tighter
-// cut from per-pair bounds (the columns' BF16 rounding-error norms) on the
-// candidates alone.
+// owns one (query, column half) and appends every reference whose optimistic
+// key reaches its cut to a per-(query, segment, half) list.  The cut is never
+// above the query's final one, so the union of the lists holds every reference
+// that the slab screen keeps; k_tc_merge applies the final cut, then a second,
+// tighter one from per-pair bounds (the columns' BF16 rounding-error norms) on
+// the candidates alone.  Where the cut comes from is the MODE of the kernel:
+// a threshold from a sample of the references (a first launch), or, where
+// there are too few references to sample, the k-th best pessimistic key of the
+// thread's own share so far, kept as a sorted list in registers.
 //
 // Hot test.  An epilogue thread tests x = a s - w[r] against one threshold
 // e_thr per query (a = 1, w = 0 for cosine; a = 2, w = (1 - c) Nr for
@@ -36,12 +36,19 @@
 // 2 rel sqrt(Nq Nr) <= rel (Nq + Nr), so hi <= 2 s - (1 - c)(Nq + Nr) + 1e-30
 // and hi >= cut implies x >= cut + (1 - c) Nq; for cosine hi = s + rel.
 // e_thr subtracts 2^-12 (|cut| + Nq) (euclidean) or 2^-12 (|cut| + 1)
-// (cosine) more, far above the FP32 rounding of x.  The test's maximum, the
-// pass mask and the pick of a passing value are trees five levels deep, and
-// two 32-column chunks are tested together.  Passing references wait in eight
-// shared-memory slots per thread and are processed by the whole warp at once
-// when some lane's slots run out, so the slow path (key bounds, append,
-// sorted insert) runs with most lanes active.
+// (cosine) more, far above the FP32 rounding of x.  Two 32-column chunks are
+// tested together: their maxima (trees of three-input maxima), one vote, and
+// only in a chunk that holds a passing reference the mask and the picks.  The
+// weights of a tile half are fetched a tile ahead, one load per warp, and read
+// from shared memory: read from global memory where they are used they cost
+// the euclidean launch 5,165 us instead of 3,690 (4,096 x 2,000,000, d = 256).
+//
+// What bounds it: 4,096 x 2,000,000, cosine, k = 20, both launches: d = 256
+// 2.28 ms (3.18 before the sample, the issue loop of one elected lane and
+// pairs), d = 128 1.65 (2.65), d = 64 1.44 (2.50); euclidean d = 256 2.89
+// (5.17).  At d = 256 the tensor pipe: 1.23 us for 128 x 256 x 256 products, 1.1
+// times the rate of a measured cuBLAS burst; up to d = 128 the epilogue, which
+// tests 32,768 keys a tile in 0.8 us.
 //
 // Warp roles (320 threads): warp 0 TMA producer, warp 1 TMEM allocator + MMA
 // issuer, warps 2..9 epilogue.  Every mbarrier wait is bounded (1 s of
@@ -49,7 +56,7 @@
 // runs out sets *status, raises the CTA's abort flag, and the CTA drains its
 // own copies and MMAs, frees TMEM and returns.
 //
-// CTA pairs (PAIR = true, dense mode 3).  A cluster of two CTAs shares each
+// CTA pairs (PAIR = true).  A cluster of two CTAs shares each
 // UMMA: the even CTA issues tcgen05.mma.cta_group::2 with M = 256 (its 128
 // queries in rows 0-127, the odd CTA's in 128-255) and N = 256, each CTA
 // holding its own query tile and one 128-column half of every reference chunk
@@ -58,10 +65,6 @@
 // odd CTA's epilogue releases the even CTA's accumulator barrier remotely;
 // TMEM is allocated and freed by a warp of each CTA, and a cluster barrier
 // keeps either CTA from leaving while the other may still touch its memory.
-// Measured on the 256 x 2,000,000 workload it is no faster than one CTA per
-// group (3.55 against 3.41 ms): the loop is bound by the per-tile hand-off
-// between the MMAs and the epilogue through the two TMEM buffers, not by the
-// reference chunks' supply that the pairs halve.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -92,7 +95,9 @@ constexpr uint32_t TMEM_COLS = 2 * BN;         // two accumulator buffers
 constexpr int MAX_DCH = 4;              // dpad <= 256
 constexpr int MAX_STAGES = 8;
 // 1 KB alignment slack, A chunks, B ring, candidate slots, barriers
-constexpr size_t SMEM_BYTES = 1024 + (size_t)MAX_DCH * A_BYTES + RING_BYTES + (size_t)NB * EPI_THREADS * 8 + 256;
+constexpr uint32_t W_BYTES = BN / 2 * 4;     // an epilogue warp's weights of one tile half
+constexpr size_t SMEM_BYTES = 1024 + (size_t)MAX_DCH * A_BYTES + RING_BYTES + (size_t)NB * EPI_THREADS * 8 +
+                              EPI_THREADS / 32 * W_BYTES + 256;
 
 // One CTA (PAIR = false): a query group is 128 queries, the CTA loads whole
 // 256-column reference chunks (32 KB, a 4-stage ring) and issues
@@ -127,6 +132,7 @@ struct TcArgs {
   float* lists;               // [nq][nslots][k] (one pass)
   float* maxima;              // MODE 1: [nq][2 * ntiles * gran]
   int gran;                   // MODE 1: maxima per tile half (1 or 4)
+  int sample;                 // MODE 1: the sample's stride (sampled)
   int use_w;                  // MODE 1, cosine: some reference is degenerate
   int32_t* ecount;            // [nq][nslots]
   int32_t* eidx;              // [nq][nslots][ecap]
@@ -140,6 +146,27 @@ struct TcArgs {
 using kth::fkey;
 using kth::fkey_value;
 constexpr int SHARE_TILES = 8;          // tiles between exchanges of the shared running key
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// two FMAs in one instruction, each rounded as fmaf
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a NaN loses to a number, as in fmaxf
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 // the first and the last work unit (a CTA, or a CTA pair) whose span holds an
 // item of query group g
@@ -158,18 +185,24 @@ __host__ __device__ __forceinline__ int32_t tile_of(int64_t f, int64_t g, int64_
   return (int32_t)((f - g * ntiles + (g * ntiles) % per) % ntiles);
 }
 
-// MODE 0: the running lists described above, one pass over the references.
-// MODE 1 and 2: two passes for blocks whose pass is short.  MODE 1 keeps no
-// list: every thread stores the largest x' = a s - w[r] of each tile half (or of
-// each of its four 32-column chunks) with w[r] chosen so that x' less a
-// constant of the query is at most the reference's pessimistic key
-// (k_tc_maxima); the k-th largest of a query's maxima (k_tc_threshold) is then
-// reached by k references, so it is at most the k-th best key, and with several
-// times k maxima hardly below it.  MODE 2 appends the references that pass the
-// hot test at that threshold.  A running list starts from nothing in every CTA
-// and column half: for 777 queries x 150,001 references each of a query's 44
-// lists saw 3,500 references and took the slow path for a hundred of them, 80 %
-// of the launch's instructions.
+// Column c of a sample of stride s is reference c s + (c / BN) mod s: every
+// s-th reference, from another place in each tile, so that references stored in
+// turn by class (period s, or a multiple or divisor of it) are sampled alike.
+__host__ __device__ __forceinline__ int64_t sampled(int64_t c, int s) { return c * s + (c / BN) % s; }
+
+// MODE 0: running lists, one pass over the references; for few references.
+// MODE 1 keeps no list: every thread stores the largest x' = a s - w[r] of each
+// tile half (or of each of its four 32-column chunks) of a sample of the
+// references, with w[r] chosen so that x' less a constant of the query is at
+// most the reference's pessimistic key; the k-th largest of a query's maxima
+// (k_tc_threshold) is then reached by k references, so it is at most the k-th
+// best key, and with many times k maxima hardly below the sample's.
+// MODE 2 (cosine) and 3 (euclidean) append the references that pass the hot
+// test at that threshold.  A running list starts from nothing in every CTA and
+// column half: for 777 queries x 150,001 references each of a query's 44 lists
+// saw 3,500 references and took the slow path for a hundred of them, 80 % of
+// the launch's instructions; 4,096 x 2,000,000 still appended 2,147 references
+// a query where a sample of every 16th leaves 488.
 template <int KL, bool PAIR, int MODE>
 __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__ CUtensorMap qmap,
                                                        const __grid_constant__ CUtensorMap rmap, TcArgs P) {
@@ -184,7 +217,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
   // warp's accesses to one slot are conflict-free
   int32_t* buf_r = (int32_t*)(sB + (size_t)RING_BYTES);
   float* buf_s = (float*)(buf_r + NB * EPI_THREADS);
-  uint64_t* bars = (uint64_t*)(buf_s + NB * EPI_THREADS);
+  float* wts = buf_s + NB * EPI_THREADS;                   // per epilogue warp: -w of its tile half
+  uint64_t* bars = (uint64_t*)(wts + EPI_THREADS / 32 * (W_BYTES / 4));
   uint64_t* full = bars;
   uint64_t* emptyb = bars + MAX_STAGES;
   uint64_t* acc_full = bars + 2 * MAX_STAGES;
@@ -262,10 +296,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             if (!wait(emptyb + s, ph ^ 1u)) { ok = false; break; }
             if constexpr (PAIR) {
               if (leader) mbar_expect_tx(full + s, 2u * B_BYTES);
-              tma_load_2d_pair(sB + (size_t)s * B_BYTES, &rmap, cluster_addr(full + s, 0), c * BK, rcol);
+              const uint32_t bar = cluster_addr(full + s, 0);
+              if constexpr (MODE == 1)
+                tma_load_3d_pair(sB + (size_t)s * B_BYTES, &rmap, bar, c * BK, tile % P.sample, rcol);
+              else
+                tma_load_2d_pair(sB + (size_t)s * B_BYTES, &rmap, bar, c * BK, rcol);
             } else {
               mbar_expect_tx(full + s, B_BYTES);
-              tma_load_2d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, rcol);
+              if constexpr (MODE == 1)
+                tma_load_3d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, tile % P.sample, rcol);
+              else
+                tma_load_2d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, rcol);
             }
           }
         }
@@ -281,24 +322,28 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
     __syncwarp();
   } else if (warp == 1) {
     if (!PAIR || leader) {
-      // ---- MMA issuer ----
-      if (lane == 0 && f1 > f0) {
+      // ---- MMA issuer: the whole warp walks the loop, one lane issues ----
+      if (f1 > f0) {
+        const bool one = elect_one();
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
+          return __all_sync(0xffffffffu, wait(bar, parity));
+        };
+        const uint32_t a_lo = sw128_desc_lo(smem_u32(sA)), b_lo = sw128_desc_lo(smem_u32(sB));
         int it = 0, seg = 0;
         int64_t j = 0;
         bool ok = true;
         for (int64_t f = f0; f < f1 && ok; ++seg) {
           const int64_t g = f / ntiles;
           const int64_t fe = min(f1, (g + 1) * ntiles);
-          if (!wait(a_full, (uint32_t)seg & 1u)) break;
+          if (!wait_all(a_full, (uint32_t)seg & 1u)) break;
           fence_after();
-          const uint32_t a0 = smem_u32(sA);
           for (; f < fe && ok; ++f, ++j) {
             const int buf = (int)(j & 1);
             // the epilogue has drained this buffer's previous tile
             // (with P.stall the first wait asks for the phase the epilogue has not
             // begun, so it runs out: the failure-detection test's path)
             const uint32_t flip = (P.stall && j == 0) ? 0u : 1u;
-            if (!wait(acc_empty + buf, ((uint32_t)(j >> 1) & 1u) ^ flip)) {
+            if (!wait_all(acc_empty + buf, ((uint32_t)(j >> 1) & 1u) ^ flip)) {
               ok = false;
               break;
             }
@@ -307,31 +352,37 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             for (int c = 0; c < dch; ++c, ++it) {
               const int s = it % STAGES;
               const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-              if (!wait(full + s, ph)) { ok = false; break; }
+              if (!wait_all(full + s, ph)) { ok = false; break; }
               fence_after();
-              const uint32_t b_addr = smem_u32(sB + (size_t)s * B_BYTES);
-              const uint32_t a_addr = a0 + (uint32_t)c * A_BYTES;
+              const uint32_t al = a_lo + (uint32_t)c * (A_BYTES >> 4), bl = b_lo + (uint32_t)s * (B_BYTES >> 4);
+              if (one) {
 #pragma unroll
-              for (int kk = 0; kk < BK / 16; ++kk) {
-                if constexpr (PAIR)
-                  umma_f16_pair(d_addr, sw128_desc(a_addr + kk * 32), sw128_desc(b_addr + kk * 32), C::IDESC,
-                                (c | kk) != 0);
-                else
-                  umma_f16(d_addr, sw128_desc(a_addr + kk * 32), sw128_desc(b_addr + kk * 32), C::IDESC,
-                           (c | kk) != 0);
+                for (int kk = 0; kk < BK / 16; ++kk) {
+                  if constexpr (PAIR) umma_f16_pair(d_addr, al + kk * 2, bl + kk * 2, C::IDESC, (c | kk) != 0);
+                  else umma_f16(d_addr, al + kk * 2, bl + kk * 2, C::IDESC, (c | kk) != 0);
+                }
+                // the stage is free (in both CTAs of a pair) once these MMAs have read it
+                if constexpr (PAIR) umma_commit_pair(emptyb + s, 3); else umma_commit(emptyb + s);
+                // after the last chunk: the tile's accumulators are complete
+                if (c == dch - 1) {
+                  if constexpr (PAIR) umma_commit_pair(acc_full + buf, 3); else umma_commit(acc_full + buf);
+                }
               }
-              // the stage is free (in both CTAs of a pair) once these MMAs have read it
-              if constexpr (PAIR) umma_commit_pair(emptyb + s, 3); else umma_commit(emptyb + s);
+              __syncwarp();
             }
             if (!ok) break;
-            // the tile's accumulators are complete
-            if constexpr (PAIR) umma_commit_pair(acc_full + buf, 3); else umma_commit(acc_full + buf);
           }
           // the query chunks are free once the segment's MMAs are done
-          if constexpr (PAIR) umma_commit_pair(a_empty, 3); else umma_commit(a_empty);
+          if (one) {
+            if constexpr (PAIR) umma_commit_pair(a_empty, 3); else umma_commit(a_empty);
+          }
+          __syncwarp();
         }
         // all issued MMAs complete before TMEM is freed
-        if constexpr (PAIR) umma_commit_pair(mma_done, 3); else umma_commit(mma_done);
+        if (one) {
+          if constexpr (PAIR) umma_commit_pair(mma_done, 3); else umma_commit(mma_done);
+        }
+        __syncwarp();
         drain(mma_done, 0);
       }
     } else if constexpr (PAIR) {
@@ -347,7 +398,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
     const int K = P.k;
     const int32_t d = P.d;
     const float rel = 0.0040f + (float)d * 2.384185791015625e-7f;
-    const bool cosine = P.method == COSINE;
+    // known at compile time where references are appended (see MODE)
+    const bool cosine = MODE == 2 || (MODE != 3 && P.method == COSINE);
+    constexpr bool APPEND = MODE >= 2;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int et = threadIdx.x - 64;                  // epilogue thread 0 .. 255
 
@@ -416,33 +469,37 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       nbuf = 0;
       __syncwarp();
     };
-    // The hot test of one 32-reference chunk: the mask of the references with
-    // x >= e_thr (0 for an inactive lane); maximum and mask as trees.
-    auto hot_mask = [&](const uint32_t (&v)[32], int64_t r0) -> uint32_t {
-      if (!active) return 0u;
-      float x[32];
-      if (cosine) {
+    // The hot test's x of one 32-reference chunk at column c0 of the tile half
+    float* sw = wts + (warp - 2) * (W_BYTES / 4);
+    const uint64_t aa = pack2(P.a, P.a);
+    auto values = [&](const uint32_t (&v)[32], int c0, bool weigh, float (&x)[32]) {
+      if (weigh) {
+        const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(sw + c0);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const ulonglong2 ww = w2[t];
+          unpack2(fma2(aa, pack2(__uint_as_float(v[4 * t]), __uint_as_float(v[4 * t + 1])), ww.x), x[4 * t],
+                  x[4 * t + 1]);
+          unpack2(fma2(aa, pack2(__uint_as_float(v[4 * t + 2]), __uint_as_float(v[4 * t + 3])), ww.y), x[4 * t + 2],
+                  x[4 * t + 3]);
+        }
+      } else {
 #pragma unroll
         for (int t = 0; t < 32; ++t) x[t] = __uint_as_float(v[t]);
-      } else {
-        const float4* w4 = reinterpret_cast<const float4*>(P.w + r0);
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 ww = __ldg(w4 + j4);
-          x[4 * j4 + 0] = fmaf(P.a, __uint_as_float(v[4 * j4 + 0]), -ww.x);
-          x[4 * j4 + 1] = fmaf(P.a, __uint_as_float(v[4 * j4 + 1]), -ww.y);
-          x[4 * j4 + 2] = fmaf(P.a, __uint_as_float(v[4 * j4 + 2]), -ww.z);
-          x[4 * j4 + 3] = fmaf(P.a, __uint_as_float(v[4 * j4 + 3]), -ww.w);
-        }
       }
-      float m[16];
+    };
+    auto maximum = [](const float (&x)[32]) -> float {
+      float m[11];
 #pragma unroll
-      for (int t = 0; t < 16; ++t) m[t] = fmaxf(x[2 * t], x[2 * t + 1]);
+      for (int t = 0; t < 10; ++t) m[t] = max3(x[3 * t], x[3 * t + 1], x[3 * t + 2]);
+      m[10] = fmaxf(x[30], x[31]);
 #pragma unroll
-      for (int wdt = 8; wdt > 0; wdt >>= 1)
-#pragma unroll
-        for (int t = 0; t < wdt; ++t) m[t] = fmaxf(m[t], m[t + wdt]);
-      if (!(m[0] >= e_thr)) return 0u;
+      for (int t = 0; t < 3; ++t) m[t] = max3(m[3 * t], m[3 * t + 1], m[3 * t + 2]);
+      m[3] = fmaxf(m[9], m[10]);
+      return fmaxf(max3(m[0], m[1], m[2]), m[3]);
+    };
+    // the bits t of x[t] >= e_thr
+    auto mask_of = [&](const float (&x)[32]) -> uint32_t {
       uint32_t b[16];
 #pragma unroll
       for (int t = 0; t < 16; ++t)
@@ -452,6 +509,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
 #pragma unroll
         for (int t = 0; t < wdt; ++t) b[t] |= b[t + wdt];
       return b[0];
+    };
+    // The mask of the references of one chunk with x >= e_thr (0 for an
+    // inactive lane); the warp leaves together when no lane's maximum passes
+    auto hot_mask = [&](const uint32_t (&v)[32], int c0) -> uint32_t {
+      float x[32];
+      values(v, c0, !cosine, x);
+      const bool hit = active && maximum(x) >= e_thr;
+      if (!__any_sync(0xffffffffu, hit)) return 0u;
+      return hit ? mask_of(x) : 0u;
     };
     // v[jj] as a five-level tree of selects on the bits of jj
     auto pick = [](const uint32_t (&v)[32], int jj) -> float {
@@ -489,8 +555,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       __syncwarp();
     };
 
-    // MODE 2: the passing references of one chunk straight to the list
-    auto append = [&](const uint32_t (&v)[32], uint32_t mask, int64_t r0) {
+    // MODE 2: a chunk's passing references straight to the list; mx: this
+    // lane's maximum (-inf for an inactive lane).  x is formed again where a
+    // lane passes: held since the test, a pair's would be 64 more registers.
+    auto append = [&](const uint32_t (&v)[32], float mx, int c0, int64_t r0) {
+      if (!__any_sync(0xffffffffu, mx >= e_thr)) return;
+      float x[32];
+      values(v, c0, !cosine, x);
+      uint32_t mask = mx >= e_thr ? mask_of(x) : 0u;
       while (mask) {
         const int jj = __ffs(mask) - 1;
         mask &= mask - 1;
@@ -502,37 +574,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       }
       __syncwarp();
     };
+    int64_t own = -1;                                 // MODE 1: the query's own column of the sample
     // MODE 1: the largest x' of one chunk; weigh: subtract w[r] (+inf for
     // degenerate and padding references)
-    auto chunk_max = [&](const uint32_t (&v)[32], int64_t r0, bool weigh) -> float {
+    auto chunk_max = [&](const uint32_t (&v)[32], int64_t r0, int c0, bool weigh) -> float {
       float x[32];
-      if (weigh) {
-        const float4* w4 = reinterpret_cast<const float4*>(P.w + r0);
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 ww = __ldg(w4 + j4);
-          x[4 * j4 + 0] = fmaf(P.a, __uint_as_float(v[4 * j4 + 0]), -ww.x);
-          x[4 * j4 + 1] = fmaf(P.a, __uint_as_float(v[4 * j4 + 1]), -ww.y);
-          x[4 * j4 + 2] = fmaf(P.a, __uint_as_float(v[4 * j4 + 2]), -ww.z);
-          x[4 * j4 + 3] = fmaf(P.a, __uint_as_float(v[4 * j4 + 3]), -ww.w);
-        }
-      } else {
-#pragma unroll
-        for (int t = 0; t < 32; ++t) x[t] = __uint_as_float(v[t]);
-      }
-      if (P.self && __any_sync(0xffffffffu, q >= r0 && q < r0 + 32)) {
+      values(v, c0, weigh, x);
+      if (P.self && __any_sync(0xffffffffu, own >= r0 && own < r0 + 32)) {
 #pragma unroll
         for (int t = 0; t < 32; ++t)
-          if (r0 + t == q) x[t] = -INFINITY;
+          if (r0 + t == own) x[t] = -INFINITY;
       }
-      float m[16];
-#pragma unroll
-      for (int t = 0; t < 16; ++t) m[t] = fmaxf(x[2 * t], x[2 * t + 1]);
-#pragma unroll
-      for (int wdt = 8; wdt > 0; wdt >>= 1)
-#pragma unroll
-        for (int t = 0; t < wdt; ++t) m[t] = fmaxf(m[t], m[t + wdt]);
-      return m[0];
+      return maximum(x);
+    };
+    // this lane's four weights of the tile half that comes next
+    const bool weighted = !cosine || MODE == 1;
+    float4 wn = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch_w = [&](int32_t tile) {
+      if (weighted) wn = __ldg(reinterpret_cast<const float4*>(P.w + (int64_t)tile * BN + half * (BN / 2)) + lane);
     };
 
     int64_t j = 0;                                    // tile counter (the MMA's order)
@@ -545,6 +604,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       active = ql < P.nq;
       if (active) active = !P.qempty[q];           // a degenerate query has no list
       Nq = active ? P.qnorm2[q] : 0.f;
+      if (MODE == 1) own = sampled(q / P.sample, P.sample) == q ? q / P.sample : -1;
 #pragma unroll
       for (int i = 0; i < KL; ++i) lst[i] = (i < KL - K) ? INFINITY : -INFINITY;
       T = -INFINITY;
@@ -558,7 +618,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       my_idx = P.eidx + slot * P.ecap;
       my_s = P.es + slot * P.ecap;
       int32_t tile = tile_of(f, g, ntiles, per);
-      for (; f < fe; ++f, ++j, tile = tile + 1 < (int32_t)ntiles ? tile + 1 : 0) {
+      fetch_w(tile);
+      for (int32_t next = 0; f < fe; ++f, ++j, tile = next) {
+        next = tile + 1 < (int32_t)ntiles ? tile + 1 : 0;
+        if (weighted) {
+          __syncwarp();
+          reinterpret_cast<float4*>(sw)[lane] = make_float4(-wn.x, -wn.y, -wn.z, -wn.w);
+          __syncwarp();
+          fetch_w(next);
+        }
         const int buf = (int)(j & 1);
         const bool got = wait(acc_full + buf, (uint32_t)(j >> 1) & 1u);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }   // the warp leaves together
@@ -588,8 +656,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             tmem_ld_wait(va);
             tmem_ld_wait(vb);
             if (hh == BN / 64 - 2) release();
-            cm[hh] = chunk_max(va, r_half + hh * 32, weigh);
-            cm[hh + 1] = chunk_max(vb, r_half + hh * 32 + 32, weigh);
+            cm[hh] = chunk_max(va, r_half + hh * 32, hh * 32, weigh);
+            cm[hh + 1] = chunk_max(vb, r_half + hh * 32 + 32, hh * 32 + 32, weigh);
           }
           if (active) {
             float* out = P.maxima + ql * (2 * ntiles * P.gran) + ((int64_t)tile * 2 + half) * P.gran;
@@ -607,12 +675,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             tmem_ld_wait(va);
             tmem_ld_wait(vb);
             if (hh == BN / 64 - 2) release();
-            const uint32_t ma = hot_mask(va, r_half + hh * 32), mb = hot_mask(vb, r_half + hh * 32 + 32);
-            if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
-              if constexpr (MODE == 2) {
-                append(va, ma, r_half + hh * 32);
-                append(vb, mb, r_half + hh * 32 + 32);
-              } else {
+            if constexpr (APPEND) {
+              float x[32], y[32];
+              values(va, hh * 32, !cosine, x);
+              values(vb, hh * 32 + 32, !cosine, y);
+              const float mx = active ? maximum(x) : -INFINITY, my = active ? maximum(y) : -INFINITY;
+              if (__any_sync(0xffffffffu, fmaxf(mx, my) >= e_thr)) {
+                append(va, mx, hh * 32, r_half + hh * 32);
+                append(vb, my, hh * 32 + 32, r_half + hh * 32 + 32);
+              }
+            } else {
+              const uint32_t ma = hot_mask(va, hh * 32), mb = hot_mask(vb, hh * 32 + 32);
+              if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
                 take(va, ma, r_half + hh * 32);
                 take(vb, mb, r_half + hh * 32 + 32);
               }
@@ -625,7 +699,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
             uint32_t va[32];
             tmem_ld32(tb + hh * 32, va);
             if (hh == BN / 64 - 1) release();
-            const uint32_t ma = hot_mask(va, r_half + hh * 32);
+            const uint32_t ma = hot_mask(va, hh * 32);
             if (__any_sync(0xffffffffu, ma != 0u)) take(va, ma, r_half + hh * 32);
           }
         }
@@ -868,19 +942,19 @@ __global__ void k_tc_key_init(int64_t nq, unsigned* keys) {
 }
 
 // w[r]: +inf for degenerate references and the padding; 0 (cosine) or
-// (1 - c) Nr (euclidean) otherwise; wp (two passes, or null): the same with
-// one_plus_c for the first pass's x'
-__global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_c, float one_plus_c,
-                             const float* norm2, const uint8_t* empty, float* w, float* wp) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= nw) return;
-  float v = INFINITY, vp = INFINITY;
-  if (r < n && !empty[r]) {
-    v = (method == COSINE) ? 0.f : one_minus_c * norm2[r];
-    vp = (method == COSINE) ? 0.f : one_plus_c * norm2[r];
-  }
-  w[r] = v;
-  if (wp) wp[r] = vp;
+// (1 - c) Nr (euclidean) otherwise; wp: the same with one_plus_c for the x' of
+// a first pass over n1 sampled references, padded to nw1 (at most nw; 0 without
+// one)
+__global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_c,
+                             const float* norm2, const uint8_t* empty, float* w, int sample, int64_t n1, int64_t nw1,
+                             float one_plus_c, float* wp) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  auto weight = [&](int64_t r, float c) {
+    if (r >= n || empty[r]) return INFINITY;
+    return (method == COSINE) ? 0.f : c * norm2[r];
+  };
+  if (i < nw) w[i] = weight(i, one_minus_c);
+  if (i < nw1) wp[i] = i < n1 ? weight(sampled(i, sample), one_plus_c) : INFINITY;
 }
 
 // Two passes: each query's threshold, the k-th largest of its maxima less what
@@ -932,18 +1006,26 @@ __global__ void __launch_bounds__(256) k_tc_threshold(int method, int64_t q0, in
   }
 }
 
-// Whether two passes beat one for a block of nq queries: a pass costs 1.4 us a
-// tile up to d = 128 and 2.1 beyond (1.4 times that where the references exceed
-// the L2), the running lists about 50 + 8 k us of filling; with few queries in a
-// group hardly any lane fills a list.  One pass / two passes, us: 777 x 150,001, d =
-// 100, k = 15: 254 / 131; 3,000 x 60,000, d = 64, k = 30: 319 / 164; 500 x
-// 1,000,000, d = 128, k = 50: 622 / 280; 4,096 x 150,000, d = 256, k = 20: 490 /
-// 515; 1,024 x 800,000, d = 200, k = 20: 608 / 975; 1 x 400,000, d = 256: 60 / 80.
-bool two_passes(int64_t nq, int64_t n, int dpad, int k, int64_t tiles_per_cta, int64_t maxima) {
-  if (nq < 64 || maxima < 4 * (int64_t)k || maxima > INT32_MAX) return false;
-  double pass_us = (double)tiles_per_cta * (dpad <= 128 ? 1.4 : 2.1);
-  if (n * dpad * 2 > (int64_t)96 << 20) pass_us *= 1.4;
-  return pass_us < 50.0 + 8.0 * k;
+constexpr int64_t granularity(int64_t refs, int k) { return refs >= (int64_t)(BN / 2) * 8 * k ? 1 : 4; }
+int64_t maxima_per_query(int64_t refs, int k) { return 2 * ((refs + BN - 1) / BN) * granularity(refs, k); }
+
+// The stride of the sample whose maxima give each query's threshold; 0 (one pass
+// with running lists) where even all references give fewer than 4 k maxima.  A
+// stride of s leaves about s k references of a query above the threshold, and
+// the 768 slots of the query's shortest set of lists (two) have to hold them
+// with room to spare, hence s k <= 192; the first pass costs 1 / s of the second
+// and the candidates are re-bounded by the merge, so there is nothing to gain
+// beyond 8; below 16 k maxima the threshold drops (3,000 x 60,000, d = 64, k =
+// 30: 110 us with s = 6 and 4 k maxima against 108, the merge 13 us longer).
+// One pass / s = 8, us: 4,096 x 2,000,000, d = 256: 3,184 / 2,926; 4,096 x
+// 150,000: 487 / 300; 128 x 2,000,000: 233 / 194; 1 x 2,000,000: 170 / 184, but
+// merge and re-rank of fewer candidates make it 430 / 406 a call; 8 x 200,000,
+// euclidean: 127 / 37.  s = 1 / rule: 777 x 150,001, d = 100: 96 / 90.
+int sample_stride(int64_t n, int k) {
+  if (maxima_per_query(n, k) < 4 * (int64_t)k || maxima_per_query(n, k) > INT32_MAX) return 0;
+  int s = std::max(1, std::min(8, 192 / k));
+  while (s > 1 && maxima_per_query(n / s, k) < 16 * (int64_t)k) --s;
+  return s;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -983,30 +1065,46 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   // one map per operand: 64-row x 128-column (query) / 256-column (reference)
   // boxes of the K-major BF16 copy (rows padded to dpad with zeros; columns
   // beyond the matrix read as zero)
+  auto base_of = [&](const sdg_dense* M) { return (void*)((method == COSINE) ? M->ubp : M->xbp); };
   auto encode = [&](const sdg_dense* M, int box_cols, CUtensorMap* map) {
-    const __nv_bfloat16* base_ptr = (method == COSINE) ? M->ubp : M->xbp;
     const cuuint64_t gdim[2] = {(cuuint64_t)M->dpad, (cuuint64_t)M->n};
     const cuuint64_t gstride[1] = {(cuuint64_t)M->dpad * 2};
     const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_cols};
     const cuuint32_t estr[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base_ptr, gdim, gstride, box, estr,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base_of(M), gdim, gstride, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  // the references in n / sample whole runs of `sample` columns: a box takes the
+  // column at one place of each of box_cols runs
+  auto encode_sample = [&](int sample, int box_cols, CUtensorMap* map) {
+    const cuuint64_t gdim[3] = {(cuuint64_t)D->dpad, (cuuint64_t)sample, (cuuint64_t)(D->n / sample)};
+    const cuuint64_t gstride[2] = {(cuuint64_t)D->dpad * 2, (cuuint64_t)D->dpad * 2 * sample};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, 1, (cuuint32_t)box_cols};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base_of(D), gdim, gstride, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   // the list length: the smallest of 16 / 24 / 32 / 48 / 64 that holds k
-  auto pick_kernel = [&](bool pair) {
-    if (pair)
-      return (k <= 16) ? k_dense_tc<16, true, 0> : (k <= 24) ? k_dense_tc<24, true, 0>
-           : (k <= 32) ? k_dense_tc<32, true, 0> : (k <= 48) ? k_dense_tc<48, true, 0> : k_dense_tc<64, true, 0>;
+  auto pick_kernel = [&]() {
     return (k <= 16) ? k_dense_tc<16, false, 0> : (k <= 24) ? k_dense_tc<24, false, 0>
          : (k <= 32) ? k_dense_tc<32, false, 0> : (k <= 48) ? k_dense_tc<48, false, 0> : k_dense_tc<64, false, 0>;
   };
-  // CTA pairs (clusters of two) where the block has more than one 128-query
-  // group and the device can hold such clusters; the work unit is then a pair
+  // thresholds from a sample (MODE 1), then the references that pass (MODE 2,
+  // 3); or one pass with running lists (MODE 0)
+  const int sample = sample_stride(n, k);
+  const bool first = sample > 0;
+  // CTA pairs (clusters of two; the work unit is then a pair) where they pay or
+  // are asked for and the device can hold such clusters.  A pair's SM receives
+  // half the bytes of a reference chunk.  One CTA / pairs, us: 4,096 x 2,000,000,
+  // d = 256: 2,557 / 2,280; 1,024 x 800,000, d = 200: 286 / 274; 4,096 x
+  // 2,000,000, d = 128: 1,651 / 1,677; d = 64: 1,440 / 1,488; an odd number of
+  // 128-query groups pads one (257 x 1,000,000, d = 256: 161 / 182).
   int64_t units = 0;
   bool pair = false;
-  if (allow_pairs && nq > BM) {
-    auto kp = pick_kernel(true);
+  if (first && nq > BM && (allow_pairs || (D->dpad > 2 * BK && (nq + BM - 1) / BM % 2 == 0))) {
+    auto kp = method == COSINE ? k_dense_tc<1, true, 2> : k_dense_tc<1, true, 3>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1021,11 +1119,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     }
     cudaGetLastError();
   }
-  if (!pair) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, D->device);
-    units = std::max(sms, 1);
-  }
+  int sm_count = 0;
+  cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, D->device);
+  const int64_t sms = std::max(sm_count, 1);
+  if (!pair) units = sms;
   const int GM = pair ? Cfg<true>::GM : Cfg<false>::GM;
   CUtensorMap qmap, rmap;
   if (!encode(Q, BM, &qmap) || !encode(D, pair ? Cfg<true>::BNL : Cfg<false>::BNL, &rmap))
@@ -1047,10 +1144,9 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   const float rel = 0.0040f + (float)D->d * 2.384185791015625e-7f;
   const float omc = 1.f - (rel + 9.5367431640625e-7f);
 
-  // two passes (MODE 1 and 2) where a pass is short
-  const int gran = n >= (int64_t)(BN / 2) * 8 * k ? 1 : 4;
-  const int64_t m = 2 * ntiles * gran;
-  const bool two = !pair && two_passes(nq, n, D->dpad, k, per, m);
+  const int64_t n1 = first ? n / sample : 0, ntiles1 = (n1 + BN - 1) / BN;
+  const int gran = (int)granularity(n1, k);
+  const int64_t m = 2 * ntiles1 * gran;
   const float opc = 1.f + rel + 1.9073486328125e-6f;     // 2^-19
 
   float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
@@ -1058,10 +1154,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   unsigned* tshared = nullptr;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-  const int64_t nw = ntiles * BN;
+  const int64_t nw = ntiles * BN, nw1 = ntiles1 * BN;
   chk(cudaMallocAsync(&w, sizeof(float) * (size_t)nw, s));
-  if (two) {
-    chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw, s));
+  if (first) {
+    chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw1, s));
     chk(cudaMallocAsync(&maxima, sizeof(float) * (size_t)(nq * m), s));
   } else {
     chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
@@ -1072,10 +1168,11 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   chk(cudaMallocAsync(&cand_s, sizeof(float) * (size_t)(nq * cap), s));
   chk(cudaMallocAsync(&tshared, sizeof(unsigned) * (size_t)nq, s));
   if (e == cudaSuccess) {
-    // every query's shared key starts at fkey(-inf)
-    if (!two) k_tc_key_init<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(nq, tshared);
+    // every query's shared key starts at fkey(-inf) or at its threshold
+    if (!first) k_tc_key_init<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(nq, tshared);
     chk(cudaMemsetAsync(ecount, 0, sizeof(int32_t) * (size_t)(nq * nslots), s));
-    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, opc, D->norm2, D->empty, w, wp);
+    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, D->norm2, D->empty, w, sample, n1,
+                                                             nw1, opc, wp);
     TcArgs P;
     P.method = method; P.k = k; P.dch = dch; P.ecap = ecap;
     P.self = self ? 1 : 0;
@@ -1085,39 +1182,42 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     P.w = w; P.norm2 = D->norm2; P.qnorm2 = Q->norm2; P.qempty = Q->empty;
     P.tshared = tshared;
     P.lists = lists; P.ecount = ecount; P.eidx = eidx; P.es = es;
-    P.maxima = maxima; P.gran = gran; P.use_w = D->n_empty > 0 ? 1 : 0;
+    P.maxima = maxima; P.gran = gran; P.sample = sample; P.use_w = D->n_empty > 0 ? 1 : 0;
     P.status = status;
     P.stall = tc_take_stall() ? 1 : 0;
-    auto kern = two ? k_dense_tc<1, false, 2> : pick_kernel(pair);
-    chk(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+    auto launch = [&](auto kern, int64_t blocks, const CUtensorMap& refs, const TcArgs& A) {
+      chk(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = pair ? 2 : 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)(pair ? 2 * blocks : blocks), 1, 1); cfg.blockDim = dim3(THREADS, 1, 1);
+      cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = s;
+      cfg.attrs = attr; cfg.numAttrs = pair ? 1 : 0;
+      if (e == cudaSuccess) chk(cudaLaunchKernelEx(&cfg, kern, qmap, refs, A));
+    };
     sdg_time_begin(ctx);
-    if (two && e == cudaSuccess) {
-      chk(cudaFuncSetAttribute(k_dense_tc<1, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)SMEM_BYTES));
+    if (first) {
+      CUtensorMap map1;
+      if (!encode_sample(sample, pair ? Cfg<true>::BNL : Cfg<false>::BNL, &map1)) chk(cudaErrorInvalidValue);
+      const int64_t items1 = G * ntiles1;
       TcArgs P1 = P;
-      P1.w = wp;
-      if (e == cudaSuccess) k_dense_tc<1, false, 1><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(qmap, rmap, P1);
+      P1.w = wp; P1.n = n1; P1.ntiles = ntiles1;
+      P1.tiles_per_cta = (items1 + std::min(units, items1) - 1) / std::min(units, items1);
+      launch(pair ? k_dense_tc<1, true, 1> : k_dense_tc<1, false, 1>,
+             (items1 + P1.tiles_per_cta - 1) / P1.tiles_per_cta, map1, P1);
       P.stall = 0;                                     // one launch is stalled at a time
       if (e == cudaSuccess)
         k_tc_threshold<<<(unsigned)((nq + 7) / 8), 256, 0, s>>>(method, q0, nq, (int)m, k, rel, opc, Q->norm2,
                                                                 Q->empty, maxima, tshared);
     }
-    if (e == cudaSuccess) {
-      if (pair) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)(2 * grid), 1, 1); cfg.blockDim = dim3(THREADS, 1, 1);
-        cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = s;
-        cfg.attrs = attr; cfg.numAttrs = 1;
-        chk(cudaLaunchKernelEx(&cfg, kern, qmap, rmap, P));
-      } else {
-        kern<<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(qmap, rmap, P);
-      }
-    }
+    launch(!first            ? pick_kernel()
+           : method == COSINE ? (pair ? k_dense_tc<1, true, 2> : k_dense_tc<1, false, 2>)
+                              : (pair ? k_dense_tc<1, true, 3> : k_dense_tc<1, false, 3>),
+           grid, rmap, P);
     sdg_time_end(ctx);
     chk(cudaGetLastError());
+    ctx_stats_add(ctx, 3, first ? 5 : 4);              // weights, maxima and threshold (or key init), screen, merge
     MergeArgs M;
     M.q0 = q0; M.nq = nq; M.gm = GM; M.ntiles = ntiles; M.per = per; M.nslots = nslots;
     M.K = k; M.ecap = ecap; M.method = method; M.d = D->d;

@@ -515,7 +515,7 @@ __device__ __forceinline__ void key_and_bound(int method, float s, int32_t nq_, 
 // shared rows <= 31.1 u (A_P + A_Q), A = a column's sum of |x log x| + x.
 // The recursive FP32 sum of n <= min(nnz) terms adds <= n u / (1 - n u) times
 // sum |g~| <= log 2 (C_P + C_Q) + 31.1 u (A_P + A_Q) (0 <= g <= S log 2, C =
-// a column's sum).  With n u <= 1/16 (n is below the row table's 56 K rows)
+// a column's sum).  With n u <= 1/16 (n is at most kScreenMaxRows)
 // the two give E_G = u (33.5 (A_P + A_Q) + 0.75 n (C_P + C_Q)) 1.01; the key's
 // own rounding (u |key|, the FP64 S_P log 2 rounded once) is added.
 __device__ __forceinline__ void js_key_and_bound(float G, double SP, double SQ, float AP, float AQ,
@@ -1376,7 +1376,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
       stats[1] += h_count[(size_t)t];
     }
     stats[0] += nb * nr;
-    stats[3] += 5;
+    stats[3] += 6;
   }
   std::sort(overflow_queries.begin(), overflow_queries.end());
   overflow_queries.erase(std::unique(overflow_queries.begin(), overflow_queries.end()),

@@ -193,8 +193,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_sparse_tc(const __grid_constant_
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---- MMA issuer ----
-    if (lane == 0 && ntile > 0) {
+    // ---- MMA issuer: the whole warp walks the loop, one lane issues ----
+    if (ntile > 0) {
+      const bool one = elect_one();
+      auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, P.status));
+      };
+      const uint32_t lo = sw128_desc_lo(smem_u32(base));
       int it = 0;
       bool ok = true;
       for (int j = 0; j < ntile && ok; ++j) {
@@ -202,29 +207,31 @@ __global__ void __launch_bounds__(THREADS, 1) k_sparse_tc(const __grid_constant_
         // (with P.stall the first wait asks for the phase the epilogue has not
         // begun, so it runs out: the failure-detection test's path)
         const uint32_t flip = (P.stall && j == 0) ? 0u : 1u;
-        if (!mbar_wait(acc_empty, ((uint32_t)j & 1u) ^ flip, abort_flag, P.status)) break;
+        if (!wait_all(acc_empty, ((uint32_t)j & 1u) ^ flip)) break;
         fence_after();
         for (int c = 0; c < kch; ++c, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-          if (!mbar_wait(full + s, ph, abort_flag, P.status)) { ok = false; break; }
+          if (!wait_all(full + s, ph)) { ok = false; break; }
           fence_after();
-          const uint32_t a0 = smem_u32(base + (size_t)s * STAGE_BYTES);
-          const uint32_t a1 = a0 + A_BYTES, b = a0 + 2 * A_BYTES;
+          const uint32_t a0 = lo + (uint32_t)s * (uint32_t)(STAGE_BYTES >> 4);
+          const uint32_t a1 = a0 + (uint32_t)(A_BYTES >> 4), b = a1 + (uint32_t)(A_BYTES >> 4);
+          if (one) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t bd = sw128_desc(b + kk * 32);
-            const uint32_t acc = (c | kk) != 0;
-            umma_f16(tmem, sw128_desc(a0 + kk * 32), bd, IDESC, acc);
-            umma_f16(tmem + BN, sw128_desc(a1 + kk * 32), bd, IDESC, acc);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              const uint32_t acc = (c | kk) != 0;
+              umma_f16(tmem, a0 + kk * 2, b + kk * 2, IDESC, acc);
+              umma_f16(tmem + BN, a1 + kk * 2, b + kk * 2, IDESC, acc);
+            }
+            umma_commit(emptyb + s);          // the stage is free once these MMAs have read it
+            if (c == kch - 1) umma_commit(acc_full);   // tile j's accumulators are complete
           }
-          umma_commit(emptyb + s);            // the stage is free once these MMAs have read it
+          __syncwarp();
         }
-        if (!ok) break;
-        umma_commit(acc_full);                // tile j's accumulators are complete
       }
       // all issued MMAs complete before TMEM is freed
-      umma_commit(mma_done);
+      if (one) umma_commit(mma_done);
+      __syncwarp();
       mbar_drain(mma_done, 0);
     }
     __syncwarp();

@@ -92,6 +92,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// the same from a three-dimensional map
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
@@ -107,13 +114,19 @@ __device__ __forceinline__ void fence_after() {
 // swizzle (bits 61-63).  The tile base is 1024-byte aligned, so the base
 // offset (bits 49-51) is 0; a K step of 16 16-bit elements advances the start
 // by 32 B.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;                  // LBO = 16 B (ignored)
-  d |= (uint64_t)(1024 >> 4) << 32;        // SBO
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
+// As two words, so that a K step or another tile is one 32-bit addition to the
+// low one (the start address, below 2^14 units of 16 bytes).
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+constexpr uint32_t SW128_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+// One lane of the (converged) warp, the same at every call.  A loop that issues
+// MMAs runs in the whole warp and only the instructions themselves are
+// predicated: addresses and descriptors then stay in uniform registers.  Inside an
+// `if (lane == 0)` each tcgen05.mma cost its warp 70 cycles of operand moves, and
+// issuing, not the tensor pipe, set the pace.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 // Instruction descriptor of kind::f16 with FP32 accumulation (bits 4-5 = 1),
 // A and B of one 16-bit type (bits 7-9 and 10-12: 0 = FP16, 1 = BF16), both
@@ -122,13 +135,16 @@ constexpr uint32_t idesc_f16(int m, int n, bool bf16) {
   return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(m >> 4) << 24);
 }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accum) {
+// alo, blo: the descriptors' low words (sw128_desc_lo)
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                            uint32_t accum) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accum), "r"(SW128_DESC_HI)
       : "memory");
 }
 // Arrives on bar once every MMA this thread issued before has completed.
@@ -172,13 +188,23 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
       ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar_cluster)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accum) {
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster, int x,
+                                                 int y, int z) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, "
+      "%3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(bar_cluster)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                                 uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accum), "r"(SW128_DESC_HI)
       : "memory");
 }
 // Arrives on the barrier at bar's offset in every CTA of `mask` once every
