@@ -735,10 +735,10 @@ def run_dense_main(args):
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the bounding
 # kernel at the bench's full size, from a one-pass ncu capture
-# (profiles/k_dense_tc_cosine_2000000x256_q4096.md,
+# (profiles/k_dense_tc_cosine_400000x256_q4096.md,
 # profiles/launches_logcount_cosine_30000x200000_q4096.md)
-DENSE_TRAFFIC = 7.03e9 + 0.145e9
-LOGCOUNT_TRAFFIC = 65.22e9 + 0.181e9
+DENSE_TRAFFIC = (0.142e9 + 0.021e9) + (1.28e9 + 0.034e9)
+LOGCOUNT_TRAFFIC = 69.44e9 + 0.181e9
 
 
 def run_batched(args):
