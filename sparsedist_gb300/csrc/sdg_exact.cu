@@ -559,14 +559,15 @@ __device__ double pair_value_lookup(int method, bool dist, const DevCsc& R, cons
 
 // One query column per blockIdx.y, one reference column per thread.  With
 // `lookup` (a lookup method and nrow <= LOOKUP_MAX_ROWS) the block first holds
-// its query column as a row lookup in dynamic shared memory.
+// its query column as a row lookup in dynamic shared memory.  The query columns
+// are q0 + blockIdx.y, or queries[blockIdx.y].
 __global__ void k_exact_slab(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry, ColAux qa,
-                             int64_t q0, const uint8_t* ref_mask, int restore_self,
+                             int64_t q0, const int32_t* queries, const uint8_t* ref_mask, int restore_self,
                              double self_value, double* D, int lookup) {
   extern __shared__ uint32_t lk_bits[];
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t b = blockIdx.y;
-  const int64_t q = q0 + b;
+  const int64_t q = queries ? (int64_t)queries[b] : q0 + b;
   const int32_t words = (qry.nrow + 31) >> 5;
   int32_t* lk_base = reinterpret_cast<int32_t*>(lk_bits + words);
   if (lookup) {
@@ -1325,14 +1326,15 @@ void launch_check_js(const double* x, int64_t nnz, int* err, cudaStream_t s) {
 void launch_exact_slab(int method, int dist, const DevCsc& ref, const ColAux& ra,
                        const DevCsc& qry, const ColAux& qa, int64_t q0, int64_t nb,
                        const uint8_t* ref_mask, int restore_self, double self_value,
-                       double* D, cudaStream_t s) {
+                       double* D, cudaStream_t s, const int32_t* queries) {
   if (ref.ncol == 0 || nb == 0) return;
   for (int64_t b0 = 0; b0 < nb; b0 += 65535) {            // gridDim.y limit
     const int64_t cnt = (nb - b0 < 65535) ? nb - b0 : 65535;
     dim3 grid(blocks_for(ref.ncol, 128), (unsigned)cnt);
     const bool lookup = lookup_method(method) && qry.nrow <= LOOKUP_MAX_ROWS;
     const size_t smem = lookup ? (size_t)((qry.nrow + 31) / 32) * 8 : 0;
-    k_exact_slab<<<grid, 128, smem, s>>>(method, dist, ref, ra, qry, qa, q0 + b0, ref_mask,
+    k_exact_slab<<<grid, 128, smem, s>>>(method, dist, ref, ra, qry, qa, q0 + b0,
+                                         queries ? queries + b0 : nullptr, ref_mask,
                                          restore_self, self_value, D + b0 * (int64_t)ref.ncol, lookup ? 1 : 0);
   }
 }

@@ -53,7 +53,7 @@ bool tc_take_stall();
 void launch_exact_slab(int method, int dist, const DevCsc& ref, const ColAux& ra,
                        const DevCsc& qry, const ColAux& qa, int64_t q0, int64_t nb,
                        const uint8_t* ref_mask, int restore_self, double self_value,
-                       double* D, cudaStream_t s);
+                       double* D, cudaStream_t s, const int32_t* queries = nullptr);
 
 // Single-matrix sparseDist: columns c0 .. c0 + nb - 1 of the n x n result
 // into D (nb columns of length n); the upper triangle is computed only with
@@ -100,6 +100,9 @@ struct SelectArgs {
   const uint8_t* elem_mask = nullptr;
   int64_t skip_base = -1;
   const int64_t* skip_arr = nullptr;
+  // the query column of each segment, or null (segment seg is query skip_base + seg):
+  // its row is out_row0 + seg_query[seg] and skip_base >= 0 skips seg_query[seg]
+  const int32_t* seg_query = nullptr;
   const int32_t* seed_idx = nullptr;
   const double* seed_val = nullptr;
   int64_t seed_ld = 0;

@@ -1391,14 +1391,8 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   if (units) SK(cudaFreeAsync(units, s));
   if (rlo) SK(cudaFreeAsync(rlo, s));
   if (rhi) SK(cudaFreeAsync(rhi, s));
-  // queries the screen could not bound: the exact slab engine, run by runs
-  size_t a = 0;
-  while (a < overflow_queries.size()) {
-    size_t b = a + 1;
-    while (b < overflow_queries.size() && overflow_queries[b] == overflow_queries[b - 1] + 1) ++b;
-    hooks.exact_range(overflow_queries[a], (int64_t)(b - a));
-    a = b;
-  }
+  // queries the screen could not bound: the exact slab engine
+  if (!overflow_queries.empty()) hooks.exact_list(overflow_queries);
   return 0;
 }
 

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cuda_fp16.h>
 #include <functional>
+#include <vector>
 
 #include "sdg_common.cuh"
 
@@ -75,6 +76,7 @@ struct ScreenHooks {
   std::function<void()> check_cancel;
   std::function<void()> time_begin, time_end;        // bracket the screen kernel
   std::function<void(int64_t, int64_t)> exact_range;  // finish queries [q0, q0+n) exactly
+  std::function<void(const std::vector<int>&)> exact_list;   // finish these queries exactly
 };
 
 // The fused tcgen05 screen of the tensor engine (sdg_sparse_tc.cu): the FP16

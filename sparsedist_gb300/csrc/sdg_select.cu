@@ -22,7 +22,7 @@ using namespace topk;
 __device__ void select_row(const SelectArgs& a, int64_t seg, uint64_t* lk, double* lv, int32_t* li, int lane) {
   const int K = a.k;
   const bool dec = a.decreasing != 0;
-  const int64_t row = a.out_row0 + seg;
+  const int64_t row = a.out_row0 + (a.seg_query ? (int64_t)a.seg_query[seg] : seg);
   int n = 0;
 
   const bool blank = a.seg_blank && a.seg_blank[row];
@@ -42,7 +42,7 @@ __device__ void select_row(const SelectArgs& a, int64_t seg, uint64_t* lk, doubl
         if (bm) break;
       }
     }
-    const int64_t skip = (a.skip_base >= 0) ? a.skip_base + seg
+    const int64_t skip = (a.skip_base >= 0) ? (a.seg_query ? (int64_t)a.seg_query[seg] : a.skip_base + seg)
                          : (a.skip_arr ? a.skip_arr[seg] : (int64_t)-1);
     const double* base = a.vals + seg * a.seg_stride;
     const int64_t len = a.cand ? (int64_t)a.cand_count[seg] : a.len;
