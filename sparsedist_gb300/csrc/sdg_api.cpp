@@ -466,8 +466,9 @@ constexpr double kTensorMinDensity = 0.025;
 // 663 / 556; at 8e7 982 / 127, 1,365 / 610; binary, 2,000 x 2,000 at 3e8 306 /
 // 156, 747 / 710; log counts, 128 x 30,000 at 1.2e10 steps 222,000 / 2,400.
 // Where a query matches few columns, the screen keeps whole tied sets and
-// falls back to the exact slab query by query (2,000 x 2,000 at 0.5 % of 500
-// rows: 225 / 10,300): it is taken only with 16 k matched columns expected.
+// leaves such queries to the exact slab (2,000 x 2,000 at 0.5 % of 500 rows,
+// cosine, from the host: 403 / 467 with 180 queries left over, 516 / 391 at 1 %
+// with none): it is taken only with 16 k matched columns expected.
 bool exact_is_cheaper(int method, int k, int64_t nr, int64_t nq, int32_t nrow, double nnz_r, double nnz_q) {
   if (nr * nq > (int64_t)1 << 22) return false;
   const double pairs = (double)nr * (double)nq;
