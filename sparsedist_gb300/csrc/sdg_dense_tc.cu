@@ -133,6 +133,7 @@ struct TcArgs {
   float* maxima;              // MODE 1: [nq][2 * ntiles * gran]
   int gran;                   // MODE 1: maxima per tile half (1 or 4)
   int sample;                 // MODE 1: the sample's stride (sampled)
+  const int* gate;            // nothing to do unless *gate is set (null: always run)
   int use_w;                  // MODE 1, cosine: some reference is degenerate
   int32_t* ecount;            // [nq][nslots]
   int32_t* eidx;              // [nq][nslots][ecap]
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
   constexpr int STAGES = C::STAGES;
   constexpr uint32_t B_BYTES = C::B_BYTES;
   extern __shared__ uint8_t smem_raw[];
+  if (MODE == 0 && P.gate && !*P.gate) return;          // every thread of the grid alike
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = base;                                     // MAX_DCH query chunks
   uint8_t* sB = base + (size_t)MAX_DCH * A_BYTES;          // STAGES reference chunks
@@ -764,6 +766,8 @@ struct MergeArgs {
   int32_t* count;
   int32_t* over;
   size_t smem_query;           // shared-memory bytes of one query's prefix and keys
+  int* any_over;               // set when a query's list overflows (or null)
+  const int* gate;             // nothing to do unless *gate is set (null: always run)
 };
 
 // The per-pair bound of one candidate from the columns' BF16 copies: with v
@@ -825,6 +829,7 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
   __shared__ int s_count[QPB], s_kept[QPB];
   const int lane = threadIdx.x & 31;
   const int slot_q = WPQ == 1 ? (int)(threadIdx.x >> 5) : 0;
+  if (A.gate && !*A.gate) return;                        // every thread of the grid alike
   const int64_t ql = (int64_t)blockIdx.x * QPB + slot_q;
   if (ql >= A.nq) return;
   const kth::Group<WPQ> G{red};
@@ -860,7 +865,11 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
   bool ovf = G.sum(big ? 1u : 0u) != 0;
   G.sync();
   if (ovf) {
-    if (rank == 0) { A.count[ql] = 0; A.over[ql] = 1; }
+    if (rank == 0) {
+      A.count[ql] = 0;
+      A.over[ql] = 1;
+      if (A.any_over) *A.any_over = 1;
+    }
     return;
   }
   // T from the keys above the shared one
@@ -933,7 +942,11 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
     G.sync();
     total = s_kept[slot_q];
   }
-  if (rank == 0) { A.count[ql] = ovf ? 0 : total; A.over[ql] = ovf ? 1 : 0; }
+  if (rank == 0) {
+    A.count[ql] = ovf ? 0 : total;
+    A.over[ql] = ovf ? 1 : 0;
+    if (ovf && A.any_over) *A.any_over = 1;
+  }
 }
 
 __global__ void k_tc_key_init(int64_t nq, unsigned* keys) {
@@ -1013,7 +1026,8 @@ int64_t maxima_per_query(int64_t refs, int k) { return 2 * ((refs + BN - 1) / BN
 // with running lists) where even all references give fewer than 4 k maxima.  A
 // stride of s leaves about s k references of a query above the threshold, and
 // the 768 slots of the query's shortest set of lists (two) have to hold them
-// with room to spare, hence s k <= 192; the first pass costs 1 / s of the second
+// with room to spare, hence s k <= 192 (clusters that overflow them all the same
+// are repeated with running lists, see tc_screen); the first pass costs 1 / s of the second
 // and the candidates are re-bounded by the merge, so there is nothing to gain
 // beyond 8; below 16 k maxima the threshold drops (3,000 x 60,000, d = 64, k =
 // 30: 110 us with s = 6 and 4 k maxima against 108, the merge 13 us longer).
@@ -1087,7 +1101,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   // the list length: the smallest of 16 / 24 / 32 / 48 / 64 that holds k
-  auto pick_kernel = [&]() {
+  auto pick_kernel = [&](bool pair) {
+    if (pair)
+      return (k <= 16) ? k_dense_tc<16, true, 0> : (k <= 24) ? k_dense_tc<24, true, 0>
+           : (k <= 32) ? k_dense_tc<32, true, 0> : (k <= 48) ? k_dense_tc<48, true, 0> : k_dense_tc<64, true, 0>;
     return (k <= 16) ? k_dense_tc<16, false, 0> : (k <= 24) ? k_dense_tc<24, false, 0>
          : (k <= 32) ? k_dense_tc<32, false, 0> : (k <= 48) ? k_dense_tc<48, false, 0> : k_dense_tc<64, false, 0>;
   };
@@ -1152,6 +1169,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
   int32_t *ecount = nullptr, *eidx = nullptr;
   unsigned* tshared = nullptr;
+  int* any = nullptr;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   const int64_t nw = ntiles * BN, nw1 = ntiles1 * BN;
@@ -1159,9 +1177,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   if (first) {
     chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw1, s));
     chk(cudaMallocAsync(&maxima, sizeof(float) * (size_t)(nq * m), s));
-  } else {
-    chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
+    chk(cudaMallocAsync(&any, sizeof(int), s));
+    if (e == cudaSuccess) chk(cudaMemsetAsync(any, 0, sizeof(int), s));
   }
+  chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
   chk(cudaMallocAsync(&ecount, sizeof(int32_t) * (size_t)(nq * nslots), s));
   chk(cudaMallocAsync(&eidx, sizeof(int32_t) * (size_t)(nq * nslots * ecap), s));
   chk(cudaMallocAsync(&es, sizeof(float) * (size_t)(nq * nslots * ecap), s));
@@ -1182,7 +1201,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     P.w = w; P.norm2 = D->norm2; P.qnorm2 = Q->norm2; P.qempty = Q->empty;
     P.tshared = tshared;
     P.lists = lists; P.ecount = ecount; P.eidx = eidx; P.es = es;
-    P.maxima = maxima; P.gran = gran; P.sample = sample; P.use_w = D->n_empty > 0 ? 1 : 0;
+    P.gate = nullptr; P.maxima = maxima; P.gran = gran; P.sample = sample; P.use_w = D->n_empty > 0 ? 1 : 0;
     P.status = status;
     P.stall = tc_take_stall() ? 1 : 0;
     auto launch = [&](auto kern, int64_t blocks, const CUtensorMap& refs, const TcArgs& A) {
@@ -1211,17 +1230,17 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
         k_tc_threshold<<<(unsigned)((nq + 7) / 8), 256, 0, s>>>(method, q0, nq, (int)m, k, rel, opc, Q->norm2,
                                                                 Q->empty, maxima, tshared);
     }
-    launch(!first            ? pick_kernel()
+    launch(!first            ? pick_kernel(pair)
            : method == COSINE ? (pair ? k_dense_tc<1, true, 2> : k_dense_tc<1, false, 2>)
                               : (pair ? k_dense_tc<1, true, 3> : k_dense_tc<1, false, 3>),
            grid, rmap, P);
     sdg_time_end(ctx);
     chk(cudaGetLastError());
-    ctx_stats_add(ctx, 3, first ? 5 : 4);              // weights, maxima and threshold (or key init), screen, merge
+    ctx_stats_add(ctx, 3, first ? 7 : 4);   // weights, maxima and threshold (or key init), screen, merge, their repeat
     MergeArgs M;
     M.q0 = q0; M.nq = nq; M.gm = GM; M.ntiles = ntiles; M.per = per; M.nslots = nslots;
     M.K = k; M.ecap = ecap; M.method = method; M.d = D->d;
-    M.qempty = Q->empty; M.tshared = tshared; M.lists = lists; M.ecount = ecount; M.eidx = eidx; M.es = es;
+    M.qempty = Q->empty; M.tshared = tshared; M.lists = first ? nullptr : lists; M.ecount = ecount; M.eidx = eidx; M.es = es;
     M.norm2 = D->norm2; M.qnorm2 = Q->norm2;
     M.re = (method == COSINE) ? D->ue : D->xe; M.rn = (method == COSINE) ? D->un : D->xn;
     M.qe = (method == COSINE) ? Q->ue : Q->xe; M.qn = (method == COSINE) ? Q->un : Q->xn;
@@ -1233,12 +1252,26 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     auto mk = narrow ? k_tc_merge<1> : widest ? k_tc_merge<32> : k_tc_merge<8>;
     const size_t msm = M.smem_query * (narrow ? 8 : 1);
     if (msm > 48 * 1024) chk(cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm));
-    if (e == cudaSuccess)
-      mk<<<(unsigned)(narrow ? (nq + 7) / 8 : nq), widest ? 1024 : 256, msm, s>>>(M);
-    chk(cudaGetLastError());
+    auto merge = [&](const MergeArgs& A) {
+      if (e == cudaSuccess) mk<<<(unsigned)(narrow ? (nq + 7) / 8 : nq), widest ? 1024 : 256, msm, s>>>(A);
+      chk(cudaGetLastError());
+    };
+    M.any_over = any; M.gate = nullptr;
+    merge(M);
+    // A query in a dense cluster can have thousands of references between its
+    // threshold and its k-th best key (400,000 references in 50 clusters, k = 5: a
+    // list of 913 of 1,000 queries overflowed; exact rows for them took 7.8 s).
+    // Then the block runs once more with running lists, which tighten as they
+    // go, from the same thresholds; otherwise both launches return at once.
+    if (first) {
+      P.gate = any;
+      launch(pick_kernel(pair), grid, rmap, P);
+      M.lists = lists; M.any_over = nullptr; M.gate = any;
+      merge(M);
+    }
   }
   // stream-ordered frees: the caller reads *status with its own results
-  for (void* p : {(void*)w, (void*)wp, (void*)maxima, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared})
+  for (void* p : {(void*)w, (void*)wp, (void*)maxima, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared, (void*)any})
     if (p) cudaFreeAsync(p, s);
   if (e != cudaSuccess) {
     set_error(cudaGetErrorString(e));

@@ -65,3 +65,17 @@ def test_self_search(method, code, d, n, nq, k):
     ctx.lib.sdg_dense_free(h)
     wi, wd, _ = OracleBackend().knn(as_csc(X), k=k, method=method)
     assert same_bits(got[0], wi[1000:1000 + nq]) and same_bits(got[1], wd[1000:1000 + nq])
+
+
+@pytest.mark.parametrize("method,code", [("cosine", 1), ("euclidean", 2)])
+@pytest.mark.parametrize("d,nq,k", [(32, 70, 5), (200, 256, 3)])
+def test_clusters_that_overflow_the_lists(method, code, d, nq, k):
+    """Contiguous clusters of 4,000 within the bound of one another: the lists of
+    what passes the thresholds overflow and the block repeats with running lists."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    centres = torch.randn(5, d, generator=g, device="cuda")
+    label = torch.cat([torch.arange(5, device="cuda").repeat_interleave(4000), torch.arange(nq, device="cuda") % 5])
+    X = (centres[label] + 0.05 * torch.randn(20000 + nq, d, generator=g, device="cuda")).contiguous()
+    check(X, 20000, code, method, k)
