@@ -628,12 +628,16 @@ struct ScreenBounds {
       }
     }
     if (A.selfmode && q >= c && q < c + 4 && !(A.include_self && A.method == COVARIANCE)) {
-      // a restored self value (R/sparseKNN.R:270-279) is the best key; a
-      // covariance self pair keeps its computed value and is an ordinary pair
+      // A restored self value (R/sparseKNN.R:270-279) is the best value there is:
+      // no upper bound.  Its lower bound stays the pair's own: an exact copy of
+      // the query ties with it and comes first where its index is lower, so the
+      // copy's interval has to reach the k-th best lower bound (with the lower
+      // bound at +inf and k = 1 the query alone was kept).  A covariance self
+      // pair keeps its computed value and is an ordinary pair.
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (c + u == q) {
-          lo[u] = hi[u] = INFINITY;
+          hi[u] = INFINITY;
           if (!A.include_self) ok &= ~(1u << u);
         }
     }
@@ -904,43 +908,40 @@ __global__ void k_rescreen(RescreenArgs A) {
   for (int t = warp; t < n; t += nw) {
     const int32_t c = A.cand[ql * (int64_t)A.cap + t];
     float lo, hi;
-    if (A.selfmode && c == q) {
-      lo = hi = INFINITY;                       // the restored self pair
-    } else {
-      float acc = 0.f;
-      const int64_t c0 = A.ref.p[c], c1 = A.ref.p[c + 1];
-      for (int64_t a0 = c0; a0 < c1; a0 += 128) {
-        int32_t r[4];
+    float acc = 0.f;
+    const int64_t c0 = A.ref.p[c], c1 = A.ref.p[c + 1];
+    for (int64_t a0 = c0; a0 < c1; a0 += 128) {
+      int32_t r[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int64_t e = a0 + 32 * u + lane;
-          r[u] = (e < c1) ? __ldg(A.ref.i + e) : -1;
-        }
-        int qe[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          qe[u] = -1;
-          if (r[u] >= 0) {
-            const uint32_t wd = bits[r[u] >> 5];
-            const uint32_t bit = 1u << (r[u] & 31);
-            if (wd & bit) qe[u] = first[r[u] >> 5] + __popc(wd & (bit - 1u));
-          }
-        }
-        float f[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) f[u] = (qe[u] >= 0) ? __ldg(A.rf + a0 + 32 * u + lane) : 0.f;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (qe[u] >= 0) acc = fmaf(f[u], qv[qe[u]], acc);
+      for (int u = 0; u < 4; ++u) {
+        const int64_t e = a0 + 32 * u + lane;
+        r[u] = (e < c1) ? __ldg(A.ref.i + e) : -1;
       }
+      int qe[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      float key, err;
-      key_and_bound(A.method, acc, nq_, Nq, A.rnnz[c], A.rnorm ? A.rnorm[c] : 0.f, key, err);
-      lo = key - err;
-      hi = key + err;
-      if (!(fabsf(key) <= FLT_MAX) || !(err <= FLT_MAX)) { lo = -INFINITY; hi = INFINITY; }
+      for (int u = 0; u < 4; ++u) {
+        qe[u] = -1;
+        if (r[u] >= 0) {
+          const uint32_t wd = bits[r[u] >> 5];
+          const uint32_t bit = 1u << (r[u] & 31);
+          if (wd & bit) qe[u] = first[r[u] >> 5] + __popc(wd & (bit - 1u));
+        }
+      }
+      float f[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) f[u] = (qe[u] >= 0) ? __ldg(A.rf + a0 + 32 * u + lane) : 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (qe[u] >= 0) acc = fmaf(f[u], qv[qe[u]], acc);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    float key, err;
+    key_and_bound(A.method, acc, nq_, Nq, A.rnnz[c], A.rnorm ? A.rnorm[c] : 0.f, key, err);
+    lo = key - err;
+    hi = key + err;
+    if (!(fabsf(key) <= FLT_MAX) || !(err <= FLT_MAX)) { lo = -INFINITY; hi = INFINITY; }
+    if (A.selfmode && c == q) hi = INFINITY;  // the restored self pair (see ScreenBounds)
     if (lane == 0) {
       A.lo[ql * (int64_t)A.cap + t] = lo;
       A.hi[ql * (int64_t)A.cap + t] = hi;

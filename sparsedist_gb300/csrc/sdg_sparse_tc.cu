@@ -302,17 +302,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_sparse_tc(const __grid_constant_
           mask &= mask - 1;
           const int64_t r = r0 + jj;
           if (r >= P.nr || (P.ref_mask && P.ref_mask[r])) continue;
-          float lo, hi;
-          if (P.selfmode && r == q) {
-            if (!P.include_self) continue;
-            lo = hi = INFINITY;
-          } else {
-            float s = 0.f;
+          const bool own = P.selfmode && r == q;
+          if (own && !P.include_self) continue;
+          float lo, hi, s = 0.f;
 #pragma unroll
-            for (int t = 0; t < 32; ++t) s = (t == jj) ? __uint_as_float(v[t]) : s;
-            tcb::tc_bounds(P.method, s, nq_, Nq, P.rnnz[r], P.rnorm ? P.rnorm[r] : 0.f, eq, bq, P.rerr[r], P.rbn[r],
-                           lo, hi);
-          }
+          for (int t = 0; t < 32; ++t) s = (t == jj) ? __uint_as_float(v[t]) : s;
+          tcb::tc_bounds(P.method, s, nq_, Nq, P.rnnz[r], P.rnorm ? P.rnorm[r] : 0.f, eq, bq, P.rerr[r], P.rbn[r],
+                         lo, hi);
+          // the restored self value has no better one; its lower bound stays the
+          // pair's, so that exact copies of the query, which tie with it, are kept
+          if (own) hi = INFINITY;
           if (hi >= cut) {
             if (cnt < ECAP) { my_idx[cnt] = (int32_t)r; my_hi[cnt] = hi; }
             ++cnt;
