@@ -327,7 +327,12 @@ SDG_API int sdg_knn_block(sdg_ctx* ctx, const sdg_matrix* X, const sdg_matrix* Y
 
 /* As sdg_knn_resident, with idx / dist_out in DEVICE memory (caller
  * allocated, ncol(X) * k each); nothing is copied back and the call returns
- * once the work is queued on the context's stream (stream order). */
+ * once the work is queued on the context's stream (stream order; a search that
+ * takes a screen has waited for the stream, whose counts it reads).  While the
+ * context's stream is being captured into a CUDA graph, a search of at most 2^22
+ * pairs takes the exact slab and can be part of the graph, when the method has
+ * searched these matrices before (their per-column data is then prepared); as
+ * can sdg_knn_block with device_out. */
 SDG_API int sdg_knn_resident_device(sdg_ctx* ctx, const sdg_matrix* X, const sdg_matrix* Y,
                                     int method, int dist, int k, int include_self,
                                     int drop_degenerate, int32_t* idx, double* dist_out,

@@ -499,6 +499,12 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
   if (!screen_supported(P.method, P.k) || !screen_fits(nrow)) return 1;
   if (c->engine == 2) return 2;
   if (c->engine == 3) return (tensor_supported(P.method) && stc_supported(P.k)) ? 3 : 2;
+  if (nr * nq <= (int64_t)1 << 22) {
+    // into a graph that is being captured: the screens read counts back, the slab
+    // does not, so a small search of prepared matrices can be captured
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) return 1;
+  }
   const double nnz_q = (double)X->nnz * (double)nq / (double)std::max<int64_t>(X->ncol, 1);
   if (exact_is_cheaper(P.method, P.k, nr, nq, nrow, (double)ref->nnz, nnz_q)) return 1;
   // the tensor screen where the reference is dense enough and the dense copies
