@@ -655,7 +655,11 @@ struct ScreenBounds {
 // listed is a better T0 and the pass runs again.
 //
 // Bound by the slab's read (the second pass finds its row in the L2) and, for
-// short rows, by the two bit searches.  us: 10,000 queries x 10,000 references
+// short rows, by the two bit searches; pearson and covariance by the FP64 bounds,
+// so the cut at T reads the upper bounds that the second pass left in shared
+// memory (formed again by one warp, four columns a lane, it cost more than a
+// pass: 10,000 queries x 1,000 references, k = 100, pearson 7,207 us and 4,960
+// now, covariance 3,249 and 2,160).  us: 10,000 queries x 10,000 references
 // (binary) 655 with scalar loads, per-pair term counts and IEEE divisions, 296
 // now; 12,001 x 1,500 163 and 126; 1,500 x 12,001 121 and 52.  A warp per query
 // with k-long sorted insertions, reading the norms through a column permutation,
@@ -663,7 +667,8 @@ struct ScreenBounds {
 template <int KIND, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A) {
   constexpr int NT = WARPS * 32;
-  extern __shared__ uint32_t keys[];                 // max(slices * NT, cap)
+  extern __shared__ uint32_t keys[];                 // max(slices * NT, 2 cap)
+  float* his = reinterpret_cast<float*>(keys + A.cap);   // second pass: the candidates' upper bounds
   __shared__ float s_t;
   __shared__ int s_n;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -719,6 +724,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
           if (at < A.cap) {
             out[at] = (int32_t)(4 * g + u);
             keys[at] = kth::fkey(lo[u]);
+            his[at] = hi[u];
           }
         }
       }
@@ -745,15 +751,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
       kept = 0;
       for (int t0 = 0; t0 < n; t0 += 32) {
         const int t = t0 + lane;
-        int32_t c = 0;
-        bool keep = false;
-        if (t < n) {
-          c = out[t];
-          float lo[4], hi[4];
-          bounds(c & ~3, A.nr, S4[c >> 2], lo, hi);
-          const float h = (c & 2) ? ((c & 1) ? hi[3] : hi[2]) : ((c & 1) ? hi[1] : hi[0]);
-          keep = h >= cut;
-        }
+        const int32_t c = t < n ? out[t] : 0;
+        const bool keep = t < n && his[t] >= cut;
         const unsigned m = __ballot_sync(0xffffffffu, keep);   // every lane has read slot t first
         if (keep) out[kept + __popc(m & ((1u << lane) - 1u))] = c;
         kept += __popc(m);
@@ -1343,7 +1342,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     const bool wide = nb < 2 * nsm;
     const int nt = wide ? 1024 : 256;
     B.slices = std::max(1, (4 * r.k + nt - 1) / nt);
-    const size_t ssmem = sizeof(uint32_t) * (size_t)std::max(B.slices * nt, cap);
+    const size_t ssmem = sizeof(uint32_t) * (size_t)std::max(B.slices * nt, 2 * cap);   // <= 64 KB (cap <= 8,192)
     auto pick = [&](auto k8, auto k32) { return wide ? k32 : k8; };
     auto select = r.method == COSINE ? pick(k_screen_select<0, 8>, k_screen_select<0, 32>)
                   : r.method == BINARY ? pick(k_screen_select<2, 8>, k_screen_select<2, 32>)
@@ -1351,6 +1350,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
                   : (r.method == PEARSON || r.method == COVARIANCE)
                       ? pick(k_screen_select<4, 8>, k_screen_select<4, 32>)
                       : pick(k_screen_select<1, 8>, k_screen_select<1, 32>);
+    if (ssmem > 40 * 1024) SK(cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
     select<<<(unsigned)nb, nt, ssmem, s>>>(B);
     SK(cudaGetLastError());
     }
