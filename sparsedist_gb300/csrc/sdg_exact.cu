@@ -1009,6 +1009,36 @@ __global__ void __launch_bounds__(RR_MAX_WARPS * 32) k_rerank(int method, int di
   }
 }
 
+// The same by a thread per candidate, walking both columns (pair_value): for
+// short columns of the methods without a product form (and covariance), where
+// k_rerank's passes over 32 candidates are mostly barriers.  The rule is on the
+// stored entries of a mean reference and a mean query column together.  k_rerank
+// / walk, us, 10,000 queries x 1,000 references, k = 100, a million candidates, at
+// 20, 40, 80 and 160 entries: manhattan 374 / 135, 472 / 250, 762 / 508, 1,362 /
+// 1,109, at 320 2,636 / 2,450; euclidean 396 / 293, 515 / 531, 834 / 1,004, 1,458 /
+// 2,125; covariance 420 / 167, 432 / 280, 459 / 481, 496 / 872; js 5,856 / 1,591 (ten
+// million), 2,719 / 1,915, 2,531 / 3,660, 2,579 / 8,470.  The products and counts
+// gain as much but stay on k_rerank: a thread would walk a long column among
+// short ones alone.
+double walk_max_nnz(int method) {
+  if (method == MANHATTAN) return 128.0;
+  return (method == EUCLIDEAN || method == JS || method == COVARIANCE) ? 48.0 : 0.0;
+}
+
+__global__ void __launch_bounds__(128) k_rerank_walk(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry, ColAux qa,
+                                                     const int32_t* cand, const int32_t* count, int cap,
+                                                     int64_t q_begin, int restore_self, double self_value,
+                                                     double* out) {
+  const int64_t ql = blockIdx.x;
+  const int32_t q = (int32_t)(q_begin + ql);
+  const int n = count[ql];
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const int32_t c = cand[ql * (int64_t)cap + t];
+    out[ql * (int64_t)cap + t] =
+        (restore_self && c == q) ? self_value : pair_value(method, dist != 0, ref, ra, c, qry, qa, q);
+  }
+}
+
 // The single-matrix sparseDist of the match-only methods: CTA (x, y) takes
 // column q = x of m as the query and the reference columns c = y * 2048 .. of m
 // below it (c < q) as its candidates, in the reference's orientation (first
@@ -1385,8 +1415,14 @@ void launch_mirror_lower(double* D, int64_t n, cudaStream_t s) {
 
 int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, const DevCsc& qry, const ColAux& qa,
                   const int32_t* cand, const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
-                  int restore_self, double self_value, double* out, double mean_nnz, cudaStream_t s) {
+                  int restore_self, double self_value, double* out, double mean_nnz, double mean_qnnz,
+                  cudaStream_t s) {
   if (nq_local <= 0) return 0;
+  if (mean_nnz + mean_qnnz <= walk_max_nnz(method)) {
+    k_rerank_walk<<<(unsigned)nq_local, 128, 0, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin,
+                                                     restore_self, self_value, out);
+    return (int)cudaGetLastError();
+  }
   const int kind = method == BINARY ? 0 : method == JS ? 2 : method == MANHATTAN ? 3 : method == EUCLIDEAN ? 4 : 1;
   // eight warps (products, 4,096 queries of 30,000 log-count columns: 1.55 ms
   // where five take 1.92 and sixteen 1.76); counts of short columns have less
