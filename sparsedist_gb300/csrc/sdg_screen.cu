@@ -540,8 +540,16 @@ __device__ __forceinline__ void js_key_and_bound(float G, double SP, double SQ, 
 // and both bounds are clamped to [-1, 1] as the exact value is.  A pearson
 // denominator below 1e-200 could let cov / den overflow (exact value 0 then):
 // the bounds are [-1, 1].  Larger key = better for both methods.
+// a column's standard deviation, sqrt(v), with the exact path's rounded operations
+__device__ __forceinline__ double moment_root(int32_t nrow, double S, double SS) {
+  const double N = (double)nrow;
+  const double norm = (nrow > 1) ? __dsub_rn(N, 1.0) : 1.0;
+  return sqrt(__dsub_rn(SS, __dmul_rn(S, S) / N) / norm);
+}
+// root_q: the query's moment_root (pearson)
 __device__ __forceinline__ void moment_key_and_bound(bool pearson, float s, int32_t n_, int32_t nrow, double SP,
-                                                     double SSP, double SQ, double SSQ, float& key, float& err) {
+                                                     double SSP, double SQ, double SSQ, double root_q, float& key,
+                                                     float& err) {
   const double N = (double)nrow;
   const double norm = (nrow > 1) ? __dsub_rn(N, 1.0) : 1.0;
   const double sd = (double)s;
@@ -554,9 +562,7 @@ __device__ __forceinline__ void moment_key_and_bound(bool pearson, float s, int3
     lo = cov - Ecov * 1.0001;
     hi = cov + Ecov * 1.0001;
   } else {
-    const double vp = __dsub_rn(SSP, __dmul_rn(SP, SP) / N) / norm;
-    const double vq = __dsub_rn(SSQ, __dmul_rn(SQ, SQ) / N) / norm;
-    const double den = __dmul_rn(sqrt(vp), sqrt(vq));
+    const double den = __dmul_rn(moment_root(nrow, SP, SSP), root_q);
     if (!(den > 0.0) || !isfinite(den)) { key = 0.f; err = 0.f; return; }   // the exact value is 0
     if (den < 1e-200) { key = 0.f; err = 1.0001f; return; }
     const double c = cov / den;
@@ -581,9 +587,12 @@ struct ScreenBounds {
   const int64_t q;
   const int32_t nq_;
   const float Nq, e, a;
+  const double SQ, SSQ, root_q;              // KIND 4: the query's moments
   __device__ __forceinline__ ScreenBounds(const SelectScreenArgs& A_, int64_t q_)
       : A(A_), q(q_), nq_(A_.qnnz[q_]), Nq(A_.qnorm ? A_.qnorm[q_] : 0.f),
-        e(((float)nq_ + (KIND == 0 ? 40.f : 46.f)) * U32 * 1.01f + 1e-12f), a(A_.method == EUCLIDEAN ? 2.f : 1.f) {}
+        e(((float)nq_ + (KIND == 0 ? 40.f : 46.f)) * U32 * 1.01f + 1e-12f), a(A_.method == EUCLIDEAN ? 2.f : 1.f),
+        SQ(KIND == 4 ? A_.qs[q_] : 0.0), SSQ(KIND == 4 ? A_.qss[q_] : 0.0),
+        root_q(KIND == 4 && A_.method == PEARSON ? moment_root(A_.nrow, SQ, SSQ) : 0.0) {}
   __device__ __forceinline__ unsigned operator()(int64_t c, int64_t end, const float4& sv, float (&lo)[4],
                                                  float (&hi)[4]) const {
     const float s[4] = {sv.x, sv.y, sv.z, sv.w};
@@ -620,7 +629,7 @@ struct ScreenBounds {
             js_key_and_bound(s[u], A.rsum[c + u], A.qsum[q], Nc[u], Nq, min(nq_, nn[u]), key, err);
           else
             moment_key_and_bound(A.method == PEARSON, s[u], min(nq_, nn[u]), A.nrow, A.rs[c + u], A.rss[c + u],
-                                 A.qs[q], A.qss[q], key, err);
+                                 SQ, SSQ, root_q, key, err);
         }
         lo[u] = key - err;
         hi[u] = key + err;
