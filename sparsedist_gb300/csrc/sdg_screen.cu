@@ -474,6 +474,7 @@ struct SelectScreenArgs {
   int cap;
   int slices;                                // stretches of a row in the first pass
   int32_t* cand;                             // [qlocal * cap + t] reference column
+  float* hi;                                 // the same places: the candidates' upper bounds
   int32_t* count;                            // kept pairs per query (capped)
   int32_t* overflow;                         // 1 = finish with the exact engine
 };
@@ -665,8 +666,8 @@ struct ScreenBounds {
 //
 // Bound by the slab's read (the second pass finds its row in the L2) and, for
 // short rows, by the two bit searches; pearson and covariance by the FP64 bounds,
-// so the cut at T reads the upper bounds that the second pass left in shared
-// memory (formed again by one warp, four columns a lane, it cost more than a
+// so the cut at T reads the upper bounds that the second pass stored
+// (formed again by one warp, four columns a lane, it cost more than a
 // pass: 10,000 queries x 1,000 references, k = 100, pearson 7,207 us and 4,960
 // now, covariance 3,249 and 2,160).  us: 10,000 queries x 10,000 references
 // (binary) 655 with scalar loads, per-pair term counts and IEEE divisions, 296
@@ -676,8 +677,7 @@ struct ScreenBounds {
 template <int KIND, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A) {
   constexpr int NT = WARPS * 32;
-  extern __shared__ uint32_t keys[];                 // max(slices * NT, 2 cap)
-  float* his = reinterpret_cast<float*>(keys + A.cap);   // second pass: the candidates' upper bounds
+  extern __shared__ uint32_t keys[];                 // max(slices * NT, cap)
   __shared__ float s_t;
   __shared__ int s_n;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -694,11 +694,16 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
   const float4* S4 = reinterpret_cast<const float4*>(Srow);
   const kth::Group<1> G{nullptr};
   const int64_t n4 = (A.nr + 3) / 4, stretch = (n4 + A.slices - 1) / A.slices;
+  // The thread's place in a stretch: the warps take turns at the first places, so
+  // that the stretches' short last rounds (always warp 0 otherwise, the same
+  // quarter of every SM) spread over the FP64 pipes: covariance, 6,063 queries x
+  // 5,669 references, k = 300, 8,156 us without
+  auto turn = [&](int sl) { return (tid + 32 * (int)((blockIdx.x + sl) % WARPS)) % NT; };
   for (int sl = 0; sl < A.slices; ++sl) {
     const int64_t g1 = min((sl + 1) * stretch, n4);
     float best = -INFINITY;
 #pragma unroll 2
-    for (int64_t g = sl * stretch + tid; g < g1; g += NT) {
+    for (int64_t g = sl * stretch + turn(sl); g < g1; g += NT) {
       float lo[4], hi[4];
       const unsigned ok = bounds(4 * g, A.nr, S4[g], lo, hi);
 #pragma unroll
@@ -717,13 +722,14 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
     return T - ((T == -INFINITY || T == INFINITY) ? 0.f : fabsf(T) * (8.f * U32) + 1e-30f);
   };
   int32_t* out = A.cand + ql * (int64_t)A.cap;
+  float* his = A.hi + ql * (int64_t)A.cap;
   int n = 0;
   for (int round = 0; round < 4; ++round) {
     const float cut = cut_of(s_t);
     if (tid == 0) s_n = 0;
     __syncthreads();
 #pragma unroll 2
-    for (int64_t g = tid; g < n4; g += NT) {
+    for (int64_t g = turn(0); g < n4; g += NT) {
       float lo[4], hi[4];
       const unsigned ok = bounds(4 * g, A.nr, S4[g], lo, hi);
 #pragma unroll
@@ -1351,7 +1357,8 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     const bool wide = nb < 2 * nsm;
     const int nt = wide ? 1024 : 256;
     B.slices = std::max(1, (4 * r.k + nt - 1) / nt);
-    const size_t ssmem = sizeof(uint32_t) * (size_t)std::max(B.slices * nt, 2 * cap);   // <= 64 KB (cap <= 8,192)
+    const size_t ssmem = sizeof(uint32_t) * (size_t)std::max(B.slices * nt, cap);
+    B.hi = reinterpret_cast<float*>(rvals);          // free until the exact values are written
     auto pick = [&](auto k8, auto k32) { return wide ? k32 : k8; };
     auto select = r.method == COSINE ? pick(k_screen_select<0, 8>, k_screen_select<0, 32>)
                   : r.method == BINARY ? pick(k_screen_select<2, 8>, k_screen_select<2, 32>)
@@ -1359,7 +1366,6 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
                   : (r.method == PEARSON || r.method == COVARIANCE)
                       ? pick(k_screen_select<4, 8>, k_screen_select<4, 32>)
                       : pick(k_screen_select<1, 8>, k_screen_select<1, 32>);
-    if (ssmem > 40 * 1024) SK(cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
     select<<<(unsigned)nb, nt, ssmem, s>>>(B);
     SK(cudaGetLastError());
     }
