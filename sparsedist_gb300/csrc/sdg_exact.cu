@@ -716,7 +716,8 @@ __device__ double match_finish(int method, bool dist, double sum, int64_t common
 // reference adds them) runs one pair per LANE of one warp, and the terms of the
 // sums are formed 32 at a time.
 //
-// A CTA takes one query of the candidate table, 32 candidates at a time.  Warps
+// A CTA takes one query of the candidate table, 32 candidates at a time (the
+// gridDim.y CTAs of a query in turn).  Warps
 // 1 .. produce: for each candidate in turn a warp streams the column,
 // coalesced, and writes the next (at most RM) terms of its sum, in row order,
 // to the candidate's list in shared memory.  Warp 0 adds: lane j runs candidate
@@ -767,7 +768,7 @@ __global__ void __launch_bounds__(RR_MAX_WARPS * 32) k_rerank(int method, int di
   const int64_t ql = blockIdx.x;
   const int32_t q = (int32_t)(q_begin + ql);
   const int n = count[ql];
-  if (n == 0) return;
+  if (32 * (int)blockIdx.y >= n) return;
   const int64_t qb = qry.p[q];
   const int32_t nq = (int32_t)(qry.p[q + 1] - qb);
   for (int w = threadIdx.x; w < W; w += blockDim.x) bits[w] = 0u;
@@ -796,7 +797,7 @@ __global__ void __launch_bounds__(RR_MAX_WARPS * 32) k_rerank(int method, int di
   const double* rv = (method == COSINE) ? ra.uval : ref.x;
   const unsigned below = (1u << lane) - 1u;
   const bool q_empty = (method == COSINE) && qa.scale[q] == 0.0;
-  for (int g = 0; g < n; g += 32) {
+  for (int g = 32 * blockIdx.y; g < n; g += 32 * gridDim.y) {
     const int ng = min(32, n - g);
     // warp 0, lane j: candidate g + j and its sums
     int32_t c = -1;
@@ -1437,7 +1438,14 @@ int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, con
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  k<<<(unsigned)nq_local, nw * 32, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin, restore_self,
+  // a query's candidates over several CTAs where the queries are few (2 queries,
+  // 24,774 references of 5,500 entries, k = 300, manhattan: 27 ms with one each,
+  // where the exact slab takes 10.6)
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t parts = std::min<int64_t>((cap + 31) / 32, (4 * (int64_t)sms + nq_local - 1) / nq_local);
+  k<<<dim3((unsigned)nq_local, (unsigned)parts), nw * 32, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin, restore_self,
                                               self_value, out);
   return (int)cudaGetLastError();
 }
