@@ -1184,12 +1184,14 @@ static int ensure_rows(ScreenCache* c, const DevCsc& M, cudaStream_t s) {
   return 0;
 }
 
-// The columns of a part (a multiple of the sub-range) and the warps of a CTA:
-// a run (one row's entries of a part) should give the lanes about 32 entries,
-// the accumulators of a CTA's warps share kScreenAccBytes, and there should be
-// an item for every warp of the chip.  At 5 % density 1,024 columns take 6.2 ms
-// where 512 take 7.5 and 1,536 take 6.6 (24 or 28 warps were slower than 32).
-static void screen_shape(const ScreenCache* rc, int64_t nr, int32_t nrow, int64_t nq, int nsm, int* part_subs,
+// The columns of a part (a multiple of the sub-range) and the warps of a CTA for
+// `units` stretches of queries: a run (one row's entries of a part) should give
+// the lanes about 32 entries, the accumulators of a CTA's warps share
+// kScreenAccBytes, and there should be an item for every warp of the chip.  At 5 %
+// density 1,024 columns take 6.2 ms where 512 take 7.5 and 1,536 take 6.6 (24 or 28
+// warps were slower than 32).  With fewer items than warps the CTAs get fewer
+// warps, so that the items spread over the SMs.
+static void screen_shape(const ScreenCache* rc, int64_t nr, int32_t nrow, int64_t units, int nsm, int* part_subs,
                          int* warps) {
   const int64_t sub = (int64_t)1 << rc->sub_lg;
   const double density = (double)rc->nnz_total / ((double)nrow * (double)nr);
@@ -1199,9 +1201,10 @@ static void screen_shape(const ScreenCache* rc, int64_t nr, int32_t nrow, int64_
   int64_t cols = (int64_t)std::min(13312.0, std::max(1024.0, 32.0 / std::max(density, 1e-9)));
   cols = std::min(cols, std::max<int64_t>(nr, 1));
   int64_t m = std::max<int64_t>(1, cols / sub);
-  while (m > 1 && nq * ((nr + m * sub - 1) / (m * sub)) < (int64_t)nsm * warps_of(m * sub)) m /= 2;
+  auto items = [&] { return units * ((nr + m * sub - 1) / (m * sub)); };
+  while (m > 1 && items() < (int64_t)nsm * warps_of(m * sub)) m /= 2;
   *part_subs = (int)m;
-  *warps = warps_of(m * sub);
+  *warps = (int)std::min<int64_t>(warps_of(m * sub), std::max<int64_t>(1, (items() + nsm - 1) / nsm));
 }
 
 int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColAux& ra,
@@ -1320,7 +1323,9 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     } else {
     ScreenArgs A;
     int warps = 1;
-    screen_shape(rc, nr, nrow, nb, nsm, &A.part_subs, &warps);
+    // stretches of the chunk's queries, by the query matrix's mean
+    const int64_t chunk_units = nb + (int64_t)((double)qc->nnz_total * (double)nb / (double)nq / SCREEN_SEG);
+    screen_shape(rc, nr, nrow, chunk_units, nsm, &A.part_subs, &warps);
     A.rows = rc->rows; A.ent = static_cast<const int2*>(rc->ent); A.exl = rc->exl;
     A.nsub = rc->nsub; A.lg = rc->sub_lg; A.nr = nr; A.ldS = ldS;
     A.qp = qry.p; A.qi = qry.i; A.qv = qc->fval; A.qxl = qc->fxl; A.q_begin = q0; A.nq = nb;
@@ -1337,7 +1342,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
     auto kernel = r.method == MANHATTAN ? k_screen_rows<1> : r.method == JS ? k_screen_rows<2> : k_screen_rows<0>;
     // a function attribute is per device: set on every call (cheap, thread-safe)
     SK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScreenAccBytes));
-    const int64_t grid = std::min<int64_t>(nsm, (nb * A.nparts + warps - 1) / warps);
+    const int64_t grid = std::min<int64_t>(nsm, (chunk_units * A.nparts + warps - 1) / warps);
     hooks.time_begin();
     kernel<<<(unsigned)grid, warps * 32, smem, s>>>(A);
     hooks.time_end();
