@@ -456,37 +456,75 @@ void exact_engine(sdg_ctx* c, const KnnPlan& P, sdg_matrix* ref, sdg_matrix* qry
 // 784 / 483, 4,096 x 30,000 log counts at 5 % 39,209 / 6,510.
 constexpr double kTensorMinDensity = 0.025;
 
-// Whether the exact FP64 slab beats the screens, for searches of at most 2^22
-// pairs (above, the screens always win).  Exact: merge steps (nr nnz_q + nq
-// nnz_r) at the method's measured rate, plus the selection over every pair;
-// screened: about 250 us of launches and per-column preparation plus the
-// screen's work per pair (pearson and covariance bound every pair in FP64).
-// Measured, exact / FP32 screen, us, euclidean: 301 x 301 at 9e6 steps 190 /
-// 117 resident, 519 / 557 from the host; 1,000 x 1,000 at 2e7 steps 347 / 106,
-// 663 / 556; at 8e7 982 / 127, 1,365 / 610; binary, 2,000 x 2,000 at 3e8 306 /
-// 156, 747 / 710; log counts, 128 x 30,000 at 1.2e10 steps 222,000 / 2,400.
-// Where a query matches few columns, the screen keeps whole tied sets and
-// leaves such queries to the exact slab (2,000 x 2,000 at 0.5 % of 500 rows,
-// cosine, from the host: 403 / 467 with 180 queries left over, 516 / 391 at 1 %
-// with none): it is taken only with 16 k matched columns expected.
-bool exact_is_cheaper(int method, int k, int64_t nr, int64_t nq, int32_t nrow, double nnz_r, double nnz_q) {
-  if (nr * nq > (int64_t)1 << 22) return false;
-  const double pairs = (double)nr * (double)nq;
-  const double shared = nrow > 0 ? nnz_q * nnz_r / (pairs * (double)nrow) : 0.0;   // expected rows per pair
-  if ((double)nr * std::min(shared, 1.0) < 16.0 * k) return true;
-  const double steps = (double)nr * nnz_q + (double)nq * nnz_r;
-  double rate = 0.0;                                  // merge steps per microsecond
-  switch (method) {
-    case BINARY: rate = 8.0e5; break;
-    case COSINE: rate = 3.3e5; break;
-    case EUCLIDEAN: rate = 8.8e4; break;
-    case MANHATTAN: rate = 1.7e5; break;
-    case JS: rate = 5.5e4; break;
-    default: rate = 1.9e5;                            // pearson, covariance
-  }
-  const double exact_us = steps / rate + pairs / 2.0e4;
-  const double screen_us = 250.0 + pairs / ((method == PEARSON || method == COVARIANCE) ? 2.0e3 : 4.0e4);
-  return exact_us <= screen_us;
+// Searches of at most 2^22 pairs take the exact FP64 slab or a screen by predicted
+// time; above, the screens always win.  The coefficients (us) are least-squares
+// fits of every engine's time, forced in turn, over 826 shapes of 1 .. 3,000 queries,
+// 300 .. 60,000 references, 500 .. 30,000 rows, 0.4 .. 30 % density, k = 10, and
+// 200 x 7 drawn ones with k = 1 .. 300.
+constexpr int64_t kSmallPairs = (int64_t)1 << 22;
+// The most device memory that a small search adds to its matrices for good: what
+// a screen's slab may take for the length of a call.
+constexpr size_t kSmallCopyBytes = (size_t)4 << 30;
+
+struct SearchSize {
+  int method, k;
+  int64_t nr, nq;
+  int32_t nrow;
+  double nnz_r, nnz_q;                       // of the references, of the searched query columns
+  double matched() const { return nnz_q * nnz_r / std::max<double>(nrow, 1.0); }   // expected, over all pairs
+};
+struct ExactCost { double base, len, rate, pair; };
+// us: fixed; per entry of a reference column (a thread walks it); merge steps a us; per pair
+constexpr ExactCost kExactCost[kMethodCount] = {
+    {17, 0.058, 1.37e6, 1.75e-5}, {15, 0.20, 4.2e5, 3.1e-5}, {15, 1.06, 9.15e4, 5.3e-5}, {11, 0.95, 1.71e5, 1.4e-5},
+    {18, 0.196, 4.2e5, 1.78e-4},  {0, 1.36, 1.2e5, 0.0},     {16, 0.195, 4.24e5, 6.2e-5}};
+double exact_us(const SearchSize& z) {
+  const ExactCost& c = kExactCost[z.method];
+  const double nr = (double)z.nr, nq = (double)z.nq, k = z.k;
+  // the selection: a warp a query, over every pair (nr) and into a list of k
+  return c.base + c.len * z.nnz_r / nr + (nr * z.nnz_q + nq * z.nnz_r) / c.rate + c.pair * nr * nq + 0.015 * nr +
+         0.88 * k * std::log(1.0 + nr / k);
+}
+struct ScreenCost { double base, match, pair, ref, len, cand, item; };
+// us: fixed; per matched row; bounds per pair and per reference (pearson and
+// covariance in FP64); per entry of a mean query and reference (re-rank latency);
+// per entry of all k nq candidate pairs; per batch of 32 entries of an item's runs
+constexpr ScreenCost kScreenCost[kMethodCount] = {
+    {99, 9.6e-7, 5.0e-6, 2.8e-4, 0.052, 2.5e-6, 0.10},  {95, 9.4e-7, 4.1e-6, 1.3e-4, 0.060, 4.3e-6, 0.104},
+    {95, 8.6e-7, 4.6e-6, 2.1e-4, 0.090, 1.13e-5, 0.105}, {98, 9.4e-7, 4.0e-6, 1.8e-4, 0.090, 1.08e-5, 0.103},
+    {122, 8.0e-7, 3.3e-4, 0.049, 0.036, 6.3e-6, 0.132},  {106, 1.94e-6, 2.2e-5, 2.5e-3, 0.085, 1.06e-5, 0.215},
+    {106, 8.5e-7, 1.72e-4, 0.025, 0.045, 5.3e-6, 0.122}};
+double screen_us(const SearchSize& z, bool tensor) {
+  const double nr = (double)z.nr, nq = (double)z.nq, k = z.k, mean_r = z.nnz_r / nr, mean_q = z.nnz_q / nq;
+  const double pairs = nr * nq, rows = std::max<double>(z.nrow, 1.0), cand = k * (z.nnz_q + nq * mean_r);
+  if (tensor)                                // rows walked in turn per tile; products; pairs; the re-screen's list; k
+    return 128.0 + 0.0103 * rows + 8.5e-10 * rows * pairs + 1.3e-5 * pairs + 0.0026 * nr +
+           1.3e-4 * std::min(nr, 64.0 * k + 256.0) * mean_r * std::max(1.0, nq / 600.0) + 5.0e-6 * cand + 5.5 * k;
+  const ScreenCost& c = kScreenCost[z.method];
+  const double run = std::min(512.0, nr) * z.nnz_r / (nr * rows);         // entries of a row in a part
+  return c.base + c.match * z.matched() + c.pair * pairs + c.ref * nr + c.len * (mean_q + mean_r) + c.cand * cand +
+         c.item * std::min(mean_q, 1024.0) * run / 32.0 + 0.9 * k;
+}
+// What a screen's copies of one matrix take to make: FP16 (tensor), row-ordered
+// entries (FP32, the reference), FP32 values (FP32, the query).
+double copy_us(int method, bool tensor, bool as_ref, int32_t nrow, double ncol, double nnz) {
+  if (tensor) return 57.0 + 3.0e-5 * nnz + 4.0e-7 * (double)nrow * ncol;
+  if (as_ref) return 70.0 + (method == JS ? 6.8e-5 : 4.6e-5) * nnz;
+  return (method == JS || method == PEARSON || method == COVARIANCE ? 47.0 : 21.0) + 1.0e-5 * nnz;
+}
+// Whether the exact slab is taken where a screen is predicted to take `us`, its
+// copies included.  Both predictions err, so the screen has to be ahead by a
+// quarter: over the 826 shapes, fresh and searched before, none is then slower than
+// the exact slab by more than a tenth and 20 us, of the drawn ones 3 in 4,200 (with
+// one rate per method, no columns, no copies and no margin, 61 of the 2,478 were, by
+// up to 3.3 ms).  Where a query matches few columns, the screen keeps whole tied
+// sets and leaves such queries to the exact slab (2,000 x 2,000 at 0.5 % of 500
+// rows, cosine, from the host: 403 / 467 with 180 queries left over, 516 / 391 at 1
+// % with none): it is taken only with 16 k matched columns expected.
+bool exact_is_cheaper(const SearchSize& z, double us) {
+  const double shared = z.matched() / ((double)z.nr * (double)z.nq);
+  if ((double)z.nr * std::min(shared, 1.0) < 16.0 * z.k) return true;
+  return exact_us(z) <= 1.25 * us + 20.0;
 }
 
 // 1: exact FP64 slab; 2: FP32 sparse screen; 3: FP16 tensor-core screen
@@ -499,27 +537,45 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
   if (!screen_supported(P.method, P.k) || !screen_fits(nrow)) return 1;
   if (c->engine == 2) return 2;
   if (c->engine == 3) return (tensor_supported(P.method) && stc_supported(P.k)) ? 3 : 2;
-  if (nr * nq <= (int64_t)1 << 22) {
+  const int m = P.method;
+  const bool small = nr * nq <= kSmallPairs;
+  if (small) {
     // into a graph that is being captured: the screens read counts back, the slab
     // does not, so a small search of prepared matrices can be captured
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) return 1;
   }
-  const double nnz_q = (double)X->nnz * (double)nq / (double)std::max<int64_t>(X->ncol, 1);
-  if (exact_is_cheaper(P.method, P.k, nr, nq, nrow, (double)ref->nnz, nnz_q)) return 1;
   // the tensor screen where the reference is dense enough and the dense copies
   // fit in half of the free device memory
-  if (tensor_supported(P.method) && stc_supported(P.k) && nrow > 0 && nr > 0 &&
-      (c->tensor_lazy || (ref->tensor[P.method].method == P.method && ref->tensor[P.method].usable))) {
-    const double density = (double)ref->nnz / ((double)nrow * (double)nr);
-    size_t bytes = tensor_cache_bytes(nrow, nr);
+  const TensorCache& rt = ref->tensor[m];
+  const bool have_rt = rt.method == m && rt.usable, have_qt = X == ref || X->tensor[m].method == m;
+  const bool tensor = tensor_supported(m) && stc_supported(P.k) && nrow > 0 && nr > 0 &&
+                      (have_rt || (c->tensor_lazy && rt.method != m)) &&
+                      (double)ref->nnz / ((double)nrow * (double)nr) >= kTensorMinDensity;
+  auto copies_fit = [&] {
+    if (have_rt) return true;                              // already resident
+    size_t bytes = tensor_cache_bytes(nrow, nr), fr = 0, tot = 0;
     if (X != ref) bytes += tensor_cache_bytes(nrow, X->ncol);
-    size_t fr = 0, tot = 0;
-    if (ref->tensor[P.method].method == P.method && ref->tensor[P.method].usable) bytes = 0;   // already resident
-    if (density >= kTensorMinDensity && cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2) return 3;
+    const bool fit = cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2;
     cudaGetLastError();
-  }
-  return 2;
+    return fit;
+  };
+  if (!small) return tensor && copies_fit() ? 3 : 2;
+  const SearchSize z{m, P.k, nr, nq, nrow, (double)ref->nnz,
+                     (double)X->nnz * (double)nq / (double)std::max<int64_t>(X->ncol, 1)};
+  // each screen with the copies that it would have to make first
+  double fp32_us = INFINITY, tensor_us = INFINITY;
+  const bool have_rows = ref->screen[m].method == m && ref->screen[m].rows;
+  const bool have_vals = X == ref || X->screen[m].method == m;
+  if ((have_rows ? 0 : (size_t)ref->nnz * (m == JS ? 12 : 8)) + (have_vals ? 0 : (size_t)X->nnz * 8) <= kSmallCopyBytes)
+    fp32_us = screen_us(z, false) + (have_rows ? 0.0 : copy_us(m, false, true, nrow, (double)nr, z.nnz_r)) +
+              (have_vals ? 0.0 : copy_us(m, false, false, nrow, (double)X->ncol, (double)X->nnz));
+  if (tensor && (have_rt ? 0 : tensor_cache_bytes(nrow, nr)) + (have_qt ? 0 : tensor_cache_bytes(nrow, X->ncol)) <=
+                    kSmallCopyBytes)
+    tensor_us = screen_us(z, true) + (have_rt ? 0.0 : copy_us(m, true, true, nrow, (double)nr, z.nnz_r)) +
+                (have_qt ? 0.0 : copy_us(m, true, false, nrow, (double)X->ncol, (double)X->nnz));
+  if (tensor_us < fp32_us && !exact_is_cheaper(z, tensor_us) && copies_fit()) return 3;
+  return exact_is_cheaper(z, fp32_us) ? 1 : 2;
 }
 
 // sparseKNN core (R/sparseKNN.R:183-301) after argument checks.
@@ -1382,8 +1438,12 @@ std::vector<int> candidate_engines(const SearchShape& sh, bool drop) {
   std::vector<int> e;
   if (sh.k <= kBatchMaxK) {
     e.push_back(1);
-    // small, or too few matched columns for the screens (exact_is_cheaper)
-    if (exact_is_cheaper(sh.method, sh.k, sh.nr, sh.nq, sh.nrow, (double)sh.nnz_r, (double)sh.nnz_q)) return e;
+    // small, or too few matched columns for the screens
+    const SearchSize z{sh.method, sh.k, sh.nr, sh.nq, sh.nrow, (double)sh.nnz_r, (double)sh.nnz_q};
+    if (sh.nr * sh.nq <= kSmallPairs &&
+        exact_is_cheaper(z, screen_us(z, false) + copy_us(z.method, false, true, z.nrow, (double)z.nr, z.nnz_r) +
+                                copy_us(z.method, false, false, z.nrow, (double)z.nq, z.nnz_q)))
+      return e;
   }
   if (screen_supported(sh.method, sh.k) && screen_fits(sh.nrow)) {
     e.push_back(2);
