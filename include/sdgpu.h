@@ -348,7 +348,8 @@ SDG_API int sdg_ctx_set_stream(sdg_ctx* ctx, void* stream);
  * whose candidate buffer overflowed (finished by the exact path), out[3] =
  * kernels launched, out[4] = screening kernel time in microseconds (device
  * events), out[5] = total device time in microseconds, out[6] = dense flops
- * of the tensor-core screen's GEMMs. */
+ * of the tensor-core screen's GEMMs, out[7] = blocks of a dense search that
+ * repeated with running lists. */
 SDG_API int sdg_last_stats(sdg_ctx* ctx, int64_t* out, int n);
 
 /* Device time of the kernel that bounds the kNN path (the pair-value slab of

@@ -178,7 +178,8 @@ class Context:
         check(self.lib.sdg_last_stats(self.handle, out.ctypes.data, 8))
         return {"pairs_screened": int(out[0]), "pairs_exact": int(out[1]),
                 "overflow_queries": int(out[2]), "kernels": int(out[3]),
-                "screen_us": int(out[4]), "device_us": int(out[5]), "tensor_flops": int(out[6])}
+                "screen_us": int(out[4]), "device_us": int(out[5]), "tensor_flops": int(out[6]),
+                "repeated_blocks": int(out[7])}
 
 
 _tls = threading.local()

@@ -969,7 +969,7 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
   float *segtop = nullptr, *cut = nullptr;
   int32_t *cand = nullptr, *count = nullptr, *over = nullptr, *o_idx = idx;
   int64_t* off = nullptr;
-  int* tc_status = nullptr;                            // the fused screen's wait status (0 = ok)
+  int* tc_status = nullptr;                            // the fused screen's status (see tc_screen)
   double *vals = nullptr, *o_val = dist_out, *row = nullptr;
   if (!fused) {
     DK(cudaMallocAsync(&S, sizeof(float) * (size_t)(chunk * ldS), s));
@@ -982,8 +982,8 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
   DK(cudaMallocAsync(&vals, sizeof(double) * (size_t)(chunk * cap), s));
   if (smode == 0) DK(cudaMallocAsync(&off, sizeof(int64_t) * (size_t)(chunk + 1), s));
   if (fused) {
-    DK(cudaMallocAsync(&tc_status, sizeof(int), s));
-    DK(cudaMemsetAsync(tc_status, 0, sizeof(int), s));
+    DK(cudaMallocAsync(&tc_status, 2 * sizeof(int), s));
+    DK(cudaMemsetAsync(tc_status, 0, 2 * sizeof(int), s));
   }
   if (!device_out) {
     DK(cudaMallocAsync(&o_idx, sizeof(int32_t) * (size_t)(nq * k), s));
@@ -1085,13 +1085,13 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
     launch_select(sa, s);
     DK(cudaGetLastError());
     std::vector<int32_t> h_over((size_t)nb), h_count((size_t)nb);
-    int h_status = 0, h_build = 0;
+    int h_status[2] = {0, 0}, h_build = 0;
     DK(cudaMemcpyAsync(h_over.data(), over, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
     DK(cudaMemcpyAsync(h_count.data(), count, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
-    if (tc_status) DK(cudaMemcpyAsync(&h_status, tc_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (tc_status) DK(cudaMemcpyAsync(h_status, tc_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (build_err) DK(cudaMemcpyAsync(&h_build, build_err, sizeof(int), cudaMemcpyDeviceToHost, s));
     DK(cudaStreamSynchronize(s));
-    if (h_build || h_status) {
+    if (h_build || h_status[0]) {
       // the flags were raised before this chunk's kernels ran on the results;
       // nothing is returned
       release_all();
@@ -1099,6 +1099,7 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
       if (h_build) return fail_with(SDG_E_NONFINITE, "Cosine requires finite input (found NA, NaN or Inf).");
       return fail_with(SDG_E_CUDA, "tensor-core screen: a pipeline wait timed out");
     }
+    ctx_stats_add(ctx, 7, h_status[1] ? 1 : 0);
     for (int64_t t = 0; t < nb; ++t) {
       if (h_over[(size_t)t]) overflow.push_back(c0 + t);
       ctx_stats_add(ctx, 1, h_over[(size_t)t] ? n : h_count[(size_t)t]);   // pairs valued exactly

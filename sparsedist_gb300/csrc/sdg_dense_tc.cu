@@ -804,7 +804,11 @@ __device__ __forceinline__ void tight_bounds(const MergeArgs& A, float s, int64_
 // the k-th largest per-pair lower bound (tight_bounds) among them is again at
 // most the exact k-th best key (k candidates reach it), so every member of the
 // exact top k (ties included) has its per-pair upper bound at or above
-// dense_cut(max(T, T2)) and is kept.
+// dense_cut(max(T, T2)) and is kept.  Where more pass the first cut than the table
+// holds, T2 is taken over all appended references instead (400,000 references in 50
+// clusters, 1,000 queries, k = 5: 913 queries had 576 and more; the block repeated
+// with running lists and 26 queries still went through exact rows, 223 ms; 9 ms now
+// and 1 such query).
 //
 // A list keeps only keys above the shared key it saw, so when some list's
 // view of the shared key reached the final k-th best, fewer than k keys at or
@@ -888,14 +892,17 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
   int32_t* out = A.cand + ql * (int64_t)A.cap;
   float* out_s = A.cand_s + ql * (int64_t)A.cap;
   const int all = pre[used - 1];
-  for (int p = rank; p < all; p += nt) {
+  auto place = [&](int p) -> int64_t {                // of the p-th appended reference
     int lo = 0, hi = used - 1;                       // the first list whose inclusive count exceeds p
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       if (pre[mid] > p) hi = mid;
       else lo = mid + 1;
     }
-    const int64_t at = (ql * A.nslots + lo) * (int64_t)A.ecap + (p - (lo ? pre[lo - 1] : 0));
+    return (ql * A.nslots + lo) * (int64_t)A.ecap + (p - (lo ? pre[lo - 1] : 0));
+  };
+  for (int p = rank; p < all; p += nt) {
+    const int64_t at = place(p);
     const int32_t ref = A.eidx[at];
     const float sv = A.es[at];
     float key, err;
@@ -907,9 +914,61 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
   }
   G.sync();                                          // the kept pairs are visible to the group
   int total = s_kept[slot_q];
-  ovf = total > A.cap;
-  if (!ovf && total > K) {
-    const float qe = A.qe[q], qn = A.qn[q];
+  const float qe = A.qe[q], qn = A.qn[q];
+  if (total > A.cap) {
+    // More than the table holds (a query in a dense cluster, whose references lie
+    // within the uniform bound of one another): the second cut is taken over all
+    // appended references, T2 by a histogram of eight bits of the key at a time.
+    uint32_t prefix = 0, want = (uint32_t)K;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      for (int i = rank; i < 256; i += nt) keys[i] = 0u;
+      G.sync();
+      for (int p = rank; p < all; p += nt) {
+        const int64_t at = place(p);
+        float lo, hi;
+        tight_bounds(A, A.es[at], A.eidx[at], Nq, qe, qn, lo, hi);
+        const uint32_t key = fkey(fmaxf(lo, -INFINITY));
+        if (shift == 24 || (key >> (shift + 8)) == prefix) atomicAdd(&keys[(key >> shift) & 255u], 1u);
+      }
+      G.sync();
+      // lane l: bins 255 - 8 l downwards (every warp of the group alike)
+      uint32_t own = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) own += keys[255 - 8 * lane - j];
+      uint32_t x = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      const int src = __ffs(__ballot_sync(0xffffffffu, x >= want)) - 1;   // all >= want: some lane reaches it
+      uint32_t above = x - own;
+      int bin = 255 - 8 * lane;
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+        if (bin == 255 - 8 * lane - j && above + keys[bin] < want) above += keys[bin--];
+      prefix = (prefix << 8) | (uint32_t)__shfl_sync(0xffffffffu, bin, src);
+      want -= __shfl_sync(0xffffffffu, above, src);
+      G.sync();
+    }
+    const float cut2 = dense_cut(fmaxf(T, fkey_value(prefix)));
+    if (rank == 0) s_kept[slot_q] = 0;
+    G.sync();
+    for (int p = rank; p < all; p += nt) {
+      const int64_t at = place(p);
+      const int32_t ref = A.eidx[at];
+      const float sv = A.es[at];
+      float lo, hi;
+      tight_bounds(A, sv, ref, Nq, qe, qn, lo, hi);
+      if (hi >= cut2) {
+        const int w = atomicAdd(&s_kept[slot_q], 1);
+        if (w < A.cap) { out[w] = ref; out_s[w] = sv; }
+      }
+    }
+    G.sync();
+    total = s_kept[slot_q];
+    ovf = total > A.cap;
+  } else if (total > K) {
     for (int p = rank; p < total; p += nt) {
       float lo, hi;
       tight_bounds(A, out_s[p], out[p], Nq, qe, qn, lo, hi);
@@ -945,7 +1004,6 @@ __global__ void __launch_bounds__(WPQ == 1 ? 256 : WPQ * 32) k_tc_merge(MergeArg
   if (rank == 0) {
     A.count[ql] = ovf ? 0 : total;
     A.over[ql] = ovf ? 1 : 0;
-    if (ovf && A.any_over) *A.any_over = 1;
   }
 }
 
@@ -1169,7 +1227,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
   int32_t *ecount = nullptr, *eidx = nullptr;
   unsigned* tshared = nullptr;
-  int* any = nullptr;
+  int* any = status + 1;                               // a list overflowed: the block repeats
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   const int64_t nw = ntiles * BN, nw1 = ntiles1 * BN;
@@ -1177,7 +1235,6 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   if (first) {
     chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw1, s));
     chk(cudaMallocAsync(&maxima, sizeof(float) * (size_t)(nq * m), s));
-    chk(cudaMallocAsync(&any, sizeof(int), s));
     if (e == cudaSuccess) chk(cudaMemsetAsync(any, 0, sizeof(int), s));
   }
   chk(cudaMallocAsync(&lists, sizeof(float) * (size_t)(nq * nslots * k), s));
@@ -1258,11 +1315,10 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     };
     M.any_over = any; M.gate = nullptr;
     merge(M);
-    // A query in a dense cluster can have thousands of references between its
-    // threshold and its k-th best key (400,000 references in 50 clusters, k = 5: a
-    // list of 913 of 1,000 queries overflowed; exact rows for them took 7.8 s).
-    // Then the block runs once more with running lists, which tighten as they
-    // go, from the same thresholds; otherwise both launches return at once.
+    // Where a list overflows all the same (thousands of references of one span
+    // within the bound of a query's threshold), the block runs once more with
+    // running lists, which tighten as they go, from the same thresholds; otherwise
+    // both launches return at once.
     if (first) {
       P.gate = any;
       launch(pick_kernel(pair), grid, rmap, P);
@@ -1271,7 +1327,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     }
   }
   // stream-ordered frees: the caller reads *status with its own results
-  for (void* p : {(void*)w, (void*)wp, (void*)maxima, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared, (void*)any})
+  for (void* p : {(void*)w, (void*)wp, (void*)maxima, (void*)lists, (void*)ecount, (void*)eidx, (void*)es, (void*)cand_s, (void*)tshared})
     if (p) cudaFreeAsync(p, s);
   if (e != cudaSuccess) {
     set_error(cudaGetErrorString(e));
