@@ -116,6 +116,34 @@ struct Cfg {
 };
 static_assert(Cfg<true>::STAGES <= MAX_STAGES && Cfg<false>::STAGES <= MAX_STAGES, "barrier space");
 
+// The sample of every s-th reference.  The matrix is SAMPLE_RUNS runs of `span`
+// references, a place of a run is s references, and sample tile t takes one
+// reference (the (t mod s)-th) of each of SAMPLE_PLACES neighbouring places in
+// every run.  A tile half is then spread over half of the matrix, so references
+// stored class by class are sampled as evenly as shuffled ones: a tile of 256
+// neighbouring places sees one class, the k-th best of the maxima lies outside a
+// query's class, its lists overflow and the block repeats.  Screen us of
+// references stored in cluster order with 2 / 16 / 64 / 256 runs: 400,000 x 128 in 100
+// clusters 2,924 / 837 / 785 / 792, 1,000,000 x 256 in 1,000 3,921 / 3,110 / 2,087 /
+// 1,997, 1,000,000 x 64 in 20,000 669 / 647 / 593 / 506; of others, 2,000,000 x 256:
+// 2,249 / 2,268 / 2,274 / 2,462.
+constexpr int SAMPLE_RUNS = 64, SAMPLE_PLACES = BN / SAMPLE_RUNS;
+struct SampleMap {
+  int s;
+  int64_t span, tiles;
+  // the reference of column c
+  __host__ __device__ __forceinline__ int64_t at(int64_t c) const {
+    const int64_t t = c / BN, col = c % BN;
+    return col / SAMPLE_PLACES * span + (t * SAMPLE_PLACES + col % SAMPLE_PLACES) * s + t % s;
+  }
+  // the column of reference r, or -1
+  __host__ __device__ __forceinline__ int64_t column(int64_t r) const {
+    const int64_t run = r / span, p = r % span / s, t = p / SAMPLE_PLACES;
+    if (run >= SAMPLE_RUNS || t >= tiles || r % span % s != t % s) return -1;
+    return t * BN + run * SAMPLE_PLACES + p % SAMPLE_PLACES;
+  }
+};
+
 struct TcArgs {
   int method, k, dch, ecap;
   int self;                   // queries are columns of the reference (skip r == q)
@@ -132,7 +160,7 @@ struct TcArgs {
   float* lists;               // [nq][nslots][k] (one pass)
   float* maxima;              // MODE 1: [nq][2 * ntiles * gran]
   int gran;                   // MODE 1: maxima per tile half (1 or 4)
-  int sample;                 // MODE 1: the sample's stride (sampled)
+  SampleMap sample;           // MODE 1
   const int* gate;            // nothing to do unless *gate is set (null: always run)
   int use_w;                  // MODE 1, cosine: some reference is degenerate
   int32_t* ecount;            // [nq][nslots]
@@ -185,11 +213,6 @@ __host__ __device__ __forceinline__ int64_t last_cta(int64_t g, int64_t ntiles, 
 __host__ __device__ __forceinline__ int32_t tile_of(int64_t f, int64_t g, int64_t ntiles, int64_t per) {
   return (int32_t)((f - g * ntiles + (g * ntiles) % per) % ntiles);
 }
-
-// Column c of a sample of stride s is reference c s + (c / BN) mod s: every
-// s-th reference, from another place in each tile, so that references stored in
-// turn by class (period s, or a multiple or divisor of it) are sampled alike.
-__host__ __device__ __forceinline__ int64_t sampled(int64_t c, int s) { return c * s + (c / BN) % s; }
 
 // MODE 0: running lists, one pass over the references; for few references.
 // MODE 1 keeps no list: every thread stores the largest x' = a s - w[r] of each
@@ -300,13 +323,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
               if (leader) mbar_expect_tx(full + s, 2u * B_BYTES);
               const uint32_t bar = cluster_addr(full + s, 0);
               if constexpr (MODE == 1)
-                tma_load_3d_pair(sB + (size_t)s * B_BYTES, &rmap, bar, c * BK, tile % P.sample, rcol);
+                tma_load_4d_pair(sB + (size_t)s * B_BYTES, &rmap, bar, c * BK, tile % P.sample.s, tile * SAMPLE_PLACES,
+                                 (int)crank * (SAMPLE_RUNS / 2));
               else
                 tma_load_2d_pair(sB + (size_t)s * B_BYTES, &rmap, bar, c * BK, rcol);
             } else {
               mbar_expect_tx(full + s, B_BYTES);
               if constexpr (MODE == 1)
-                tma_load_3d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, tile % P.sample, rcol);
+                tma_load_4d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, tile % P.sample.s, tile * SAMPLE_PLACES,
+                            0);
               else
                 tma_load_2d(sB + (size_t)s * B_BYTES, &rmap, full + s, c * BK, rcol);
             }
@@ -606,7 +631,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_dense_tc(const __grid_constant__
       active = ql < P.nq;
       if (active) active = !P.qempty[q];           // a degenerate query has no list
       Nq = active ? P.qnorm2[q] : 0.f;
-      if (MODE == 1) own = sampled(q / P.sample, P.sample) == q ? q / P.sample : -1;
+      if (MODE == 1) own = P.sample.column(q);
 #pragma unroll
       for (int i = 0; i < KL; ++i) lst[i] = (i < KL - K) ? INFINITY : -INFINITY;
       T = -INFINITY;
@@ -1014,18 +1039,17 @@ __global__ void k_tc_key_init(int64_t nq, unsigned* keys) {
 
 // w[r]: +inf for degenerate references and the padding; 0 (cosine) or
 // (1 - c) Nr (euclidean) otherwise; wp: the same with one_plus_c for the x' of
-// a first pass over n1 sampled references, padded to nw1 (at most nw; 0 without
-// one)
+// a first pass over n1 sampled references (at most nw; 0 without one)
 __global__ void k_tc_weights(int method, int64_t n, int64_t nw, float one_minus_c,
-                             const float* norm2, const uint8_t* empty, float* w, int sample, int64_t n1, int64_t nw1,
-                             float one_plus_c, float* wp) {
+                             const float* norm2, const uint8_t* empty, float* w, SampleMap sample,
+                             int64_t n1, float one_plus_c, float* wp) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   auto weight = [&](int64_t r, float c) {
     if (r >= n || empty[r]) return INFINITY;
     return (method == COSINE) ? 0.f : c * norm2[r];
   };
   if (i < nw) w[i] = weight(i, one_minus_c);
-  if (i < nw1) wp[i] = i < n1 ? weight(sampled(i, sample), one_plus_c) : INFINITY;
+  if (i < n1) wp[i] = weight(sample.at(i), one_plus_c);
 }
 
 // Two passes: each query's threshold, the k-th largest of its maxima less what
@@ -1084,8 +1108,8 @@ int64_t maxima_per_query(int64_t refs, int k) { return 2 * ((refs + BN - 1) / BN
 // with running lists) where even all references give fewer than 4 k maxima.  A
 // stride of s leaves about s k references of a query above the threshold, and
 // the 768 slots of the query's shortest set of lists (two) have to hold them
-// with room to spare, hence s k <= 192 (clusters that overflow them all the same
-// are repeated with running lists, see tc_screen); the first pass costs 1 / s of the second
+// with room to spare, hence s k <= 192 (what overflows them all the same is
+// repeated with running lists, see tc_screen); the first pass costs 1 / s of the second
 // and the candidates are re-bounded by the merge, so there is nothing to gain
 // beyond 8; below 16 k maxima the threshold drops (3,000 x 60,000, d = 64, k =
 // 30: 110 us with s = 6 and 4 k maxima against 108, the merge 13 us longer).
@@ -1093,11 +1117,16 @@ int64_t maxima_per_query(int64_t refs, int k) { return 2 * ((refs + BN - 1) / BN
 // 150,000: 487 / 300; 128 x 2,000,000: 233 / 194; 1 x 2,000,000: 170 / 184, but
 // merge and re-rank of fewer candidates make it 430 / 406 a call; 8 x 200,000,
 // euclidean: 127 / 37.  s = 1 / rule: 777 x 150,001, d = 100: 96 / 90.
-int sample_stride(int64_t n, int k) {
-  if (maxima_per_query(n, k) < 4 * (int64_t)k || maxima_per_query(n, k) > INT32_MAX) return 0;
+SampleMap sample_of(int64_t n, int k) {
+  auto with = [&](int s) {
+    const int64_t span = n / SAMPLE_RUNS / s * s;
+    return SampleMap{s, span, span / s / SAMPLE_PLACES};
+  };
+  auto maxima = [&](int s) { return maxima_per_query(with(s).tiles * BN, k); };
+  if (maxima(1) < 4 * (int64_t)k || maxima(1) > INT32_MAX) return SampleMap{0, 1, 0};
   int s = std::max(1, std::min(8, 192 / k));
-  while (s > 1 && maxima_per_query(n / s, k) < 16 * (int64_t)k) --s;
-  return s;
+  while (s > 1 && maxima(s) < 16 * (int64_t)k) --s;
+  return with(s);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1147,14 +1176,15 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
-  // the references in n / sample whole runs of `sample` columns: a box takes the
-  // column at one place of each of box_cols runs
-  auto encode_sample = [&](int sample, int box_cols, CUtensorMap* map) {
-    const cuuint64_t gdim[3] = {(cuuint64_t)D->dpad, (cuuint64_t)sample, (cuuint64_t)(D->n / sample)};
-    const cuuint64_t gstride[2] = {(cuuint64_t)D->dpad * 2, (cuuint64_t)D->dpad * 2 * sample};
-    const cuuint32_t box[3] = {(cuuint32_t)BK, 1, (cuuint32_t)box_cols};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base_of(D), gdim, gstride, box, estr,
+  // a box: one of the s references of SAMPLE_PLACES places of `runs` runs
+  auto encode_sample = [&](const SampleMap& z, int runs, CUtensorMap* map) {
+    const cuuint64_t ld = (cuuint64_t)D->dpad * 2;
+    const cuuint64_t gdim[4] = {(cuuint64_t)D->dpad, (cuuint64_t)z.s, (cuuint64_t)(z.span / z.s),
+                                (cuuint64_t)SAMPLE_RUNS};
+    const cuuint64_t gstride[3] = {ld, ld * z.s, ld * z.span};
+    const cuuint32_t box[4] = {(cuuint32_t)BK, 1, (cuuint32_t)SAMPLE_PLACES, (cuuint32_t)runs};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base_of(D), gdim, gstride, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
@@ -1168,8 +1198,8 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   };
   // thresholds from a sample (MODE 1), then the references that pass (MODE 2,
   // 3); or one pass with running lists (MODE 0)
-  const int sample = sample_stride(n, k);
-  const bool first = sample > 0;
+  const SampleMap sample = sample_of(n, k);
+  const bool first = sample.s > 0;
   // CTA pairs (clusters of two; the work unit is then a pair) where they pay or
   // are asked for and the device can hold such clusters.  A pair's SM receives
   // half the bytes of a reference chunk.  One CTA / pairs, us: 4,096 x 2,000,000,
@@ -1219,7 +1249,8 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   const float rel = 0.0040f + (float)D->d * 2.384185791015625e-7f;
   const float omc = 1.f - (rel + 9.5367431640625e-7f);
 
-  const int64_t n1 = first ? n / sample : 0, ntiles1 = (n1 + BN - 1) / BN;
+  int* any = status + 1;                               // a list overflowed: the block repeats
+  const int64_t ntiles1 = sample.tiles, n1 = ntiles1 * BN;
   const int gran = (int)granularity(n1, k);
   const int64_t m = 2 * ntiles1 * gran;
   const float opc = 1.f + rel + 1.9073486328125e-6f;     // 2^-19
@@ -1227,13 +1258,12 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
   float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;
   int32_t *ecount = nullptr, *eidx = nullptr;
   unsigned* tshared = nullptr;
-  int* any = status + 1;                               // a list overflowed: the block repeats
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-  const int64_t nw = ntiles * BN, nw1 = ntiles1 * BN;
+  const int64_t nw = ntiles * BN;
   chk(cudaMallocAsync(&w, sizeof(float) * (size_t)nw, s));
   if (first) {
-    chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)nw1, s));
+    chk(cudaMallocAsync(&wp, sizeof(float) * (size_t)n1, s));
     chk(cudaMallocAsync(&maxima, sizeof(float) * (size_t)(nq * m), s));
     if (e == cudaSuccess) chk(cudaMemsetAsync(any, 0, sizeof(int), s));
   }
@@ -1247,8 +1277,8 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     // every query's shared key starts at fkey(-inf) or at its threshold
     if (!first) k_tc_key_init<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(nq, tshared);
     chk(cudaMemsetAsync(ecount, 0, sizeof(int32_t) * (size_t)(nq * nslots), s));
-    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, D->norm2, D->empty, w, sample, n1,
-                                                             nw1, opc, wp);
+    k_tc_weights<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(method, n, nw, omc, D->norm2, D->empty, w, sample, n1, opc,
+                                                             wp);
     TcArgs P;
     P.method = method; P.k = k; P.dch = dch; P.ecap = ecap;
     P.self = self ? 1 : 0;
@@ -1275,7 +1305,7 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     sdg_time_begin(ctx);
     if (first) {
       CUtensorMap map1;
-      if (!encode_sample(sample, pair ? Cfg<true>::BNL : Cfg<false>::BNL, &map1)) chk(cudaErrorInvalidValue);
+      if (!encode_sample(sample, pair ? SAMPLE_RUNS / 2 : SAMPLE_RUNS, &map1)) chk(cudaErrorInvalidValue);
       const int64_t items1 = G * ntiles1;
       TcArgs P1 = P;
       P1.w = wp; P1.n = n1; P1.ntiles = ntiles1;

@@ -1,12 +1,14 @@
-"""The dense screen on clustered references: queries with more candidates within
-the uniform bound than the table holds are cut by the per-pair bound; a tight cluster that overflows the lists repeats the block with running
+"""The dense screen on clustered references: stored cluster by cluster or in turn,
+the sample's thresholds leave the lists room (no block repeats); queries with more
+candidates within the uniform bound than the table holds are cut by the per-pair
+bound; a tight cluster that overflows the lists repeats the block with running
 lists, for every list length and on CTA pairs.  Bit for bit against the slab
 screen (mode 2)."""
 import numpy as np
 import pytest
 
 from backends import same_bits
-from test_gpu_dense import dense_query
+from test_gpu_dense import dense_knn, dense_query
 from test_gpu_dense_two_pass import upload
 
 pytestmark = pytest.mark.gpu
@@ -39,6 +41,16 @@ def check(R, Q, code, k, mode):
     ctx.lib.sdg_dense_free(h)
     assert same_bits(got[0], want[0]) and same_bits(got[1], want[1])
     return stats
+
+
+@pytest.mark.parametrize("code", [1, 2])
+@pytest.mark.parametrize("order", ["in order", "in turn", "shuffled"])
+@pytest.mark.parametrize("n,d,nq,classes,k", [(150000, 64, 700, 30, 10), (120000, 160, 256, 100, 15),
+                                              (100003, 100, 300, 7, 3)])
+def test_no_block_repeats(code, order, n, d, nq, classes, k):
+    R, Q = clusters(n, nq, d, classes, 0.3, d, order)
+    stats = check(R, Q, code, k, 0)
+    assert stats["repeated_blocks"] == 0 and stats["overflow_queries"] == 0
 
 
 def beyond_the_table(R, Q, code, k):
@@ -84,3 +96,15 @@ def test_blocks_repeat(code, d, mode, k):
     R[5] = 0.0
     stats = check(R, Q, code, k, mode)
     assert stats["repeated_blocks"] == 1
+
+
+def test_self_search_own_column():
+    """The query's own column in and out of the sample, at the ends of runs."""
+    from sparsedist_gb300 import _lib
+    R, _ = clusters(20011, 1, 48, 9, 0.3, 5, "in order")
+    ctx = _lib.Context()
+    h = upload(ctx, R)
+    for q0, nq in ((0, 700), (9000, 300), (19900, 111)):
+        got, want = (dense_knn(ctx, h, q0, nq, 1, 4, mode) for mode in (0, 2))
+        assert same_bits(got[0], want[0]) and same_bits(got[1], want[1])
+    ctx.lib.sdg_dense_free(h)
