@@ -1128,12 +1128,12 @@ static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, const ColAu
 }
 
 // The entries of M in row order (see k_rows_fill), built by the first search
-// that screens against M and kept with it.  The lock and the synchronisation
-// make it complete before any other stream reads it.  rows stays null when the
-// device has no room for it.
-static int ensure_rows(ScreenCache* c, const DevCsc& M, cudaStream_t s) {
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
+// that screens against M and kept with it.  The matrix's lock and the
+// synchronisation make it complete before any other stream reads it; searches of
+// other matrices do not wait for it.  rows stays null when the device has no room
+// for it.
+static int ensure_rows(ScreenCache* c, const DevCsc& M, std::mutex* mu, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(*mu);
   if (c->rows || M.ncol == 0 || M.nrow == 0) return 0;
   // sub-ranges of 512 to 4,096 columns, about eight entries a cell
   const double density = (double)c->nnz_total / ((double)M.nrow * (double)M.ncol);
@@ -1227,7 +1227,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   const int64_t nr = ref.ncol, nq = qry.ncol;
   const int32_t nrow = ref.nrow;
   if (!use_t) {
-    SKN((cudaError_t)ensure_rows(rc, ref, s));
+    SKN((cudaError_t)ensure_rows(rc, ref, r.rows_mu, s));
     if (!rc->rows) {                               // no room for the row-ordered entries: every query exactly
       const int64_t lo = r.q_lo, hi = (r.q_hi < 0) ? nq : r.q_hi;
       if (hi > lo) hooks.exact_range(lo, hi - lo);

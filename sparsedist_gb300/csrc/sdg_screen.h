@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cuda_fp16.h>
 #include <functional>
+#include <mutex>
 #include <vector>
 
 #include "sdg_common.cuh"
@@ -56,6 +57,7 @@ struct TensorCache {
 };
 
 struct ScreenRun {
+  std::mutex* rows_mu = nullptr;           // the reference's: one thread builds its row-ordered entries
   int method = 0, dist = 1, k = 1;
   // the tensor-core screen (the fused tcgen05 FP16 screen, sdg_sparse_tc.cu)
   // instead of the FP32 sparse screen, when tensor_supported(method),
