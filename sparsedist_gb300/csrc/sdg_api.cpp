@@ -1782,7 +1782,7 @@ namespace {
 // tensor screen builds one for the queries: ld x ncol halves plus per-column
 // bounds).
 int64_t request_mem(const sdg_server* S, int method, int64_t ncol, int64_t nnz, int k) {
-  if (S->dref) return dense_query_bytes(S->dref, ncol, k);
+  if (S->dref) return dense_query_bytes(S->dref, ncol, method, k);
   const int64_t nr = S->ref->ncol;
   const int64_t slab_cols = std::min<int64_t>(ncol, std::max<int64_t>(16, ((int64_t)4 << 30) / (4 * std::max<int64_t>(nr, 1))));
   const int64_t cap = std::max(256, std::min(8192, 16 * k + 64));

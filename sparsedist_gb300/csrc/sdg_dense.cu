@@ -889,6 +889,15 @@ int query_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, int method, 
   return SDG_OK;
 }
 
+// candidates a query's table holds; queries of a block; the slab's leading
+// dimension and the queries of a pass over it (8 GB)
+int dense_cap(int k) { return std::max(512, std::min(16384, 64 * k + 256)); }
+constexpr int64_t DENSE_CHUNK = 65536;
+int64_t slab_ld(int64_t n) { return (n + 127) / 128 * 128; }
+int64_t slab_chunk(int64_t n, int64_t nq) {
+  return std::max<int64_t>(1, std::min<int64_t>(nq, ((int64_t)8 << 30) / (4 * slab_ld(n))));
+}
+
 // Rows q0 .. q0+nq-1 (query columns of Q) of sparseKNN(Q, R, k, method) with
 // drop_degenerate = TRUE: the self-search with include_self = FALSE when self
 // (Q is R), else the two-matrix search.  See sdg_dense_knn_block for modes.
@@ -955,16 +964,16 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
     ctx_stats_add(ctx, 3, 2 * nq);
     return SDG_OK;
   }
-  const int cap = std::max(512, std::min(16384, 64 * k + 256));
+  const int cap = dense_cap(k);
   // modes 0 and 3 run the fused tensor-core screen where it applies (no slab
-  // in HBM; mode 3 always on CTA pairs, mode 0 where they are faster), else the
-  // BF16 slab screen of mode 2; smode is the bound in force
+  // in HBM; mode 3 on CTA pairs wherever the references are enough for a sample,
+  // mode 0 where they are faster), else the BF16 slab screen of mode 2; smode is
+  // the bound in force
   const bool fused = (mode == 0 || mode == 3) && tc_screen_supported(D, method, k);
   const int smode = (mode == 1) ? 1 : 0;
-  const int64_t ldS = (n + 127) / 128 * 128;
+  const int64_t ldS = slab_ld(n);
   const int nseg = (int)((n + DSEG - 1) / DSEG);
-  const int64_t chunk = fused ? std::min<int64_t>(nq, 65536)
-                              : std::max<int64_t>(1, std::min<int64_t>(nq, ((int64_t)8 << 30) / (4 * ldS)));
+  const int64_t chunk = fused ? std::min<int64_t>(nq, DENSE_CHUNK) : slab_chunk(n, nq);
   float* S = nullptr;
   float *segtop = nullptr, *cut = nullptr;
   int32_t *cand = nullptr, *count = nullptr, *over = nullptr, *o_idx = idx;
@@ -1148,16 +1157,24 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
 namespace sdg {
 int32_t dense_rows(const sdg_dense* D) { return D->d; }
 int64_t dense_cols(const sdg_dense* D) { return D->n; }
-int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int k) {
-  const int64_t cap = std::max(512, std::min(16384, 64 * k + 256));
-  // the query's forms (FP64 x2, FP32 x2, BF16 x2 + padded), candidates and
-  // exact values, results, and the fused screen's per-(query, range) lists
-  // (at most 152 ranges for a single query tile, ~9 for full tiles), the
-  // sample's maxima
-  const int64_t ranges = std::max<int64_t>(9, 152 / std::max<int64_t>(1, (nq + 255) / 256));
-  return nq * (36 * (int64_t)D->dpad + cap * 12 + (int64_t)k * 12 + ranges * (768 * 8 + (int64_t)k * 4 + 4) +
-               D->n / 96 + 128 * (int64_t)k) +
-         ((int64_t)1 << 20);
+int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int method, int k) {
+  // the query's forms (FP64 x2, FP32 x2, BF16, padded BF16, sums, norms and flags) and the results
+  int64_t bytes = ((int64_t)1 << 20) + nq * (36 * (int64_t)D->dpad + 32 + 12 * (int64_t)k);
+  const int64_t avail = std::max<int64_t>(1, D->n - D->n_empty);
+  k = (int)std::min<int64_t>(k, avail);
+  if (k > kMaxK) return bytes + 8 * D->n + ((int64_t)256 << 20);   // one row at a time, the lists' scratch
+  const int cap = dense_cap(k);
+  if (tc_screen_supported(D, method, k)) {
+    const int64_t chunk = std::min<int64_t>(nq, DENSE_CHUNK);
+    int dev = -1;                            // the caller's thread may be on another device
+    cudaGetDevice(&dev);
+    cudaSetDevice(D->device);
+    bytes += chunk * (12 * (int64_t)cap + 16) + tc_screen_bytes(D, method, k, chunk, cap) + 8 * D->n;
+    if (dev >= 0) cudaSetDevice(dev);
+    return bytes;
+  }
+  const int64_t chunk = slab_chunk(D->n, nq);
+  return bytes + chunk * (4 * slab_ld(D->n) + 4 * k * ((D->n + DSEG - 1) / DSEG) + 12 * (int64_t)cap + 20) + 8 * D->n;
 }
 int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int64_t nq, int method, int k,
                 int mode, int32_t* idx, double* dist_out, int device_out, int* k_eff, int* flags) {

@@ -74,8 +74,11 @@ __device__ __forceinline__ float dense_cut(float T) {
 // Queries are columns q0.. of Q, references the columns of D (self: Q is D
 // and each query's own column is skipped).
 bool tc_screen_supported(const sdg_dense* D, int method, int k);
+// device bytes that tc_screen takes for a block of nq queries while it runs
+int64_t tc_screen_bytes(const sdg_dense* D, int method, int k, int64_t nq, int cap);
 // allow_pairs: run CTA pairs (cta_group::2, M = 256) wherever the block has
-// more than one 128-query group; otherwise where they are faster.  status: two
+// more than one 128-query group and the references are enough for a sample;
+// otherwise where they are faster.  status: two
 // device ints, [0] set to 1 by a pipeline wait that ran out, [1] whether the
 // block repeated with running lists; the call returns without synchronising and
 // the caller reads them with the results.

@@ -1129,6 +1129,62 @@ SampleMap sample_of(int64_t n, int k) {
   return with(s);
 }
 
+// How a block of nq queries is cut into work, and the workspace it takes.
+constexpr int ECAP = 768;                    // slots of a list of appended references
+struct TcPlan {
+  SampleMap sample;
+  bool pair = false;
+  int64_t units = 1;                         // CTAs, or CTA pairs, at one time
+  int64_t groups = 0, ntiles = 0, per = 1, grid = 1, nslots = 0, maxima = 0;
+  int gm() const { return pair ? Cfg<true>::GM : Cfg<false>::GM; }
+};
+TcPlan tc_plan(const sdg_dense* D, int method, int k, int64_t nq, bool allow_pairs) {
+  TcPlan z;
+  z.sample = sample_of(D->n, k);
+  // CTA pairs (clusters of two; the work unit is then a pair) where they pay or
+  // are asked for and the device can hold such clusters.  A pair's SM receives
+  // half the bytes of a reference chunk.  One CTA / pairs, us: 4,096 x 2,000,000,
+  // d = 256: 2,557 / 2,280; 1,024 x 800,000, d = 200: 286 / 274; 4,096 x
+  // 2,000,000, d = 128: 1,651 / 1,677; d = 64: 1,440 / 1,488; an odd number of
+  // 128-query groups pads one (257 x 1,000,000, d = 256: 161 / 182).  Blocks of too
+  // few references for a sample run single CTAs.
+  if (z.sample.s > 0 && nq > BM && (allow_pairs || (D->dpad > 2 * BK && (nq + BM - 1) / BM % 2 == 0))) {
+    auto kp = method == COSINE ? k_dense_tc<1, true, 2> : k_dense_tc<1, true, 3>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2, 1, 1); cfg.blockDim = dim3(THREADS, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kp, &cfg) == cudaSuccess && clusters > 0) {
+      z.pair = true;
+      z.units = clusters;
+    }
+    cudaGetLastError();
+  }
+  if (!z.pair) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, D->device);
+    z.units = std::max(sms, 1);
+  }
+  // (query group, reference tile) items in equal contiguous spans, one per unit
+  z.groups = (nq + z.gm() - 1) / z.gm();
+  z.ntiles = (D->n + BN - 1) / BN;
+  const int64_t items = z.groups * z.ntiles;
+  z.grid = std::min<int64_t>(z.units, items);
+  z.per = (items + z.grid - 1) / z.grid;
+  z.grid = (items + z.per - 1) / z.per;
+  // list slots per query: two halves per unit whose span meets its group
+  int64_t most = 1;
+  for (int64_t g = 0; g < z.groups; ++g)
+    most = std::max<int64_t>(most, last_cta(g, z.ntiles, z.per) - first_cta(g, z.ntiles, z.per) + 1);
+  z.nslots = 2 * most;
+  z.maxima = z.sample.s > 0 ? maxima_per_query(z.sample.tiles * BN, k) : 0;
+  return z;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1153,6 +1209,12 @@ int fail(int code, const char* msg) { set_error(msg); return code; }
 bool tc_screen_supported(const sdg_dense* R, int method, int k) {
   return (method == COSINE || method == EUCLIDEAN) && k >= 1 && k <= KT && R->dpad <= MAX_DCH * BK &&
          R->n < (int64_t)1 << 30 && encode_fn() != nullptr;
+}
+
+int64_t tc_screen_bytes(const sdg_dense* D, int method, int k, int64_t nq, int cap) {
+  const TcPlan z = tc_plan(D, method, k, nq, false);
+  const int64_t weights = 4 * BN * (z.ntiles + z.sample.tiles);
+  return weights + nq * (4 * (z.maxima + z.nslots * (k + 1 + 2 * ECAP) + cap) + 4);
 }
 
 int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, int method, int k, int64_t q0,
@@ -1196,63 +1258,27 @@ int tc_screen(sdg_ctx* ctx, const sdg_dense* Q, const sdg_dense* D, bool self, i
     return (k <= 16) ? k_dense_tc<16, false, 0> : (k <= 24) ? k_dense_tc<24, false, 0>
          : (k <= 32) ? k_dense_tc<32, false, 0> : (k <= 48) ? k_dense_tc<48, false, 0> : k_dense_tc<64, false, 0>;
   };
+  const TcPlan plan = tc_plan(D, method, k, nq, allow_pairs);
+  const SampleMap sample = plan.sample;
   // thresholds from a sample (MODE 1), then the references that pass (MODE 2,
   // 3); or one pass with running lists (MODE 0)
-  const SampleMap sample = sample_of(n, k);
   const bool first = sample.s > 0;
-  // CTA pairs (clusters of two; the work unit is then a pair) where they pay or
-  // are asked for and the device can hold such clusters.  A pair's SM receives
-  // half the bytes of a reference chunk.  One CTA / pairs, us: 4,096 x 2,000,000,
-  // d = 256: 2,557 / 2,280; 1,024 x 800,000, d = 200: 286 / 274; 4,096 x
-  // 2,000,000, d = 128: 1,651 / 1,677; d = 64: 1,440 / 1,488; an odd number of
-  // 128-query groups pads one (257 x 1,000,000, d = 256: 161 / 182).
-  int64_t units = 0;
-  bool pair = false;
-  if (first && nq > BM && (allow_pairs || (D->dpad > 2 * BK && (nq + BM - 1) / BM % 2 == 0))) {
-    auto kp = method == COSINE ? k_dense_tc<1, true, 2> : k_dense_tc<1, true, 3>;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2, 1, 1); cfg.blockDim = dim3(THREADS, 1, 1); cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, kp, &cfg) == cudaSuccess && clusters > 0) {
-      pair = true;
-      units = clusters;
-    }
-    cudaGetLastError();
-  }
-  int sm_count = 0;
-  cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, D->device);
-  const int64_t sms = std::max(sm_count, 1);
-  if (!pair) units = sms;
-  const int GM = pair ? Cfg<true>::GM : Cfg<false>::GM;
+  const bool pair = plan.pair;
+  const int GM = plan.gm();
   CUtensorMap qmap, rmap;
   if (!encode(Q, BM, &qmap) || !encode(D, pair ? Cfg<true>::BNL : Cfg<false>::BNL, &rmap))
     return fail(SDG_E_CUDA, "cuTensorMapEncodeTiled failed");
 
-  // (query group, reference tile) items in equal contiguous spans, one per unit
-  const int64_t G = (nq + GM - 1) / GM;
-  const int64_t ntiles = (n + BN - 1) / BN;
-  const int64_t items = G * ntiles;
-  int64_t grid = std::min<int64_t>(units, items);
-  const int64_t per = (items + grid - 1) / grid;
-  grid = (items + per - 1) / per;
-  // list slots per query: two halves per CTA whose span meets its group
-  int64_t maxc = 1;
-  for (int64_t g = 0; g < G; ++g)
-    maxc = std::max<int64_t>(maxc, last_cta(g, ntiles, per) - first_cta(g, ntiles, per) + 1);
-  const int64_t nslots = 2 * maxc;
-  const int ecap = 768;
+  const int64_t G = plan.groups, ntiles = plan.ntiles, per = plan.per, grid = plan.grid, nslots = plan.nslots;
+  const int64_t units = plan.units;
+  const int ecap = ECAP;
   const float rel = 0.0040f + (float)D->d * 2.384185791015625e-7f;
   const float omc = 1.f - (rel + 9.5367431640625e-7f);
 
   int* any = status + 1;                               // a list overflowed: the block repeats
   const int64_t ntiles1 = sample.tiles, n1 = ntiles1 * BN;
   const int gran = (int)granularity(n1, k);
-  const int64_t m = 2 * ntiles1 * gran;
+  const int64_t m = plan.maxima;
   const float opc = 1.f + rel + 1.9073486328125e-6f;     // 2^-19
 
   float *w = nullptr, *wp = nullptr, *maxima = nullptr, *lists = nullptr, *es = nullptr, *cand_s = nullptr;

@@ -184,6 +184,6 @@ int dense_query(sdg_ctx* ctx, const sdg_dense* D, const float* Q, int32_t d, int
 int32_t dense_rows(const sdg_dense* D);
 int64_t dense_cols(const sdg_dense* D);
 // device memory one dense_query of nq columns at k takes from the pool
-int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int k);
+int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int method, int k);
 
 }  // namespace sdg
