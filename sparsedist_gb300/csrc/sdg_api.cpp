@@ -1417,13 +1417,17 @@ struct Autotuner {
       if (kv.second.first > br) { br = kv.second.first; best = kv.first; }
     return best;
   }
+  // l: the log2 item size that the launch ran with, or -1 where the items were cut
+  // smaller than any of the sizes to fill the chip (the rate then says nothing of them)
   void learn_exact(int l, double steps, double seconds) {
     std::lock_guard<std::mutex> lock(mu);
     if (!(steps > 0.0) || !(seconds > 0.0)) return;
     const double rate = steps / seconds;
-    auto& r = item_rate[l];
-    r.first = r.second == 0 ? rate : 0.7 * r.first + 0.3 * rate;
-    ++r.second;
+    if (l >= 0) {
+      auto& r = item_rate[l];
+      r.first = r.second == 0 ? rate : 0.7 * r.first + 0.3 * rate;
+      ++r.second;
+    }
     exact_rate = 0.7 * exact_rate + 0.3 * rate;
   }
 };
@@ -1681,7 +1685,7 @@ SDG_API int sdg_knn_cross_batch(sdg_ctx* c, int nprob, const sdg_csc* X, const s
                            pi.as<int32_t>(), pv.as<double>(), s);
         CK(cudaGetLastError());
         const double secs = elapsed_s(e0, e1);
-        T.learn_exact(lg, total_steps, secs);
+        T.learn_exact(item_steps == std::ldexp(1.0, lg) ? lg : -1, total_steps, secs);
         if (engine_seconds) engine_seconds[0] += secs;
         c->stats[1] += (int64_t)total_steps;
         c->stats[3] += 2;
