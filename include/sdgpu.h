@@ -247,8 +247,9 @@ SDG_API int sdg_knn_resident(sdg_ctx* ctx, const sdg_matrix* X, const sdg_matrix
  * distances), the screen fused in a tcgen05 kernel (no slab in HBM) for k <= 64
  * and d <= 256, else as mode 2; mode 3: the fused screen on CTA pairs
  * (clusters of two CTAs sharing cta_group::2 UMMAs of 256 queries; the same
- * results) wherever the block has more than 128 queries, not only where mode
- * 0 finds them faster; mode 2: the same screen through a cuBLAS BF16 GEMM slab; mode 1:
+ * results) wherever the block has more than 128 queries and the references are
+ * enough for thresholds from a sample (a few thousand for k = 10), not only where
+ * mode 0 finds them faster; mode 2: the same screen through a cuBLAS BF16 GEMM slab; mode 1:
  * the plain FP32 path (FP32 GEMM, top-k on FP32 values, no re-rank).  k above
  * 1,024: every mode values every pair exactly.  No counterpart in the reference, whose
  * dense inputs are coerced to dgCMatrix (R/sparseKNN.R:194-200); the FP64
