@@ -1018,12 +1018,16 @@ __global__ void __launch_bounds__(RR_MAX_WARPS * 32) k_rerank(int method, int di
 // 20, 40, 80 and 160 entries: manhattan 374 / 135, 472 / 250, 762 / 508, 1,362 /
 // 1,109, at 320 2,636 / 2,450; euclidean 396 / 293, 515 / 531, 834 / 1,004, 1,458 /
 // 2,125; covariance 420 / 167, 432 / 280, 459 / 481, 496 / 872; js 5,856 / 1,591 (ten
-// million), 2,719 / 1,915, 2,531 / 3,660, 2,579 / 8,470.  The products and counts
-// gain as much but stay on k_rerank: a thread would walk a long column among
-// short ones alone.
-double walk_max_nnz(int method) {
-  if (method == MANHATTAN) return 128.0;
-  return (method == EUCLIDEAN || method == JS || method == COVARIANCE) ? 48.0 : 0.0;
+// million), 2,719 / 1,915, 2,531 / 3,660, 2,579 / 8,470.  Manhattan, whose step is one
+// FP64 addition, walks longer columns too where candidates are many (4,000 queries x
+// 1,500, 960 entries: k = 30 954 / 1,118, k = 100 3,145 / 2,554, k = 300 9,245 /
+// 6,963; log counts of 585 + 585: 957 / 1,054, 2,920 / 2,211, 9,169 / 7,241).  The
+// products and counts gain as much on short columns but stay on k_rerank: a thread
+// would walk a long column among short ones alone.
+constexpr int64_t WALK_MANY = (int64_t)1 << 18;      // k nq: the least candidates of a block
+bool rerank_walks(int method, int64_t nq, int k, double mean_nnz) {
+  if (method == MANHATTAN) return mean_nnz <= 128.0 || nq * k >= WALK_MANY;
+  return (method == EUCLIDEAN || method == JS || method == COVARIANCE) && mean_nnz <= 48.0;
 }
 
 __global__ void __launch_bounds__(128) k_rerank_walk(int method, int dist, DevCsc ref, ColAux ra, DevCsc qry, ColAux qa,
@@ -1416,10 +1420,10 @@ void launch_mirror_lower(double* D, int64_t n, cudaStream_t s) {
 
 int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, const DevCsc& qry, const ColAux& qa,
                   const int32_t* cand, const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
-                  int restore_self, double self_value, double* out, double mean_nnz, double mean_qnnz,
+                  int restore_self, double self_value, double* out, int k, double mean_nnz, double mean_qnnz,
                   cudaStream_t s) {
   if (nq_local <= 0) return 0;
-  if (mean_nnz + mean_qnnz <= walk_max_nnz(method)) {
+  if (rerank_walks(method, nq_local, k, mean_nnz + mean_qnnz)) {
     k_rerank_walk<<<(unsigned)nq_local, 128, 0, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin,
                                                      restore_self, self_value, out);
     return (int)cudaGetLastError();
@@ -1432,10 +1436,10 @@ int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, con
   const int rm = kind == 2 ? 32 : 64, lists = kind == 0 ? 0 : kind == 2 ? 3 : 1;
   const size_t smem = (size_t)2 * lists * 32 * (rm + 1) * 8 + (kind == 1 || kind >= 3 ? (size_t)nw * rm * 8 : 0) +
                       (size_t)((qry.nrow + 31) / 32) * 8 + (kind >= 3 ? (size_t)nw * 64 * 4 : 0);
-  auto k = kind == 0 ? k_rerank<0, 64> : kind == 1 ? k_rerank<1, 64> : kind == 2 ? k_rerank<2, 32>
-         : kind == 3 ? k_rerank<3, 64> : k_rerank<4, 64>;
+  auto kern = kind == 0 ? k_rerank<0, 64> : kind == 1 ? k_rerank<1, 64> : kind == 2 ? k_rerank<2, 32>
+            : kind == 3 ? k_rerank<3, 64> : k_rerank<4, 64>;
   if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   // a query's candidates over several CTAs where the queries are few (2 queries,
@@ -1445,8 +1449,8 @@ int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, con
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t parts = std::min<int64_t>((cap + 31) / 32, (4 * (int64_t)sms + nq_local - 1) / nq_local);
-  k<<<dim3((unsigned)nq_local, (unsigned)parts), nw * 32, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count, cap, q_begin, restore_self,
-                                              self_value, out);
+  kern<<<dim3((unsigned)nq_local, (unsigned)parts), nw * 32, smem, s>>>(method, dist, ref, ra, qry, qa, cand, count,
+                                                                         cap, q_begin, restore_self, self_value, out);
   return (int)cudaGetLastError();
 }
 

@@ -76,11 +76,11 @@ void launch_mirror_upper(double* D, int64_t n, int clear, cudaStream_t s);
 
 // Exact values of a candidate table, cand[ql * cap + t] for t < count[ql] of
 // the query columns q_begin + ql, into out at the same places; with
-// restore_self the self pair takes self_value.  nrow <= 2^18; mean_nnz,
-// mean_qnnz: stored entries of a mean reference and query column.  Returns 0 or a cudaError_t value.
+// restore_self the self pair takes self_value.  nrow <= 2^18; k neighbours;
+// mean_nnz, mean_qnnz: stored entries of a mean reference and query column.  Returns 0 or a cudaError_t value.
 int launch_rerank(int method, int dist, const DevCsc& ref, const ColAux& ra, const DevCsc& qry, const ColAux& qa,
                   const int32_t* cand, const int32_t* count, int cap, int64_t nq_local, int64_t q_begin,
-                  int restore_self, double self_value, double* out, double mean_nnz, double mean_qnnz,
+                  int restore_self, double self_value, double* out, int k, double mean_nnz, double mean_qnnz,
                   cudaStream_t s);
 
 // ---- sdg_select.cu: exact top-k selection --------------------------------------

@@ -1377,7 +1377,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
 
     // exact FP64 values of the kept pairs, then the exact top-k
     SK((cudaError_t)launch_rerank(r.method, r.dist, ref, ra, qry, qa, cand, count, cap, nb, q0,
-                                  r.selfmode && r.include_self && r.method != COVARIANCE, r.self_value, rvals,
+                                  r.selfmode && r.include_self && r.method != COVARIANCE, r.self_value, rvals, r.k,
                                   nr > 0 ? (double)rc->nnz_total / (double)nr : 0.0,
                                   nq > 0 ? (double)qc->nnz_total / (double)nq : 0.0, s));
     SelectArgs sa;

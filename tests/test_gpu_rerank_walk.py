@@ -39,3 +39,18 @@ def test_short_columns(method, stored, k, include_self):
             assert ctx.stats()["pairs_screened"] > 0
     for a, b in zip(out[:2], out[2:]):
         assert same_bits(a.idx, b.idx) and same_bits(a.dist, b.dist)
+
+
+def test_many_candidates_of_long_columns():
+    """Manhattan, k nq above the walk's limit on columns longer than its other one."""
+    import sparsedist_gb300 as sdg
+    from sparsedist_gb300 import _lib
+    X = columns(900, 2700, 100, 3)
+    out = []
+    for engine in (2, 1):
+        ctx = _lib.Context()
+        ctx.set_engine(engine)
+        out.append(sdg.sparseKNN(X, k=90, method="manhattan", include_self=True, verbose=False, ctx=ctx))
+        if engine == 2:
+            assert ctx.stats()["pairs_screened"] > 0
+    assert same_bits(out[0].idx, out[1].idx) and same_bits(out[0].dist, out[1].dist)
