@@ -232,8 +232,8 @@ struct sdg_matrix {
   DevBuf xl;                    // js: xlogx of each stored value
   DevBuf xsum;                  // js: column sums
   ScreenCache screen[kMethodCount];   // screening data per method (sdg_screen.h)
-  std::mutex rows_mu;                 // held while a screen's row-ordered entries are built
   TensorCache tensor[kMethodCount];   // dense FP16 screen values per method (tensor-core screen)
+  std::mutex screen_mu;               // held while either is built
 
   ~sdg_matrix() {
     if (ctx) {
@@ -630,7 +630,8 @@ void knn_device(sdg_ctx* c, sdg_matrix* X, sdg_matrix* Y, int method, int dist, 
   if (eng == 2 || eng == 3) {
     ScreenRun r;
     r.method = method; r.dist = dist; r.k = k; r.decreasing = P.decreasing;
-    r.rows_mu = &ref->rows_mu;
+    r.ref_mu = &ref->screen_mu; r.qry_mu = &X->screen_mu;
+    r.ref_nnz = ref->nnz; r.qry_nnz = X->nnz;
     r.selfmode = selfmode; r.include_self = P.include_self;
     r.self_value = self_value_for(P);
     r.ref_mask = P.ref_mask; r.qry_blank = P.qry_blank;

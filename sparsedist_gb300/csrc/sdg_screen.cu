@@ -1020,7 +1020,8 @@ void tensor_cache_free(TensorCache* c, cudaStream_t s) {
 // from its ScreenCache; an allocation failure leaves it unusable (the FP32
 // screen then runs) rather than failing the call.
 static int ensure_tensor(TensorCache* t, int method, const DevCsc& M, const ColAux& aux, const ScreenCache* sc,
-                         cudaStream_t s) {
+                         std::mutex* mu, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(*mu);
   if (t->method == method) return 0;
   tensor_cache_free(t, s);
   t->method = method;
@@ -1079,21 +1080,22 @@ void screen_cache_free(ScreenCache* c, cudaStream_t s) {
   if (c) *c = ScreenCache();
 }
 
-static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, const ColAux& aux,
+// The per-matrix data of a method's screens is built by the first search that
+// needs it, under the matrix's lock, and complete (synchronised) before the lock is
+// released: searches of several threads may share a matrix, each on its stream.
+static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, int64_t nnz, const ColAux& aux, std::mutex* mu,
                         cudaStream_t s) {
   const int family = method;
+  std::lock_guard<std::mutex> lock(*mu);
   if (c->method == family) return 0;
   if (method == JS && !aux.xl) {                 // the js values' x log x come first
     g_screen_site = "js x log x values missing";
     return (int)cudaErrorInvalidValue;
   }
   screen_cache_free(c, s);
-  int64_t h_nnz = 0;
-  if (M.ncol > 0) SK(cudaMemcpyAsync(&h_nnz, M.p + M.ncol, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  SK(cudaStreamSynchronize(s));
   // each array starts on a 256-byte boundary (16-byte vector loads of cnorm / nnz)
   auto seg = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
-  const size_t b_fval = seg(sizeof(float) * ((size_t)h_nnz + 4));
+  const size_t b_fval = seg(sizeof(float) * ((size_t)nnz + 4));
   const size_t b_col = seg(sizeof(float) * ((size_t)M.ncol + 4));
   const bool js = method == JS;
   const size_t bytes = (js ? 2 : 1) * b_fval + 2 * b_col + 256;
@@ -1109,29 +1111,24 @@ static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, const ColAu
   c->cnorm = reinterpret_cast<float*>(b);
   b += b_col;
   c->nnz = reinterpret_cast<int32_t*>(b);
-  c->nnz_total = h_nnz;
+  c->nnz_total = nnz;
   if (M.ncol > 0) {
     SK(cudaMemsetAsync(range_err, 0, sizeof(int), s));
     k_screen_prep<<<blocks_for(M.ncol * 32, 256), 256, 0, s>>>(M, method, aux.uval, aux.xl, c->fval, c->fxl,
                                                                 c->cnorm, c->nnz, range_err);
   }
   SK(cudaGetLastError());
-  c->values_ok = true;
-  if ((js || method == PEARSON || method == COVARIANCE) && M.ncol > 0) {
-    int h_err = 0;
+  int h_err = 0;
+  if ((js || method == PEARSON || method == COVARIANCE) && M.ncol > 0)
     SK(cudaMemcpyAsync(&h_err, range_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    SK(cudaStreamSynchronize(s));
-    c->values_ok = h_err == 0;
-  }
+  SK(cudaStreamSynchronize(s));
+  c->values_ok = h_err == 0;
   c->method = family;
   return 0;
 }
 
-// The entries of M in row order (see k_rows_fill), built by the first search
-// that screens against M and kept with it.  The matrix's lock and the
-// synchronisation make it complete before any other stream reads it; searches of
-// other matrices do not wait for it.  rows stays null when the device has no room
-// for it.
+// The entries of M in row order (see k_rows_fill).  rows stays null when the
+// device has no room for it.
 static int ensure_rows(ScreenCache* c, const DevCsc& M, std::mutex* mu, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(*mu);
   if (c->rows || M.ncol == 0 || M.nrow == 0) return 0;
@@ -1210,8 +1207,8 @@ static void screen_shape(const ScreenCache* rc, int64_t nr, int32_t nrow, int64_
 int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColAux& ra,
                ScreenCache* rc, TensorCache* rt, const DevCsc& qry, const ColAux& qa, ScreenCache* qc,
                TensorCache* qt, int32_t* d_idx, double* d_val, int64_t* stats, const ScreenHooks& hooks) {
-  SKN((cudaError_t)ensure_cache(rc, r.method, ref, ra, s));
-  SKN((cudaError_t)ensure_cache(qc, r.method, qry, qa, s));
+  SKN((cudaError_t)ensure_cache(rc, r.method, ref, r.ref_nnz, ra, r.ref_mu, s));
+  if (qc != rc) SKN((cudaError_t)ensure_cache(qc, r.method, qry, r.qry_nnz, qa, r.qry_mu, s));
   if ((r.method == JS || r.method == PEARSON || r.method == COVARIANCE) && !(rc->values_ok && qc->values_ok)) {
     // values outside the range the method's FP32 bound covers: every query exactly
     const int64_t lo = r.q_lo, hi = (r.q_hi < 0) ? qry.ncol : r.q_hi;
@@ -1220,14 +1217,14 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   }
   bool use_t = r.tensor && rt && qt && tensor_supported(r.method) && stc_supported(r.k);
   if (use_t) {
-    SKN((cudaError_t)ensure_tensor(rt, r.method, ref, ra, rc, s));
-    if (qt != rt) SKN((cudaError_t)ensure_tensor(qt, r.method, qry, qa, qc, s));
+    SKN((cudaError_t)ensure_tensor(rt, r.method, ref, ra, rc, r.ref_mu, s));
+    if (qt != rt) SKN((cudaError_t)ensure_tensor(qt, r.method, qry, qa, qc, r.qry_mu, s));
     use_t = rt->usable && qt->usable && rt->ld == qt->ld;
   }
   const int64_t nr = ref.ncol, nq = qry.ncol;
   const int32_t nrow = ref.nrow;
   if (!use_t) {
-    SKN((cudaError_t)ensure_rows(rc, ref, r.rows_mu, s));
+    SKN((cudaError_t)ensure_rows(rc, ref, r.ref_mu, s));
     if (!rc->rows) {                               // no room for the row-ordered entries: every query exactly
       const int64_t lo = r.q_lo, hi = (r.q_hi < 0) ? nq : r.q_hi;
       if (hi > lo) hooks.exact_range(lo, hi - lo);

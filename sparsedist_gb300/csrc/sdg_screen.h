@@ -57,7 +57,9 @@ struct TensorCache {
 };
 
 struct ScreenRun {
-  std::mutex* rows_mu = nullptr;           // the reference's: one thread builds its row-ordered entries
+  // the matrices' locks (one thread builds a matrix's screening data) and stored entries
+  std::mutex *ref_mu = nullptr, *qry_mu = nullptr;
+  int64_t ref_nnz = 0, qry_nnz = 0;
   int method = 0, dist = 1, k = 1;
   // the tensor-core screen (the fused tcgen05 FP16 screen, sdg_sparse_tc.cu)
   // instead of the FP32 sparse screen, when tensor_supported(method),
