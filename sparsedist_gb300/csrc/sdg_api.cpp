@@ -650,7 +650,13 @@ void knn_device(sdg_ctx* c, sdg_matrix* X, sdg_matrix* Y, int method, int dist, 
     };
     const int st = screen_knn(c->stream, r, ref->dev(), aux_of(ref), &ref->screen[method], &ref->tensor[method],
                               X->dev(), aux_of(X), &X->screen[method], &X->tensor[method], d_idx, d_val, c->stats, h);
-    if (st) cuda_check((cudaError_t)st, (std::string("screen_knn (") + screen_error_site() + ")").c_str());
+    if (st == (int)cudaErrorMemoryAllocation && c->engine == 0 && (int64_t)ref->ncol * nq <= kSmallPairs) {
+      // no room for a screen's copies or slab: the slab of a small search is at most 32 MB
+      cudaGetLastError();
+      exact_engine(c, P, ref, X, d_idx, d_val, q_lo, q_hi);
+    } else if (st) {
+      cuda_check((cudaError_t)st, (std::string("screen_knn (") + screen_error_site() + ")").c_str());
+    }
   } else {
     exact_engine(c, P, ref, X, d_idx, d_val, q_lo, q_hi);
   }

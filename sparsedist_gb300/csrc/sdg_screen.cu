@@ -1204,6 +1204,26 @@ static void screen_shape(const ScreenCache* rc, int64_t nr, int32_t nrow, int64_
   *warps = (int)std::min<int64_t>(warps_of(m * sub), std::max<int64_t>(1, (items() + nsm - 1) / nsm));
 }
 
+// Device buffers of one call, freed in stream order when it ends, also by an error
+// return or an exception of a hook.
+struct CallBuffers {
+  cudaStream_t s;
+  std::vector<void*> held;
+  explicit CallBuffers(cudaStream_t stream) : s(stream) {}
+  CallBuffers(const CallBuffers&) = delete;
+  ~CallBuffers() { release(); }
+  template <typename T>
+  cudaError_t get(T** p, size_t bytes) {
+    const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), bytes, s);
+    if (e == cudaSuccess) held.push_back(*p);
+    return e;
+  }
+  void release() {
+    for (void* p : held) cudaFreeAsync(p, s);
+    held.clear();
+  }
+};
+
 int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColAux& ra,
                ScreenCache* rc, TensorCache* rt, const DevCsc& qry, const ColAux& qa, ScreenCache* qc,
                TensorCache* qt, int32_t* d_idx, double* d_val, int64_t* stats, const ScreenHooks& hooks) {
@@ -1245,10 +1265,11 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   // the FP16 bound is wider than the FP32 one: room for more candidates
   const int cap = use_t ? std::max(512, std::min(16384, 64 * r.k + 256))
                         : std::max(256, std::min(8192, 16 * r.k + 64));
+  CallBuffers buf(s);
   float *rlo = nullptr, *rhi = nullptr;
   if (use_t) {
-    SK(cudaMallocAsync(&rlo, sizeof(float) * (size_t)(chunk * cap + 4), s));
-    SK(cudaMallocAsync(&rhi, sizeof(float) * (size_t)(chunk * cap + 4), s));
+    SK(buf.get(&rlo, sizeof(float) * (size_t)(chunk * cap + 4)));
+    SK(buf.get(&rhi, sizeof(float) * (size_t)(chunk * cap + 4)));
   }
 
   float* S = nullptr;
@@ -1260,15 +1281,15 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   double* rvals = nullptr;
   uint8_t* force = nullptr;
   const int64_t cslots = chunk * (int64_t)cap;
-  if (!use_t) SK(cudaMallocAsync(&S, sizeof(float) * (size_t)(chunk * ldS + 4), s));
-  SK(cudaMallocAsync(&cand, sizeof(int32_t) * (size_t)cslots, s));
-  SK(cudaMallocAsync(&count, sizeof(int32_t) * (size_t)chunk, s));
-  SK(cudaMallocAsync(&over, sizeof(int32_t) * (size_t)chunk, s));
-  SK(cudaMallocAsync(&rvals, sizeof(double) * (size_t)cslots, s));
-  SK(cudaMallocAsync(&work, sizeof(*work), s));
+  if (!use_t) SK(buf.get(&S, sizeof(float) * (size_t)(chunk * ldS + 4)));
+  SK(buf.get(&cand, sizeof(int32_t) * (size_t)cslots));
+  SK(buf.get(&count, sizeof(int32_t) * (size_t)chunk));
+  SK(buf.get(&over, sizeof(int32_t) * (size_t)chunk));
+  SK(buf.get(&rvals, sizeof(double) * (size_t)cslots));
+  SK(buf.get(&work, sizeof(*work)));
   if (!use_t) {
-    SK(cudaMallocAsync(&order, sizeof(int2) * (size_t)max_units, s));
-    SK(cudaMallocAsync(&units, sizeof(int32_t), s));
+    SK(buf.get(&order, sizeof(int2) * (size_t)max_units));
+    SK(buf.get(&units, sizeof(int32_t)));
   }
   // cosine cannot bound an all-zero query (its convention value is not a dot
   // product): such queries go to the exact engine.
@@ -1401,15 +1422,7 @@ int screen_knn(cudaStream_t s, const ScreenRun& r, const DevCsc& ref, const ColA
   overflow_queries.erase(std::unique(overflow_queries.begin(), overflow_queries.end()),
                          overflow_queries.end());
   stats[2] += (int64_t)overflow_queries.size();
-  if (S) SK(cudaFreeAsync(S, s));
-  SK(cudaFreeAsync(cand, s)); SK(cudaFreeAsync(count, s));
-  SK(cudaFreeAsync(over, s)); 
-  SK(cudaFreeAsync(rvals, s));
-  SK(cudaFreeAsync(work, s));
-  if (order) SK(cudaFreeAsync(order, s));
-  if (units) SK(cudaFreeAsync(units, s));
-  if (rlo) SK(cudaFreeAsync(rlo, s));
-  if (rhi) SK(cudaFreeAsync(rhi, s));
+  buf.release();
   // queries the screen could not bound: the exact slab engine
   if (!overflow_queries.empty()) hooks.exact_list(overflow_queries);
   return 0;

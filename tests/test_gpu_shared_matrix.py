@@ -1,13 +1,16 @@
 """Small searches of several threads, each with its own context and stream, against
 one fresh resident matrix (as reference, and as the query matrix of blocks): the
 matrix's screening data is built once and complete before any of them reads it, so
-every result is the exact engine's."""
+every result is the exact engine's.  And a search that is cancelled returns its
+device buffers."""
 import ctypes as C
 import threading
 
 import numpy as np
 import pytest
 import scipy.sparse as sp
+
+from test_gpu_dense_admission import USED_CURRENT, Pool
 
 pytestmark = pytest.mark.gpu
 CODES = {"binary": 0, "euclidean": 2, "manhattan": 3}
@@ -55,3 +58,19 @@ def test_threads_share_a_fresh_matrix(method):
             th.join()
         assert got == want
         assert any(c.stats()["pairs_screened"] for c in ctxs)
+
+
+def test_a_cancelled_search_returns_its_buffers():
+    from sparsedist_gb300 import _lib
+    ctx, pool = _lib.Context(), Pool()
+    Y, X = resident(ctx, 3000, 2500, 1), resident(ctx, 3000, 900, 2)
+    for engine in (2, 3):
+        ctx.set_engine(engine)
+        want = block(ctx, X, Y, 0, 900, "euclidean")
+        used = pool.get(USED_CURRENT)
+        ctx.cancel()
+        with pytest.raises(_lib.SdgError):
+            block(ctx, X, Y, 0, 900, "euclidean")
+        ctx.reset_cancel()
+        assert pool.get(USED_CURRENT) <= used
+        assert block(ctx, X, Y, 0, 900, "euclidean") == want
