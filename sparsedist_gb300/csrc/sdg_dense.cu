@@ -889,10 +889,9 @@ int query_build(sdg_ctx* ctx, const float* X, int32_t d, int64_t n, int method, 
   return SDG_OK;
 }
 
-// candidates a query's table holds; queries of a block; the slab's leading
-// dimension and the queries of a pass over it (8 GB)
+// candidates a query's table holds; the slab's leading dimension and the queries
+// of a pass over it (8 GB)
 int dense_cap(int k) { return std::max(512, std::min(16384, 64 * k + 256)); }
-constexpr int64_t DENSE_CHUNK = 65536;
 int64_t slab_ld(int64_t n) { return (n + 127) / 128 * 128; }
 int64_t slab_chunk(int64_t n, int64_t nq) {
   return std::max<int64_t>(1, std::min<int64_t>(nq, ((int64_t)8 << 30) / (4 * slab_ld(n))));
@@ -973,7 +972,7 @@ int dense_search(sdg_ctx* ctx, const sdg_dense* Q, int64_t q0, int64_t nq, const
   const int smode = (mode == 1) ? 1 : 0;
   const int64_t ldS = slab_ld(n);
   const int nseg = (int)((n + DSEG - 1) / DSEG);
-  const int64_t chunk = fused ? std::min<int64_t>(nq, DENSE_CHUNK) : slab_chunk(n, nq);
+  const int64_t chunk = fused ? tc_screen_chunk(D, k, nq) : slab_chunk(n, nq);
   float* S = nullptr;
   float *segtop = nullptr, *cut = nullptr;
   int32_t *cand = nullptr, *count = nullptr, *over = nullptr, *o_idx = idx;
@@ -1165,7 +1164,7 @@ int64_t dense_query_bytes(const sdg_dense* D, int64_t nq, int method, int k) {
   if (k > kMaxK) return bytes + 8 * D->n + ((int64_t)256 << 20);   // one row at a time, the lists' scratch
   const int cap = dense_cap(k);
   if (tc_screen_supported(D, method, k)) {
-    const int64_t chunk = std::min<int64_t>(nq, DENSE_CHUNK);
+    const int64_t chunk = tc_screen_chunk(D, k, nq);
     int dev = -1;                            // the caller's thread may be on another device
     cudaGetDevice(&dev);
     cudaSetDevice(D->device);

@@ -74,6 +74,9 @@ __device__ __forceinline__ float dense_cut(float T) {
 // Queries are columns q0.. of Q, references the columns of D (self: Q is D
 // and each query's own column is skipped).
 bool tc_screen_supported(const sdg_dense* D, int method, int k);
+// queries of one block: 65,536, fewer where the sample's maxima would take more than
+// 4 GB (from 16 million references on)
+int64_t tc_screen_chunk(const sdg_dense* D, int k, int64_t nq);
 // device bytes that tc_screen takes for a block of nq queries while it runs
 int64_t tc_screen_bytes(const sdg_dense* D, int method, int k, int64_t nq, int cap);
 // allow_pairs: run CTA pairs (cta_group::2, M = 256) wherever the block has

@@ -1211,6 +1211,13 @@ bool tc_screen_supported(const sdg_dense* R, int method, int k) {
          R->n < (int64_t)1 << 30 && encode_fn() != nullptr;
 }
 
+int64_t tc_screen_chunk(const sdg_dense* D, int k, int64_t nq) {
+  const SampleMap z = sample_of(D->n, k);
+  const int64_t per_query = 4 * std::max<int64_t>(1, z.s > 0 ? maxima_per_query(z.tiles * BN, k) : 0);
+  const int64_t most = std::max<int64_t>(1, ((int64_t)4 << 30) / per_query / (2 * BM)) * (2 * BM);
+  return std::min<int64_t>(nq, std::min<int64_t>(65536, most));
+}
+
 int64_t tc_screen_bytes(const sdg_dense* D, int method, int k, int64_t nq, int cap) {
   const TcPlan z = tc_plan(D, method, k, nq, false);
   const int64_t weights = 4 * BN * (z.ntiles + z.sample.tiles);
