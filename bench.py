@@ -737,7 +737,7 @@ def run_dense_main(args):
 # kernel at the bench's full size, from a one-pass ncu capture
 # (profiles/k_dense_tc_cosine_400000x256_q4096.md,
 # profiles/launches_logcount_cosine_30000x200000_q4096.md)
-DENSE_TRAFFIC = (0.142e9 + 0.021e9) + (1.28e9 + 0.034e9)
+DENSE_TRAFFIC = (0.142e9 + 0.021e9) + (1.26e9 + 0.032e9)
 LOGCOUNT_TRAFFIC = 69.44e9 + 0.181e9
 
 
