@@ -1077,17 +1077,24 @@ void screen_cache_free(ScreenCache* c, cudaStream_t s) {
   if (c && c->rows) cudaFreeAsync(c->rows, s);
   if (c && c->ent) cudaFreeAsync(c->ent, s);
   if (c && c->exl) cudaFreeAsync(c->exl, s);
+  if (c && c->ready) cudaEventDestroy(c->ready);
   if (c) *c = ScreenCache();
 }
 
 // The per-matrix data of a method's screens is built by the first search that
-// needs it, under the matrix's lock, and complete (synchronised) before the lock is
-// released: searches of several threads may share a matrix, each on its stream.
+// needs it, under the matrix's lock: searches of several threads may share a
+// matrix, each on its stream.  The FP32 values are built without a
+// synchronisation; a later search waits for their event on its own stream (on the
+// host, knn-size calls from fresh matrices were 20 us slower).  The FP16 copy and
+// the row-ordered entries are complete before the lock is released.
 static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, int64_t nnz, const ColAux& aux, std::mutex* mu,
                         cudaStream_t s) {
   const int family = method;
   std::lock_guard<std::mutex> lock(*mu);
-  if (c->method == family) return 0;
+  if (c->method == family) {
+    SK(cudaStreamWaitEvent(s, c->ready, 0));
+    return 0;
+  }
   if (method == JS && !aux.xl) {                 // the js values' x log x come first
     g_screen_site = "js x log x values missing";
     return (int)cudaErrorInvalidValue;
@@ -1118,11 +1125,15 @@ static int ensure_cache(ScreenCache* c, int method, const DevCsc& M, int64_t nnz
                                                                 c->cnorm, c->nnz, range_err);
   }
   SK(cudaGetLastError());
-  int h_err = 0;
-  if ((js || method == PEARSON || method == COVARIANCE) && M.ncol > 0)
+  c->values_ok = true;
+  if ((js || method == PEARSON || method == COVARIANCE) && M.ncol > 0) {
+    int h_err = 0;
     SK(cudaMemcpyAsync(&h_err, range_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  SK(cudaStreamSynchronize(s));
-  c->values_ok = h_err == 0;
+    SK(cudaStreamSynchronize(s));
+    c->values_ok = h_err == 0;
+  }
+  if (!c->ready) SK(cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming));
+  SK(cudaEventRecord(c->ready, s));
   c->method = family;
   return 0;
 }

@@ -24,6 +24,7 @@ struct ScreenCache {
   float* cnorm = nullptr;    // per column: norm term of the method (js: sum of |x log x| + x, rounded up)
   int32_t* nnz = nullptr;    // per column: stored entries
   int64_t nnz_total = 0;
+  cudaEvent_t ready = nullptr;   // the arrays above are complete
   // the entries in row order, built by the first FP32 screen against the
   // matrix (see k_rows_fill in sdg_screen.cu): (column, value) pairs and js's x
   // log x, in cells of 2^sub_lg columns, nsub cells a row
