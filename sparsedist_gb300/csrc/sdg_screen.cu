@@ -474,7 +474,7 @@ struct SelectScreenArgs {
   int cap;
   int slices;                                // stretches of a row in the first pass
   int32_t* cand;                             // [qlocal * cap + t] reference column
-  float* hi;                                 // the same places: the candidates' upper bounds
+  float* hi;                                 // the same places: the candidates' upper bounds (js, pearson, covariance)
   int32_t* count;                            // kept pairs per query (capped)
   int32_t* overflow;                         // 1 = finish with the exact engine
 };
@@ -666,10 +666,11 @@ struct ScreenBounds {
 //
 // Bound by the slab's read (the second pass finds its row in the L2) and, for
 // short rows, by the two bit searches; pearson and covariance by the FP64 bounds,
-// so the cut at T reads the upper bounds that the second pass stored
-// (formed again by one warp, four columns a lane, it cost more than a
-// pass: 10,000 queries x 1,000 references, k = 100, pearson 7,207 us and 4,960
-// now, covariance 3,249 and 2,160).  us: 10,000 queries x 10,000 references
+// so their cut at T (and js's) reads the upper bounds that the second pass stored
+// (formed again by one warp, four columns a lane, it cost more than a pass: 10,000
+// queries x 1,000 references, k = 100, pearson 7,207 us and 4,960 now, covariance
+// 3,249 and 2,160; the cheap bounds are formed again: binary, 10,000 x 10,000, 298
+// us, stored 319).  us: 10,000 queries x 10,000 references
 // (binary) 655 with scalar loads, per-pair term counts and IEEE divisions, 296
 // now; 12,001 x 1,500 163 and 126; 1,500 x 12,001 121 and 52.  A warp per query
 // with k-long sorted insertions, reading the norms through a column permutation,
@@ -694,11 +695,11 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
   const float4* S4 = reinterpret_cast<const float4*>(Srow);
   const kth::Group<1> G{nullptr};
   const int64_t n4 = (A.nr + 3) / 4, stretch = (n4 + A.slices - 1) / A.slices;
-  // The thread's place in a stretch: the warps take turns at the first places, so
-  // that the stretches' short last rounds (always warp 0 otherwise, the same
-  // quarter of every SM) spread over the FP64 pipes: covariance, 6,063 queries x
-  // 5,669 references, k = 300, 8,156 us without
-  auto turn = [&](int sl) { return (tid + 32 * (int)((blockIdx.x + sl) % WARPS)) % NT; };
+  // The thread's place in a stretch.  KIND 4: the warps take turns at the first
+  // places, so that the stretches' short last rounds (always warp 0 otherwise, the
+  // same quarter of every SM) spread over the FP64 pipes: covariance, 6,063 queries x
+  // 5,669 references, k = 300, 8,156 us without and 7,352 with
+  auto turn = [&](int sl) { return KIND == 4 ? (tid + 32 * (int)((blockIdx.x + sl) % WARPS)) % NT : tid; };
   for (int sl = 0; sl < A.slices; ++sl) {
     const int64_t g1 = min((sl + 1) * stretch, n4);
     float best = -INFINITY;
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
           if (at < A.cap) {
             out[at] = (int32_t)(4 * g + u);
             keys[at] = kth::fkey(lo[u]);
-            his[at] = hi[u];
+            if constexpr (KIND >= 3) his[at] = hi[u];
           }
         }
       }
@@ -767,7 +768,15 @@ __global__ void __launch_bounds__(WARPS * 32) k_screen_select(SelectScreenArgs A
       for (int t0 = 0; t0 < n; t0 += 32) {
         const int t = t0 + lane;
         const int32_t c = t < n ? out[t] : 0;
-        const bool keep = t < n && his[t] >= cut;
+        bool keep = false;
+        if constexpr (KIND >= 3) {
+          keep = t < n && his[t] >= cut;
+        } else if (t < n) {
+          float lo[4], hi[4];
+          bounds(c & ~3, A.nr, S4[c >> 2], lo, hi);
+          const float h = (c & 2) ? ((c & 1) ? hi[3] : hi[2]) : ((c & 1) ? hi[1] : hi[0]);
+          keep = h >= cut;
+        }
         const unsigned m = __ballot_sync(0xffffffffu, keep);   // every lane has read slot t first
         if (keep) out[kept + __popc(m & ((1u << lane) - 1u))] = c;
         kept += __popc(m);
