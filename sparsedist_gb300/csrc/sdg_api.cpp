@@ -540,12 +540,6 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
   if (c->engine == 3) return (tensor_supported(P.method) && stc_supported(P.k)) ? 3 : 2;
   const int m = P.method;
   const bool small = nr * nq <= kSmallPairs;
-  if (small) {
-    // into a graph that is being captured: the screens read counts back, the slab
-    // does not, so a small search of prepared matrices can be captured
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) return 1;
-  }
   // the tensor screen where the reference is dense enough and the dense copies
   // fit in half of the free device memory
   const TensorCache& rt = ref->tensor[m];
@@ -575,7 +569,12 @@ int pick_engine(sdg_ctx* c, const KnnPlan& P, const sdg_matrix* ref, const sdg_m
                     kSmallCopyBytes)
     tensor_us = screen_us(z, true) + (have_rt ? 0.0 : copy_us(m, true, true, nrow, (double)nr, z.nnz_r)) +
                 (have_qt ? 0.0 : copy_us(m, true, false, nrow, (double)X->ncol, (double)X->nnz));
-  if (tensor_us < fp32_us && !exact_is_cheaper(z, tensor_us) && copies_fit()) return 3;
+  if (exact_is_cheaper(z, std::min(fp32_us, tensor_us))) return 1;
+  // into a graph that is being captured: the screens read counts back, the slab
+  // does not, so a small search of prepared matrices can be captured
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) return 1;
+  if (tensor_us < fp32_us && copies_fit()) return 3;
   return exact_is_cheaper(z, fp32_us) ? 1 : 2;
 }
 
